@@ -12,9 +12,10 @@
 // prefix (flag PREFIX), and publishes its own prefix (decoupled look-back).
 // The first pass's digit counts come from one read of the keys; each pass
 // counts the next pass's digits of the keys it holds.
-// Status words are 64 bits (flag in the high half, count in the low half),
-// written and read with single relaxed accesses; a wait that outlasts its
-// iteration limit sets GVIZ_ST_TREE and ends.
+// Status words are 64 bits in the scan (flag in the high half, count in the
+// low half) and 32 bits in the sort, written and read with single relaxed
+// accesses; a wait that outlasts its iteration limit sets GVIZ_ST_TREE and
+// ends.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -26,15 +27,18 @@ constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;  // 2048
 constexpr int kTopThreads = 1024;
 
-constexpr int kSortThreads = 256;
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortRounds = 16;
-constexpr int kSortTile = kSortThreads * kSortRounds;  // 4096 keys
+constexpr int kLookbackWidth = 8;
+constexpr int kSortThreads = 512;
+constexpr int kHistThreads = 256;
 constexpr int kSortPasses = (64 - GVIZ_SORT_SKIP_BITS) / 8;
 static_assert(kSortPasses % 2 == 0, "the sorted pairs must end in the input buffers");
 
 constexpr uint64_t kFlagAggregate = 1ull << 32;
 constexpr uint64_t kFlagPrefix = 2ull << 32;
+// the sort's status words: flag in the top two bits, count below (n < 2^30)
+constexpr uint32_t kAggregate32 = 1u << 30;
+constexpr uint32_t kPrefix32 = 1u << 31;
+constexpr uint32_t kCount32 = kAggregate32 - 1u;
 constexpr uint32_t kLookbackSpin = 1u << 22;  // reads of a status word before giving up
 
 __device__ __forceinline__ uint64_t ld_status(const uint64_t *p) {
@@ -47,32 +51,75 @@ __device__ __forceinline__ void st_status(uint64_t *p, uint64_t v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// The sum of the counts of tiles [0, tile) in the status column `st` of
-// stride `stride` (tile t's word is st[t * stride]), read kLookbackWidth
-// tiles at a time (independent loads). Tile 0 publishes its prefix without
-// waiting, so the walk always ends.
-constexpr int kLookbackWidth = 8;
+__device__ __forceinline__ uint32_t ld_status32(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 
-__device__ __forceinline__ uint32_t lookback(const uint64_t *st, size_t stride, uint32_t tile,
-                                             uint32_t *status) {
+__device__ __forceinline__ void st_status32(uint32_t *p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The sort's look-back, one thread per digit: the sum of the counts of tiles
+// [0, tile) in the status column `st` of stride 256 (tile t's word is
+// st[256 t]), WIDTH tiles per step (independent loads). The tiles of a pass
+// run side by side and publish their counts at about the same time, so the
+// walk is a chain of L2 round trips; its length, not its traffic, sets the
+// pass's time, hence the wide step. Tile 0 publishes its prefix without
+// waiting, so the walk always ends.
+template <int WIDTH>
+__device__ __forceinline__ uint32_t lookback_digit(const uint32_t *st, uint32_t tile,
+                                                   uint32_t *status) {
   uint32_t excl = 0;
   uint32_t spins = 0;
-  for (int64_t p = (int64_t)tile - 1; p >= 0; p -= kLookbackWidth) {
-    uint64_t w[kLookbackWidth];
+  for (int64_t p = (int64_t)tile - 1; p >= 0; p -= WIDTH) {
+    uint32_t w[WIDTH];
 #pragma unroll
-    for (int i = 0; i < kLookbackWidth; i++)
-      w[i] = p - i >= 0 ? ld_status(st + (size_t)(p - i) * stride) : kFlagPrefix;
+    for (int i = 0; i < WIDTH; i++)
+      w[i] = p - i >= 0 ? ld_status32(st + (size_t)(p - i) * 256) : kPrefix32;
 #pragma unroll
-    for (int i = 0; i < kLookbackWidth; i++) {
-      while ((w[i] >> 32) == 0) {  // not published yet
+    for (int i = 0; i < WIDTH; i++) {
+      while ((w[i] & ~kCount32) == 0) {  // not published yet
         if (++spins > kLookbackSpin) {
           atomicOr(status, GVIZ_ST_TREE);
           return excl;
         }
-        w[i] = ld_status(st + (size_t)(p - i) * stride);
+        w[i] = ld_status32(st + (size_t)(p - i) * 256);
       }
-      excl += (uint32_t)w[i];
-      if ((w[i] & ~0xffffffffull) == kFlagPrefix) return excl;
+      excl += w[i] & kCount32;
+      if (w[i] & kPrefix32) return excl;
+    }
+  }
+  return excl;
+}
+
+// The scan's look-back by one warp: lane l reads the word of the l-th tile
+// before, so a step covers 32 tiles; the result is in every lane.
+__device__ __forceinline__ uint32_t lookback_warp(const uint64_t *st, uint32_t tile,
+                                                  uint32_t *status) {
+  const uint32_t lane = lane_id();
+  uint32_t excl = 0;
+  uint32_t spins = 0;
+  for (int64_t p = (int64_t)tile - 1; p >= 0; p -= 32) {
+    uint64_t w = p - lane >= 0 ? ld_status(st + (size_t)(p - lane)) : kFlagPrefix;
+    uint32_t have;
+    for (;;) {
+      // enough once every word up to the nearest prefix is published
+      have = __ballot_sync(0xffffffffu, (w >> 32) != 0);
+      const uint32_t pre = __ballot_sync(0xffffffffu, (w & ~0xffffffffull) == kFlagPrefix);
+      const uint32_t need = pre ? (pre ^ (pre - 1u)) : 0xffffffffu;
+      if ((have & need) == need) {
+        uint32_t c = (need >> lane) & 1u ? (uint32_t)w : 0u;
+        excl += __reduce_add_sync(0xffffffffu, c);
+        if (pre) return excl;
+        break;
+      }
+      if (++spins > kLookbackSpin) {
+        if (lane == 0) atomicOr(status, GVIZ_ST_TREE);
+        return excl;
+      }
+      if ((w >> 32) == 0) w = ld_status(st + (size_t)(p - lane));
     }
   }
   return excl;
@@ -133,18 +180,15 @@ __global__ __launch_bounds__(kScanThreads) void k_scan_onepass(
   uint32_t excl;
   const uint32_t tot = block_exclusive_scan<kScanThreads>(s, excl);
   uint64_t *st = state + 1;
-  if (threadIdx.x == 0) {
-    if (tile == 0) {
-      st_status(st, kFlagPrefix | tot);
-      sExcl = 0;
-    } else {
-      st_status(st + tile, kFlagAggregate | tot);
-      const uint32_t before = lookback(st, 1, tile, status);
+  if (threadIdx.x < 32) {
+    if (tile != 0 && threadIdx.x == 0) st_status(st + tile, kFlagAggregate | tot);
+    const uint32_t before = lookback_warp(st, tile, status);
+    if (threadIdx.x == 0) {
       st_status(st + tile, kFlagPrefix | (before + tot));
       sExcl = before;
+      const uint32_t nTiles = (n + kScanTile - 1) / kScanTile;
+      if (total && tile == nTiles - 1) *total = before + tot;
     }
-    const uint32_t nTiles = (n + kScanTile - 1) / kScanTile;
-    if (total && tile == nTiles - 1) *total = sExcl + tot;
   }
   __syncthreads();
   excl += sExcl;
@@ -184,126 +228,139 @@ __global__ __launch_bounds__(kTopThreads) void k_scan_single(
 
 // Digit counts of the first sort pass (each later pass counts the digit of
 // the pass after it while it scatters).
-__global__ __launch_bounds__(kSortThreads) void k_radix_hist0(
+__global__ __launch_bounds__(kHistThreads) void k_radix_hist0(
     const uint64_t *__restrict__ keys, uint32_t n, uint32_t *ghist) {
   __shared__ uint32_t sh[256];
   sh[threadIdx.x] = 0u;
   __syncthreads();
-  const uint32_t stride = gridDim.x * kSortThreads;
-  for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += stride)
+  const uint32_t stride = gridDim.x * kHistThreads;
+  for (uint32_t i = blockIdx.x * kHistThreads + threadIdx.x; i < n; i += stride)
     atomicAdd(&sh[(uint32_t)(keys[i] >> GVIZ_SORT_SKIP_BITS) & 255u], 1u);
   __syncthreads();
   const uint32_t c = sh[threadIdx.x];
   if (c) atomicAdd(ghist + threadIdx.x, c);
 }
 
-// Stable scatter: warp w of a tile owns 512 consecutive keys, taken in
-// rounds of 32; __match_any_sync ranks equal digits inside a round.
+// The lanes holding valid keys of the same 8-bit digit d: eight ballots, one
+// per bit, which do not depend on each other.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool valid) {
+  uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const uint32_t set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+    peers &= ((d >> b) & 1u) ? set : ~set;
+  }
+  return peers;
+}
+
+// Stable scatter: warp w of a tile owns 32 * ROUNDS consecutive keys, taken
+// in rounds of 32; ballots rank equal digits inside a round. A pass moves
+// 24 B per key but is bound by latency: the ticket, the ranking rounds (each
+// reads and writes its warp's counters) and the look-back. __match_any_sync
+// in place of the ballots and 16 rounds of 256 threads took 23.5 us per pass
+// at 1,048,576 keys and 14.5 us at 1,024 (one tile); this takes 17 and 5.5.
 // Shared memory of the scatter beyond its static arrays: the tile's keys
 // and values reordered by digit.
-constexpr size_t kScatterDyn = (size_t)kSortTile * (sizeof(uint64_t) + sizeof(uint32_t));
+constexpr size_t scatter_dyn(size_t tile) { return tile * (sizeof(uint64_t) + sizeof(uint32_t)); }
 
 // One pass over digit `pass`: tile = ticket; each digit's start in the
 // output is its global start (a scan of ghist) plus its count in the tiles
 // before (look-back over the status words state[tile * 256 + digit]).
-__global__ __launch_bounds__(kSortThreads) void k_radix_onesweep(
+template <int THREADS, int ROUNDS>
+__global__ __launch_bounds__(THREADS) void k_radix_onesweep(
     const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin,
     uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, uint32_t n,
-    int pass, uint32_t *ghist, uint64_t *state, uint32_t *ticket,
+    int pass, uint32_t *ghist, uint32_t *state, uint32_t *ticket,
     uint32_t *status) {
+  constexpr int kWarps = THREADS / 32;
+  constexpr uint32_t kTile = THREADS * ROUNDS;
   extern __shared__ __align__(16) unsigned char dyn[];
   uint64_t *sk = reinterpret_cast<uint64_t *>(dyn);
-  uint32_t *sv = reinterpret_cast<uint32_t *>(sk + kSortTile);
-  __shared__ uint32_t wcnt[kSortWarps][256];
+  uint32_t *sv = reinterpret_cast<uint32_t *>(sk + kTile);
+  __shared__ uint32_t wcnt[kWarps][256];
   __shared__ uint32_t base[256];
   __shared__ uint32_t start[256];  // first in-tile position of each digit
-  __shared__ uint32_t wsum[kSortWarps];
   __shared__ uint32_t sTile;
   __shared__ uint32_t nextCnt[256];  // the next pass's digit counts of this tile
   const unsigned tid = threadIdx.x, w = tid >> 5, lane = tid & 31u;
   const int shift = GVIZ_SORT_SKIP_BITS + 8 * pass;
   const bool countNext = pass + 1 < kSortPasses;
+  const bool digitThread = tid < 256;  // thread d looks after digit d
   if (tid == 0) sTile = atomicAdd(ticket, 1u);
-  for (unsigned d = tid; d < kSortWarps * 256; d += kSortThreads)
-    (&wcnt[0][0])[d] = 0;
-  nextCnt[tid] = 0u;
+  for (unsigned d = tid; d < kWarps * 256; d += THREADS) (&wcnt[0][0])[d] = 0;
+  if (digitThread) nextCnt[tid] = 0u;
   // the digit's first output position: exclusive scan of the global counts
   uint32_t gstart;
-  block_exclusive_scan<kSortThreads>(ghist[pass * 256 + tid], gstart);
-  __syncthreads();
+  block_exclusive_scan<THREADS>(digitThread ? ghist[pass * 256 + tid] : 0u, gstart);
   const uint32_t tile = sTile;
-  const uint32_t tileBase = tile * kSortTile + w * (kSortRounds * 32);
-  uint64_t k[kSortRounds];
-  uint32_t v[kSortRounds];
-  uint32_t rank[kSortRounds];
+  const uint32_t tileBase = tile * kTile + w * (ROUNDS * 32);
+  uint64_t k[ROUNDS];
+  uint32_t v[ROUNDS];
+  uint32_t rank[ROUNDS];
+  // all of the tile's loads are in flight before the first is ranked: the
+  // ranking rounds below are ordered by warp barriers, which no load crosses
 #pragma unroll
-  for (int r = 0; r < kSortRounds; r++) {
-    uint32_t i = tileBase + r * 32 + lane;
-    bool valid = i < n;
-    k[r] = valid ? kin[i] : 0ull;
-    v[r] = valid ? vin[i] : 0u;
-    uint32_t d = valid ? ((uint32_t)(k[r] >> shift) & 255u) : 256u;
+  for (int r = 0; r < ROUNDS; r++) {
+    const uint32_t i = tileBase + r * 32 + lane;
+    k[r] = i < n ? kin[i] : 0ull;
+    v[r] = i < n ? vin[i] : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < ROUNDS; r++) {
+    const bool valid = tileBase + r * 32 + lane < n;
+    const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
     if (countNext && valid) atomicAdd(&nextCnt[(uint32_t)(k[r] >> (shift + 8)) & 255u], 1u);
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
-    uint32_t lt = peers & ((1u << lane) - 1u);
-    uint32_t before = valid ? wcnt[w][d] : 0u;
+    const uint32_t peers = digit_peers(d, valid);
+    const uint32_t lt = peers & ((1u << lane) - 1u);
+    const uint32_t before = valid ? wcnt[w][d] : 0u;
     rank[r] = before + __popc(lt);
     __syncwarp();
     if (valid && lt == 0) wcnt[w][d] = before + __popc(peers);
     __syncwarp();
   }
   __syncthreads();
-  // per digit (thread tid = digit): warps' offsets, then the tile's digit
-  // starts by a block-wide exclusive scan of the digit totals
+  // per digit: warps' offsets, then this tile's count of the digit and the
+  // counts of the tiles before; the tile's digit starts by a block-wide
+  // exclusive scan of the digit totals
   uint32_t run = 0;
+  if (digitThread) {
 #pragma unroll
-  for (int ww = 0; ww < kSortWarps; ww++) {
-    uint32_t t = wcnt[ww][tid];
-    wcnt[ww][tid] = run;
-    run += t;
-  }
-  // this tile's count of digit tid, then the counts of the tiles before
-  {
-    uint64_t *col = state + tid;
-    if (tile == 0) {
-      st_status(col, kFlagPrefix | run);
-      base[tid] = gstart;
-    } else {
-      st_status(col + (size_t)tile * 256, kFlagAggregate | run);
-      const uint32_t before = lookback(col, 256, tile, status);
-      st_status(col + (size_t)tile * 256, kFlagPrefix | (before + run));
-      base[tid] = gstart + before;
+    for (int ww = 0; ww < kWarps; ww++) {
+      const uint32_t t = wcnt[ww][tid];
+      wcnt[ww][tid] = run;
+      run += t;
     }
+    st_status32(state + tid + (size_t)tile * 256, (tile == 0 ? kPrefix32 : kAggregate32) | run);
+    if (countNext && nextCnt[tid]) atomicAdd(ghist + (pass + 1) * 256 + tid, nextCnt[tid]);
   }
-  if (countNext && nextCnt[tid]) atomicAdd(ghist + (pass + 1) * 256 + tid, nextCnt[tid]);
-  uint32_t incl = run;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= (unsigned)o) incl += y;
-  }
-  if (lane == 31) wsum[w] = incl;
-  __syncthreads();
-  uint32_t before = 0;
-  for (unsigned ww = 0; ww < w; ww++) before += wsum[ww];
-  start[tid] = before + incl - run;
+  uint32_t first;
+  block_exclusive_scan<THREADS>(run, first);
+  if (digitThread) start[tid] = first;
   __syncthreads();
   // the tile reordered by digit in shared memory (stable: warp, round, lane
   // is input order) ...
 #pragma unroll
-  for (int r = 0; r < kSortRounds; r++) {
-    uint32_t i = tileBase + r * 32 + lane;
-    if (i >= n) continue;
-    uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
+  for (int r = 0; r < ROUNDS; r++) {
+    if (tileBase + r * 32 + lane >= n) continue;
+    const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
     const uint32_t pos = start[d] + wcnt[w][d] + rank[r];
     sk[pos] = k[r];
     sv[pos] = v[r];
   }
+  if (digitThread) {
+    uint32_t *col = state + tid;
+    const uint32_t before = tile ? lookback_digit<kLookbackWidth>(col, tile, status) : 0u;
+    if (tile) st_status32(col + (size_t)tile * 256, kPrefix32 | (before + run));
+    base[tid] = gstart + before;
+  }
   __syncthreads();
   // ... then written out in order: each digit's run lands contiguously
-  const uint32_t t0 = tile * kSortTile;
-  const uint32_t cnt = n - t0 < (uint32_t)kSortTile ? n - t0 : (uint32_t)kSortTile;
-  for (uint32_t j = tid; j < cnt; j += kSortThreads) {
+  const uint32_t t0 = tile * kTile;
+  const uint32_t cnt = n - t0 < kTile ? n - t0 : kTile;
+#pragma unroll
+  for (int r = 0; r < ROUNDS; r++) {
+    const uint32_t j = r * THREADS + tid;
+    if (j >= cnt) break;
     const uint64_t kk = sk[j];
     const uint32_t d = (uint32_t)(kk >> shift) & 255u;
     const uint32_t dst = base[d] + (j - start[d]);
@@ -318,11 +375,34 @@ size_t scan_state_entries(size_t n) {
   return (n + kScanTile - 1) / kScanTile + 1;
 }
 
+struct SortShape {
+  int threads, rounds;
+  size_t tile() const { return (size_t)threads * rounds; }
+};
+
+// Tile of a pass: small tiles keep a short array's passes spread over the
+// GPU and their serial ranking rounds few; large ones shorten the look-back's
+// chain of tiles. Whole step in us, tiles of 512 x 2 / 512 x 4 / 512 x 8 keys
+// (256 x 16 with __match_any_sync before): 1,024 vertices 169 / 172 / 179
+// (196), 65,537 311 / 316 / 323 (358), 262,144 639 / 636 / 635 (669), 0.75M
+// in 512 graphs 974 / 972 / 951 (983), 1,048,576 1583 / 1570 / 1534 (1575).
+constexpr size_t kSmallSort = 1u << 17;
+
+static SortShape sort_shape(size_t n) {
+  if (n <= kSmallSort) return {kSortThreads, 2};
+  return {kSortThreads, 8};
+}
+
+static size_t sort_tiles(size_t n) {
+  const size_t t = sort_shape(n).tile();
+  return (n + t - 1) / t;
+}
+
 size_t sort_state_entries(size_t n) {
-  const size_t tiles = (n + kSortTile - 1) / kSortTile;
-  // per pass: tiles * 256 status words; then the global counts (uint32) and
-  // the tickets, in 64-bit words
-  return (size_t)kSortPasses * 256 * (tiles ? tiles : 1) + kSortPasses * 128 + kSortPasses;
+  const size_t tiles = sort_tiles(n);
+  // per pass: tiles * 256 status words; then the global counts and the
+  // tickets (all 32 bits)
+  return (size_t)kSortPasses * (256 * (tiles ? tiles : 1) + 256 + 1);
 }
 
 // Exclusive scan of n uint32 (n <= 2^31); in == out allowed. total may be
@@ -349,29 +429,31 @@ void scan_exclusive(gvizCudaForce *h, const uint32_t *in, uint32_t *out,
 // The scatter's shared memory exceeds the default per-block budget: opted
 // into once per device, at handle creation (outside any stream capture).
 void sort_set_smem_limits() {
-  cudaFuncSetAttribute(k_radix_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)kScatterDyn);
+  cudaFuncSetAttribute(k_radix_onesweep<kSortThreads, 8>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)scatter_dyn(kSortThreads * 8));
 }
 
 void radix_sort_pairs(gvizCudaForce *h, uint64_t *keys, uint32_t *vals,
                       uint64_t *keysAlt, uint32_t *valsAlt, size_t n) {
   if (n <= 1) return;
-  const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
-  uint64_t *state = h->d_sortState;
-  const size_t statusWords = (size_t)kSortPasses * 256 * tiles;
-  uint32_t *ghist = reinterpret_cast<uint32_t *>(state + statusWords);
+  const SortShape shape = sort_shape(n);
+  const uint32_t tiles = (uint32_t)sort_tiles(n);
+  uint32_t *state = h->d_sortState;
+  uint32_t *ghist = state + (size_t)kSortPasses * 256 * tiles;
   uint32_t *tickets = ghist + kSortPasses * 256;
-  cudaMemsetAsync(state, 0, (statusWords + kSortPasses * 128 + kSortPasses) * sizeof(uint64_t),
-                  h->stream);
+  cudaMemsetAsync(state, 0, sort_state_entries(n) * sizeof(uint32_t), h->stream);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const uint32_t hb = std::min<uint32_t>(tiles * 4u, (uint32_t)(sms > 0 ? sms : 1) * 2u);
-  k_radix_hist0<<<hb, kSortThreads, 0, h->stream>>>(keys, (uint32_t)n, ghist);
+  k_radix_hist0<<<hb, kHistThreads, 0, h->stream>>>(keys, (uint32_t)n, ghist);
   uint64_t *ka = keys, *kb = keysAlt;
   uint32_t *va = vals, *vb = valsAlt;
   for (int pass = 0; pass < kSortPasses; pass++) {
-    k_radix_onesweep<<<tiles, kSortThreads, kScatterDyn, h->stream>>>(
+    const auto kernel =
+        shape.rounds == 2 ? k_radix_onesweep<kSortThreads, 2> : k_radix_onesweep<kSortThreads, 8>;
+    kernel<<<tiles, shape.threads, scatter_dyn(shape.tile()), h->stream>>>(
         ka, va, kb, vb, (uint32_t)n, pass, ghist, state + (size_t)pass * 256 * tiles,
         tickets + pass, h->d_status);
     std::swap(ka, kb);
