@@ -740,7 +740,6 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     h->exactSplits = exact_splits(V, sms);
-    if (h->exactSplits > 1) rc |= dalloc(h, &h->d_exactPartial, (size_t)h->exactSplits * V);
   }
   rc |= dalloc(h, &h->d_leafDepth, Vs);
   rc |= dalloc(h, &h->d_counters, 8);
@@ -892,6 +891,12 @@ int gvizCudaForceSetParams(gvizCudaForce *h, const gvizCudaForceParams *p) {
       (p->farHubTargets > 0 && !(p->farHubTheta > 0.0 && p->farHubTheta < INFINITY)))
     return set_err(h, GVIZ_CUDA_ERR_ARG);
   DeviceGuard guard(h->device);
+  // only the exact mode needs the split sums
+  if (!p->barnesHutEnabled && p->precision == GVIZ_CUDA_FP32 && h->exactSplits > 1 &&
+      !h->d_exactPartial) {
+    const int rc = dalloc(h, &h->d_exactPartial, (size_t)h->exactSplits * h->V);
+    if (rc) return rc;
+  }
   const uint32_t hubs = (uint32_t)std::min<size_t>((size_t)p->farHubTargets, h->V);
   if (hubs != h->nFarHubs) {
     const int rc = select_hubs(h, hubs);

@@ -47,6 +47,35 @@ __device__ __forceinline__ float rcp_approx_ftz(float x) {
   return r;
 }
 
+// Two FP32 values in one 64-bit register for the packed add, multiply and
+// fused multiply-add (add/mul/fma.rn.f32x2): each half rounds exactly as the
+// scalar instruction does, at half the instructions.
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 constexpr int kExactThreads = 128;
 constexpr int kExactTile = 128;
 constexpr int kExactTpt = 4;     // exact mode: targets per thread
@@ -1501,9 +1530,12 @@ struct ExactArgs {
 // range order.
 template <int MODEL, bool OVERLAP>
 __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
-  __shared__ float4 sp[kExactTile];
+  // a source's coordinates twice each, as the packed pairs of two targets
+  // take them: {x, x, y, y} high parts, then low parts
+  __shared__ ulonglong2 sph[kExactTile], spl[kExactTile];
   __shared__ float2 sm[kExactTile];
-  __shared__ float sw[kExactTile];  // the source's share of the optimistic term's numerator
+  // minus the source's share of the optimistic term's numerator, twice
+  __shared__ f32x2 sw[kExactTile];
   __shared__ uint32_t sRange[2];
   uint32_t v[kExactTpt], gb[kExactTpt], ge[kExactTpt];
   bool act[kExactTpt];
@@ -1538,6 +1570,15 @@ __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
     }
   }
   __syncthreads();
+  // minus the targets' coordinates, two targets to a pair
+  f32x2 nxh[kExactTpt / 2], nxl[kExactTpt / 2], nyh[kExactTpt / 2], nyl[kExactTpt / 2];
+#pragma unroll
+  for (int k = 0; k < kExactTpt / 2; k++) {
+    nxh[k] = pack2(-vxh[2 * k], -vxh[2 * k + 1]);
+    nxl[k] = pack2(-vxl[2 * k], -vxl[2 * k + 1]);
+    nyh[k] = pack2(-vyh[2 * k], -vyh[2 * k + 1]);
+    nyl[k] = pack2(-vyl[2 * k], -vyl[2 * k + 1]);
+  }
   const uint32_t lo = sRange[0], hi = sRange[1];
   // this block's source range: whole tiles, split blockIdx.y of gridDim.y
   const uint32_t nTile = hi > lo ? (hi - lo + kExactTile - 1) / kExactTile : 0u;
@@ -1552,10 +1593,12 @@ __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
       float4 f;
       ds_split(q.x, f.x, f.z);
       ds_split(q.y, f.y, f.w);
-      sp[threadIdx.x] = f;
+      sph[threadIdx.x] = make_ulonglong2(pack2(f.x, f.x), pack2(f.y, f.y));
+      spl[threadIdx.x] = make_ulonglong2(pack2(f.z, f.z), pack2(f.w, f.w));
       const float m = a.massF[j];
       sm[threadIdx.x] = make_float2(m, OVERLAP ? a.radiusF[j] : 0.f);
-      sw[threadIdx.x] = MODEL == GVIZ_CUDA_MODEL_FR ? a.num * truncf(m) : m;
+      const float w = MODEL == GVIZ_CUDA_MODEL_FR ? a.num * truncf(m) : m;
+      sw[threadIdx.x] = pack2(-w, -w);
     }
     __syncthreads();
     const uint32_t cnt = min((uint32_t)kExactTile, hi - t0);
@@ -1580,19 +1623,33 @@ __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
         // the self pair, a coincident point (d2 == 0) or a d2 below the
         // normal range (flushed to zero) gives an infinite term, so the
         // chunk's partial is not finite and the chunk is summed again on
-        // the guarded path below.
+        // the guarded path below. Two targets share each packed instruction:
+        // 5.5 FP32 instructions and one reciprocal per pair instead of 11
+        // and one. The FP32 pipe (11 lane operations per pair, 1.27 ms for
+        // 65,536 vertices) then bounds the loop, not its issue slots: 1.78 ms
+        // against 2.28 with scalar instructions and four blocks per SM.
+        f32x2 qx[kExactTpt / 2], qy[kExactTpt / 2];
+#pragma unroll
+        for (int k = 0; k < kExactTpt / 2; k++) qx[k] = qy[k] = 0ull;
 #pragma unroll 4
         for (uint32_t q = c0; q < c1; q++) {
-          const float4 f = sp[q];
-          const float w = sw[q];
+          const ulonglong2 fh = sph[q], fl = spl[q];
+          const f32x2 w = sw[q];
 #pragma unroll
-          for (int k = 0; k < kExactTpt; k++) {
-            const float dx = (f.x - vxh[k]) + (f.z - vxl[k]);
-            const float dy = (f.y - vyh[k]) + (f.w - vyl[k]);
-            const float sc = w * rcp_approx_ftz(dx * dx + dy * dy);
-            px[k] = fmaf(-sc, dx, px[k]);
-            py[k] = fmaf(-sc, dy, py[k]);
+          for (int k = 0; k < kExactTpt / 2; k++) {
+            const f32x2 dx = add2(add2(fh.x, nxh[k]), add2(fl.x, nxl[k]));
+            const f32x2 dy = add2(add2(fh.y, nyh[k]), add2(fl.y, nyl[k]));
+            float d0, d1;
+            unpack2(fma2(dx, dx, mul2(dy, dy)), d0, d1);
+            const f32x2 sc = mul2(w, pack2(rcp_approx_ftz(d0), rcp_approx_ftz(d1)));
+            qx[k] = fma2(sc, dx, qx[k]);
+            qy[k] = fma2(sc, dy, qy[k]);
           }
+        }
+#pragma unroll
+        for (int k = 0; k < kExactTpt / 2; k++) {
+          unpack2(qx[k], px[2 * k], px[2 * k + 1]);
+          unpack2(qy[k], py[2 * k], py[2 * k + 1]);
         }
         // LinLog's target mass is common to the chunk's terms: one multiply
         // per chunk instead of one per pair
@@ -1618,7 +1675,11 @@ __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
         // coincident point through the deterministic direction; with
         // overlap the term of include/core/gvizVec.h:404-428 / 552-578
         for (uint32_t q = c0; q < c1; q++) {
-          const float4 f = sp[q];
+          float4 f;
+          unpack2(sph[q].x, f.x, f.x);
+          unpack2(sph[q].y, f.y, f.y);
+          unpack2(spl[q].x, f.z, f.z);
+          unpack2(spl[q].y, f.w, f.w);
           const float2 m = sm[q];
           const uint32_t jj = t0 + q;
           float dx[kExactTpt], dy[kExactTpt], d2[kExactTpt];
@@ -2001,12 +2062,15 @@ void enqueue_walk_f32(gvizCudaForce *h, uint64_t *counters) {
 }
 
 // Source ranges of the exact FP32 kernel for V vertices on a GPU of `sms`
-// SMs: enough blocks for about four waves, at least four tiles per range.
+// SMs: 28 blocks per SM where the tiles allow, four waves of the seven that
+// are resident, so that a last wave costs little (ER 65,536: 1.88 / 1.84 /
+// 1.78 ms at 8 / 16 / 28 blocks per SM, 2.25 at 4); at least one tile per
+// range, at most 32 ranges (the partial sums take 16 B per range and vertex).
 uint32_t exact_splits(size_t V, int sms) {
   const size_t tb = (V + kExactThreads * kExactTpt - 1) / (kExactThreads * kExactTpt);
   if (tb == 0) return 1;
-  size_t s = (4 * (size_t)(sms > 0 ? sms : 1) + tb - 1) / tb;
-  s = std::min<size_t>(s, (V + 4 * kExactTile - 1) / (4 * kExactTile));
+  size_t s = (28 * (size_t)(sms > 0 ? sms : 1) + tb - 1) / tb;
+  s = std::min<size_t>(s, (V + kExactTile - 1) / kExactTile);
   return (uint32_t)std::max<size_t>(1, std::min<size_t>(s, 32));
 }
 
