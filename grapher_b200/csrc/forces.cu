@@ -303,26 +303,44 @@ __device__ __forceinline__ void rep_term_apart(float dx, float dy, float d2, flo
 // pushes its children (slots from the tree build's child records) with the
 // lanes that opened it. A push that would overflow the stack is walked in
 // place with the stackless union walk below (the same decisions).
+// Issue slots bound the walk (DRAM at 8 %), so the loop over a round's nodes is
+// what counts: the loading lane prepares each record (plain_put_record), the
+// loop then takes about 20 instructions per node instead of 33. With it the
+// walk takes 63.5 us instead of 127 at 65,537 vertices (LinLog, theta 0.5),
+// 651 instead of 923 at 1,048,576 (theta 0.8, overlap prevention) and 254
+// instead of 441 over 512 graphs (0.75M vertices, FR, theta 0.7). Unrolling
+// the loop by 4 / 2 / 1: 72 / 93 / 84 us at 65,537.
 constexpr int kPlainStack = 512;  // largest stack: pending (node, lanes) entries per warp
+// The stack without a caller's or the autotuner's choice. Half the largest
+// leaves the SM more L1 for node records, and few walks fill it: the walk
+// takes 65.6 / 63.5 / 96.3 us at 65,537 vertices with 512 / 256 / 128 entries,
+// 696 / 651 / 637 us at 1,048,576 with overlap prevention, 260 / 254 / 252 us
+// over 512 graphs.
+constexpr int kPlainStackDefault = 256;
 
 // A warp's region of the plain walk's dynamic shared memory: the round's 32
 // node records (1 KiB), then a stack of stackCap entries; the region's
 // size follows the stack cap, so a smaller stack leaves room for more
 // resident warps.
+struct __align__(16) PlainRecord {
+  ulonglong2 h;
+  float4 m;
+};
+
 struct PlainWarpSmem {
-  float4 (*rec)[2];  // the round's node records
+  PlainRecord *rec;  // the round's node records
   uint2 *st;         // pending entries: node, lanes
 };
 
 __host__ __device__ constexpr uint32_t plain_warp_bytes(uint32_t cap) {
-  return 32u * 2u * 16u + ((cap * 8u + 15u) & ~15u);
+  return 32u * (uint32_t)sizeof(PlainRecord) + ((cap * 8u + 15u) & ~15u);
 }
 
 __device__ __forceinline__ PlainWarpSmem plain_warp_smem(unsigned char *dyn, uint32_t cap) {
   unsigned char *base = dyn + (size_t)(threadIdx.x >> 5) * plain_warp_bytes(cap);
   PlainWarpSmem q;
-  q.rec = reinterpret_cast<float4(*)[2]>(base);
-  q.st = reinterpret_cast<uint2 *>(base + 32 * 2 * 16);
+  q.rec = reinterpret_cast<PlainRecord *>(base);
+  q.st = reinterpret_cast<uint2 *>(base + 32 * sizeof(PlainRecord));
   return q;
 }
 
@@ -330,6 +348,7 @@ struct PlainTarget {
   uint32_t v;
   bool act;
   float vxh, vxl, vyh, vyl, mv, rv;
+  f32x2 nh, nl;  // minus the position: {x, y} high parts, low parts
 };
 
 // The reference's decision for one node and this lane's target: adds the
@@ -368,29 +387,77 @@ __device__ __forceinline__ bool plain_visit(const WalkArgs &a, const PlainTarget
   return in && massOk && !isLeaf && !accept;
 }
 
-// plain_visit without the coincidence vote: the term of a point or accepted
-// cell on the straight-line path (a coincident point gives a term that is
-// not finite; the caller then redoes the round with plain_visit).
+// A round's record of one node, made by the lane that loaded it, for the
+// round's loop over nodes. The test size of a point is below every squared
+// distance, so one comparison tells the nodes whose term is taken from the
+// cells to open; a massless node keeps no lanes.
+//   h: {x, y} high parts, low parts (packed pairs)
+//   m: mass (without overlap prevention FR's is truncated,
+//      src/embedders/gvizForceModel.c:20), test size, vertex (-1: cell), and
+//      the lanes whose walks reach the node, or its radius with overlap
+//      prevention
 template <int MODEL, bool OVERLAP>
-__device__ __forceinline__ bool plain_visit_fast(const WalkArgs &a, const PlainTarget &t, bool in,
-                                                 float4 n0, float4 n1, float &px, float &py) {
-  const float nmass = n1.x, nsize = n1.y;
-  const int32_t ninfo = __float_as_int(n1.w);
-  const float dx = (n0.x - t.vxh) + (n0.z - t.vxl);
-  const float dy = (n0.y - t.vyh) + (n0.w - t.vyl);
+__device__ __forceinline__ void plain_put_record(PlainRecord &r, float4 n0, float4 n1,
+                                                 uint32_t lanes) {
+  const bool leaf = __float_as_int(n1.w) >= 0;
+  r.h = make_ulonglong2(pack2(n0.x, n0.y), pack2(n0.z, n0.w));
+  r.m = make_float4(OVERLAP || MODEL != GVIZ_CUDA_MODEL_FR ? n1.x : truncf(n1.x),
+                    leaf ? -1.0f : n1.y, n1.w,
+                    OVERLAP ? (leaf ? n1.y : 0.0f) : __uint_as_float(lanes));
+}
+
+// One node of a round for this lane's target: adds the term of a point or an
+// accepted cell; returns true when the cell is opened. The term runs
+// straight-line on one approximate reciprocal, whose product with the
+// numerator is __fdividef's quotient wherever the squared distance is a
+// normal number; a coincident point, or a squared distance below that range,
+// gives a sum that is not finite, and the round's terms are then taken again
+// by plain_guarded.
+template <int MODEL, bool OVERLAP>
+__device__ __forceinline__ bool plain_node(const WalkArgs &a, const PlainTarget &t,
+                                           const PlainRecord &r, uint32_t lanes, uint32_t bit,
+                                           float &px, float &py) {
+  float dx, dy;
+  unpack2(add2(add2(r.h.x, t.nh), add2(r.h.y, t.nl)), dx, dy);
+  const float4 m = r.m;
   const float d2 = dx * dx + dy * dy;
-  const bool isLeaf = ninfo >= 0;
-  const bool massOk = nmass != 0.0f;
-  const bool accept = !isLeaf && nsize < d2;
-  const bool doForce = in && massOk && (isLeaf ? ((uint32_t)ninfo != t.v) : accept);
-  if (doForce) {
-    float fx, fy;
-    rep_term_apart<MODEL, OVERLAP>(dx, dy, d2, t.mv, nmass, t.rv + (isLeaf ? nsize : 0.0f),
-                                   a.num, a.overlapC, fx, fy);
-    px += fx;
-    py += fy;
+  const bool in = ((OVERLAP ? lanes : __float_as_uint(m.w)) & bit) != 0u;
+  const bool take = m.y < d2;
+  if (in && take && (uint32_t)__float_as_int(m.z) != t.v) {
+    if (OVERLAP) {
+      float fx, fy;
+      rep_term_apart<MODEL, true>(dx, dy, d2, t.mv, m.x, t.rv + m.w, a.num, a.overlapC, fx, fy);
+      px += fx;
+      py += fy;
+    } else {
+      const float r1 = rcp_approx_ftz(d2);
+      const float s = MODEL == GVIZ_CUDA_MODEL_FR ? (a.num * r1) * m.x : (t.mv * m.x) * r1;
+      px += __fmul_rn(-s, dx);  // never fused into the sum
+      py += __fmul_rn(-s, dy);
+    }
   }
-  return in && massOk && !isLeaf && !accept;
+  return in && !take;
+}
+
+// The term of plain_node for any distance.
+template <int MODEL, bool OVERLAP>
+__device__ __forceinline__ void plain_guarded(const WalkArgs &a, const PlainTarget &t,
+                                              const PlainRecord &r, uint32_t lanes, uint32_t bit,
+                                              float &px, float &py) {
+  float dx, dy;
+  unpack2(add2(add2(r.h.x, t.nh), add2(r.h.y, t.nl)), dx, dy);
+  const float4 m = r.m;
+  const float d2 = dx * dx + dy * dy;
+  const bool in = ((OVERLAP ? lanes : __float_as_uint(m.w)) & bit) != 0u;
+  const int32_t info = __float_as_int(m.z);
+  if (!(in && m.y < d2 && (uint32_t)info != t.v)) return;
+  const uint32_t other = info >= 0 ? (uint32_t)info : t.v;
+  // (the truncated mass of FR's record stays as it is when truncated again)
+  float fx, fy;
+  rep_term<MODEL, OVERLAP>(dx, dy, d2, t.mv, m.x, t.rv + (OVERLAP ? m.w : 0.0f), a.num,
+                           a.overlapC, t.v, other, fx, fy);
+  px += fx;
+  py += fy;
 }
 
 // The stackless union walk of the preorder range [lo, hi) for the lanes in
@@ -437,13 +504,11 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
   const bool valid = lane < tk.y && s < a.V;
   PlainTarget t;
   t.v = valid ? a.idx[s] : 0u;
-  const uint32_t g = (valid && a.gid) ? a.gid[t.v] : 0u;
+  const uint32_t g =
+      a.gid ? __shfl_sync(0xffffffffu, valid ? a.gid[t.v] : 0u, 0) : 0u;  // the task's graph
   t.act = valid && (a.active == nullptr || a.active[g] != 0u);
-  uint32_t root = 0, myEnd = 0;
-  if (t.act) {
-    root = a.graphBase[g];
-    myEnd = min(root + a.rootT[g], a.maxNodes);
-  }
+  const uint32_t root = a.graphBase[g];
+  const uint32_t end = min(root + a.rootT[g], a.maxNodes);
   t.vxh = t.vxl = t.vyh = t.vyl = t.mv = t.rv = 0.f;
   if (t.act) {
     const double2 p = a.pos[t.v];
@@ -452,15 +517,15 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
     t.mv = a.massF[t.v];
     if (OVERLAP) t.rv = a.radiusF[t.v];
   }
+  t.nh = pack2(-t.vxh, -t.vyh);
+  t.nl = pack2(-t.vxl, -t.vyl);
+  const uint32_t bit = 1u << lane;
   Kahan kx, ky;
   unsigned long long nInter = 0, nVisit = 0, nSerial = 0;
-  // the first entries: each distinct root among the lanes, with its lanes
-  const uint32_t key = (t.act && root < myEnd) ? root : kInf;
-  const uint32_t same = __match_any_sync(0xffffffffu, key);
-  const bool leader = key != kInf && (uint32_t)(__ffs(same) - 1) == lane;
-  const uint32_t bl = __ballot_sync(0xffffffffu, leader);
-  if (leader) q.st[__popc(bl & below)] = make_uint2(root, same);
-  uint32_t top = __popc(bl);
+  // the first entry: the root, with every active lane
+  const uint32_t all = __ballot_sync(0xffffffffu, t.act);
+  uint32_t top = all != 0u && root < end ? 1u : 0u;
+  if (lane == 0u) q.st[0] = make_uint2(root, all);
   __syncwarp();
   while (top > 0u) {
     const uint32_t n = min(top, 32u);
@@ -474,43 +539,47 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
       n1 = __ldg(reinterpret_cast<const float4 *>(a.nodes + e.x) + 1);
       kd = __ldg(a.kids + e.x);  // read for every node; used only when it is opened
     }
-    // the graph's end for the entry's lanes (they share one graph)
-    const uint32_t entryEnd = __shfl_sync(0xffffffffu, myEnd, mine ? __ffs(e.y) - 1 : 0);
     __syncwarp();  // popped, and last round's records read, before the writes below
-    if (mine) {
-      q.rec[lane][0] = n0;
-      q.rec[lane][1] = n1;
-    }
+    const uint32_t reach = n1.x != 0.0f ? e.y : 0u;  // no lane takes a massless node
+    if (mine) plain_put_record<MODEL, OVERLAP>(q.rec[lane], n0, n1, reach);
     __syncwarp();
     if (COUNT) nVisit += n;
     // the round's terms in a plain FP32 partial, which then joins the
     // target's Kahan-compensated sum (cascade summation, <= 32 terms a run)
     uint32_t myOpen = 0;
     float px = 0.f, py = 0.f;
-    if (COUNT) {  // instrumented: the guarded visits, counting terms
+    if (COUNT) {  // instrumented: the vote-guarded visits, counting terms
       for (uint32_t j = 0; j < n; j++) {
-        const uint32_t lanes = __shfl_sync(0xffffffffu, e.y, j);
-        const bool open = plain_visit<MODEL, OVERLAP>(a, t, (lanes >> lane) & 1u, q.rec[j][0],
-                                                      q.rec[j][1], px, py, nInter);
+        const uint32_t lanes = __shfl_sync(0xffffffffu, reach, j);
+        float4 m0, m1;
+        m0.x = __shfl_sync(0xffffffffu, n0.x, j);
+        m0.y = __shfl_sync(0xffffffffu, n0.y, j);
+        m0.z = __shfl_sync(0xffffffffu, n0.z, j);
+        m0.w = __shfl_sync(0xffffffffu, n0.w, j);
+        m1.x = __shfl_sync(0xffffffffu, n1.x, j);
+        m1.y = __shfl_sync(0xffffffffu, n1.y, j);
+        m1.z = __shfl_sync(0xffffffffu, n1.z, j);
+        m1.w = __shfl_sync(0xffffffffu, n1.w, j);
+        const bool open =
+            plain_visit<MODEL, OVERLAP>(a, t, (lanes & bit) != 0u, m0, m1, px, py, nInter);
         const uint32_t ob = __ballot_sync(0xffffffffu, open);
         if (lane == j) myOpen = ob;
       }
     } else {
+#pragma unroll 4
       for (uint32_t j = 0; j < n; j++) {
-        const uint32_t lanes = __shfl_sync(0xffffffffu, e.y, j);
-        const bool open = plain_visit_fast<MODEL, OVERLAP>(a, t, (lanes >> lane) & 1u, q.rec[j][0],
-                                                           q.rec[j][1], px, py);
+        const uint32_t lanes = OVERLAP ? __shfl_sync(0xffffffffu, reach, j) : 0u;
+        const bool open = plain_node<MODEL, OVERLAP>(a, t, q.rec[j], lanes, bit, px, py);
         const uint32_t ob = __ballot_sync(0xffffffffu, open);
         if (lane == j) myOpen = ob;
       }
-      // a coincident point in the round: the round again on the guarded path
+      // a coincident point in the round: its terms again on the guarded path
       // (the same decisions; the open masks above stand)
       if (__any_sync(0xffffffffu, !(isfinite(px) && isfinite(py)))) {
         px = py = 0.f;
         for (uint32_t j = 0; j < n; j++) {
-          const uint32_t lanes = __shfl_sync(0xffffffffu, e.y, j);
-          plain_visit<MODEL, OVERLAP>(a, t, (lanes >> lane) & 1u, q.rec[j][0], q.rec[j][1], px,
-                                      py, nInter);
+          const uint32_t lanes = OVERLAP ? __shfl_sync(0xffffffffu, reach, j) : 0u;
+          plain_guarded<MODEL, OVERLAP>(a, t, q.rec[j], lanes, bit, px, py);
         }
       }
     }
@@ -519,15 +588,16 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
     // opened nodes push their children (inside the graph's subtree) with the
     // lanes that opened them, in lane order, while they fit
     uint32_t nk = 0;
+    if (__float_as_int(n1.w) >= 0) myOpen = 0u;  // a point opens for no target, NaN or not
     if (myOpen) {
       if (kd.y == GVIZ_KIDS_RUN) {
-        nk = (kd.x > e.x && kd.x < entryEnd) ? min(kd.z, entryEnd - kd.x) : 0u;
+        nk = (kd.x > e.x && kd.x < end) ? min(kd.z, end - kd.x) : 0u;
         nk = min(nk, a.stackCap + 1u);  // a longer run never fits
       } else {
-        kd.x = (kd.x > e.x && kd.x < entryEnd) ? kd.x : GVIZ_NONE;
-        kd.y = (kd.y > e.x && kd.y < entryEnd) ? kd.y : GVIZ_NONE;
-        kd.z = (kd.z > e.x && kd.z < entryEnd) ? kd.z : GVIZ_NONE;
-        kd.w = (kd.w > e.x && kd.w < entryEnd) ? kd.w : GVIZ_NONE;
+        kd.x = (kd.x > e.x && kd.x < end) ? kd.x : GVIZ_NONE;
+        kd.y = (kd.y > e.x && kd.y < end) ? kd.y : GVIZ_NONE;
+        kd.z = (kd.z > e.x && kd.z < end) ? kd.z : GVIZ_NONE;
+        kd.w = (kd.w > e.x && kd.w < end) ? kd.w : GVIZ_NONE;
         nk = (uint32_t)(kd.x != GVIZ_NONE) + (uint32_t)(kd.y != GVIZ_NONE) +
              (uint32_t)(kd.z != GVIZ_NONE) + (uint32_t)(kd.w != GVIZ_NONE);
       }
@@ -561,7 +631,7 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
       const uint32_t lanes = __shfl_sync(0xffffffffu, myOpen, l);
       const uint32_t lo = __shfl_sync(0xffffffffu, e.x, l) + 1u;
       const uint32_t hi = __shfl_sync(
-          0xffffffffu, min(max((uint32_t)__float_as_int(n1.z), e.x + 1u), entryEnd), l);
+          0xffffffffu, min(max((uint32_t)__float_as_int(n1.z), e.x + 1u), end), l);
       plain_walk_range<MODEL, OVERLAP>(a, t, lanes, lo, hi, kx, ky, nInter, nVisit);
     }
     __syncwarp();
@@ -580,7 +650,7 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
 
 // Static schedule: warp w of the grid takes task w.
 template <int MODEL, bool OVERLAP, bool COUNT>
-__global__ __launch_bounds__(kWalkMaxThreads) void k_walk_f32(WalkArgs a) {
+__global__ __launch_bounds__(kWalkMaxThreads, 2) void k_walk_f32(WalkArgs a) {
   extern __shared__ __align__(16) unsigned char plainDyn[];
   const PlainWarpSmem q = plain_warp_smem(plainDyn, a.stackCap);
   const uint32_t task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -592,7 +662,7 @@ __global__ __launch_bounds__(kWalkMaxThreads) void k_walk_f32(WalkArgs a) {
 // the next task from a device counter (reset before every launch) until
 // the queue is empty, so warps that drew cheap tasks take more of them.
 template <int MODEL, bool OVERLAP, bool COUNT>
-__global__ __launch_bounds__(kWalkMaxThreads) void k_walk_f32_queue(WalkArgs a) {
+__global__ __launch_bounds__(kWalkMaxThreads, 2) void k_walk_f32_queue(WalkArgs a) {
   extern __shared__ __align__(16) unsigned char plainDyn[];
   const PlainWarpSmem q = plain_warp_smem(plainDyn, a.stackCap);
   for (;;) {
@@ -1802,10 +1872,10 @@ void enqueue_attraction_f32(gvizCudaForce *h) {
 }
 
 // the plain walk's stack entries per warp on this handle: the caller's cap
-// (gvizCudaForceSetWalkStackCap), else the autotuner's pick, else all 512
+// (gvizCudaForceSetWalkStackCap), else the autotuner's pick, else the default
 uint32_t plain_cap(const gvizCudaForce *h) {
   const uint32_t c = h->walkStackCap ? h->walkStackCap : h->walkTunedCap;
-  return (c >= 32 && c <= (uint32_t)kPlainStack) ? c : (uint32_t)kPlainStack;
+  return (c >= 32 && c <= (uint32_t)kPlainStack) ? c : (uint32_t)kPlainStackDefault;
 }
 
 // dynamic shared memory of the plain walk: one warp region per warp

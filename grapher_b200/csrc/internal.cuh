@@ -153,8 +153,8 @@ struct gvizCudaForce {
   uint32_t walkThreads = 0;
   bool walkPersistent = false;
   uint32_t walkResident = 0;
-  uint32_t walkStackCap = 0;  // FP32 walks: stack entries per warp (0: all)
-  uint32_t walkTunedCap = 0;  // plain walk: the autotuner's stack entries (0: all)
+  uint32_t walkStackCap = 0;  // FP32 walks: the caller's stack entries per warp (0: not set)
+  uint32_t walkTunedCap = 0;  // plain walk: the autotuner's stack entries (0: not tuned)
   ChunkStat *d_chunkStat = nullptr;
   uint32_t *d_status = nullptr;
 

@@ -332,8 +332,8 @@ class ForceLayout:
 
     def set_walk_stack_cap(self, entries):
         """Stack entries per warp of the FP32 walks, plain and learned
-        (32..512; 0 restores the default: the autotuner's pick for the plain
-        walk, else 512): forces agree up to the order of the per-target sums."""
+        (32..512; 0 restores the default: 512 in the learned walk, the
+        autotuner's pick or 256 in the plain one): forces agree up to the order of the per-target sums."""
         N.check(self.L.gvizCudaForceSetWalkStackCap(self.h, entries),
                 "gvizCudaForceSetWalkStackCap")
 

@@ -493,7 +493,7 @@ int gvizCudaForceFarJudgeStatus(const gvizCudaForce *h, uint64_t *checks, double
  * memory (512 entries); an opened cell whose children do not fit is walked
  * in place with the stackless preorder walk instead (the same decisions).
  * Sets the stack entries the walks may use, 32 to 512 (0 restores the
- * default: the autotuner's pick for the plain walk, else 512);
+ * default: the autotuner's pick for the plain walk, else the above);
  * forces agree up to the order of the per-target sums. A tuning and test
  * knob. No reference counterpart. */
 int gvizCudaForceSetWalkStackCap(gvizCudaForce *h, uint32_t entries);
