@@ -980,6 +980,12 @@ __global__ __launch_bounds__(kFarThreads, 5) void k_walk_f32_far(FarArgs fa) {
 // stackless preorder loop (same decisions, same lists). The order in which
 // terms are summed depends only on the group, so the result does not
 // depend on which warp drew it. Per-target sums are Kahan-compensated.
+// Bound by issue: a group of ~22 targets takes ~140 terms per target and six
+// network tiles. The list loops run straight-line (a sum that is not finite
+// takes its list again, guarded) and are unrolled by four: 683 us at
+// 1,048,576 vertices (LinLog, theta 1.225), 838 with a coincidence vote per
+// term; unrolled by 1 / 2 / 8: 726 / 694 / 683 (178 us at 262,144 vertices by
+// four, 183 by eight). Four blocks per SM (64 registers): 783.
 // The lists are at most 63 points and 47 cells: a round adds at most 32 of
 // each, and a round runs only while fewer than 32 points and 16 cells wait.
 // ---------------------------------------------------------------------------
@@ -992,11 +998,11 @@ constexpr int kCellBlocksPerSM = 3;
 // per warp: the point and cell lists (double-single positions), the MLP
 // tile's rows and outputs, the group's targets and the pending nodes
 struct __align__(16) CellWarpSmem {
-  float4 pPos[kCellRing];  // point: x hi, y hi, x lo, y lo
-  float2 pMR[kCellRing];   // point: mass, radius
-  uint32_t pV[kCellRing];  // point: vertex
-  float4 cPos[kCellRing];  // cell: centre of mass, double-single
-  float2 cMN[kCellRing];   // cell: mass, preorder slot (bits)
+  ulonglong2 pPos[kCellRing];  // point: {x, y} high parts, low parts
+  float2 pMV[kCellRing];       // point: mass (cell_mass), vertex (bits)
+  float pR[kCellRing];         // point: radius (overlap prevention only)
+  ulonglong2 cPos[kCellRing];  // cell: centre of mass, likewise
+  float2 cMN[kCellRing];       // cell: mass (cell_mass), preorder slot (bits)
   __nv_bfloat16 gx[kFarTile * MLP_XS];
   float2 out[kFarTile];
   uint32_t tgt[32];
@@ -1029,7 +1035,8 @@ __device__ __forceinline__ float warp_maxf(float x) {
 struct CellTarget {
   uint32_t v;
   bool has;
-  float vxh, vxl, vyh, vyl, mv, rv;
+  float mv, rv;
+  f32x2 nh, nl;  // minus the position: {x, y} high parts, low parts
 };
 
 struct CellGroup {
@@ -1045,42 +1052,114 @@ struct CellSums {
   unsigned long long nInter = 0, nRows = 0;  // instrumentation only
 };
 
+// The mass a list keeps: FR's terms take it truncated
+// (src/embedders/gvizForceModel.c:20), overlap prevention's truncate it
+// themselves.
+template <int MODEL, bool OVERLAP>
+__device__ __forceinline__ float cell_mass(float m) {
+  return OVERLAP || MODEL != GVIZ_CUDA_MODEL_FR ? m : truncf(m);
+}
+
+template <int MODEL, bool OVERLAP>
+__device__ __forceinline__ void put_point(CellWarpSmem &q, uint32_t e, float4 n0, float4 n1) {
+  q.pPos[e] = make_ulonglong2(pack2(n0.x, n0.y), pack2(n0.z, n0.w));
+  q.pMV[e] = make_float2(cell_mass<MODEL, OVERLAP>(n1.x), n1.w);
+  if (OVERLAP) q.pR[e] = n1.y;
+}
+
+template <int MODEL, bool OVERLAP>
+__device__ __forceinline__ void put_accepted(CellWarpSmem &q, uint32_t e, float4 n0, float4 n1,
+                                             uint32_t node) {
+  q.cPos[e] = make_ulonglong2(pack2(n0.x, n0.y), pack2(n0.z, n0.w));
+  q.cMN[e] = make_float2(cell_mass<MODEL, OVERLAP>(n1.x), __uint_as_float(node));
+}
+
+// The term of a listed point or cell for this lane's target. GUARDED: any
+// distance; otherwise straight-line on one approximate reciprocal, the same
+// value wherever the squared distance is a normal number, and not finite
+// where it is zero or below that range.
+template <int MODEL, bool OVERLAP, bool GUARDED>
+__device__ __forceinline__ void cell_term(const WalkArgs &a, const CellTarget &t, ulonglong2 pos,
+                                          float m, float radius, uint32_t other, float &fx,
+                                          float &fy) {
+  float dx, dy;
+  unpack2(add2(add2(pos.x, t.nh), add2(pos.y, t.nl)), dx, dy);
+  const float d2 = dx * dx + dy * dy;
+  if (GUARDED) {
+    rep_term<MODEL, OVERLAP>(dx, dy, d2, t.mv, m, t.rv + radius, a.num, a.overlapC, t.v, other,
+                             fx, fy);
+  } else if (OVERLAP) {
+    rep_term_apart<MODEL, true>(dx, dy, d2, t.mv, m, t.rv + radius, a.num, a.overlapC, fx, fy);
+  } else {
+    const float r1 = rcp_approx_ftz(d2);
+    const float s = MODEL == GVIZ_CUDA_MODEL_FR ? (a.num * r1) * m : (t.mv * m) * r1;
+    fx = __fmul_rn(-s, dx);  // never fused into the sums
+    fy = __fmul_rn(-s, dy);
+  }
+}
+
 // Every target takes the pair term of the first k listed points (at most
 // 32, summed in a plain FP32 partial that then joins the target's
-// Kahan-compensated sum: cascade summation, as in the plain walk).
+// Kahan-compensated sum: cascade summation, as in the plain walk). The terms
+// are taken again on the guarded path when a sum is not finite (a
+// coincident point).
+template <int MODEL, bool OVERLAP, bool GUARDED>
+__device__ __forceinline__ void cell_point_terms(const WalkArgs &a, const CellWarpSmem &q,
+                                                 const CellTarget &t, const CellSums &s,
+                                                 uint32_t k, float &px, float &py) {
+  px = py = 0.f;
+#pragma unroll 4
+  for (uint32_t j = 0; j < k; j++) {
+    const uint32_t e = (s.ph + j) & (kCellRing - 1);
+    const float2 mv = q.pMV[e];
+    const uint32_t u = __float_as_uint(mv.y);
+    float fx, fy;
+    if (GUARDED && !(t.has && u != t.v)) continue;
+    cell_term<MODEL, OVERLAP, GUARDED>(a, t, q.pPos[e], mv.x, OVERLAP ? q.pR[e] : 0.f, u, fx, fy);
+    if (u != t.v) {
+      px += fx;
+      py += fy;
+    }
+  }
+}
+
 template <int MODEL, bool OVERLAP, bool COUNT>
 __device__ __forceinline__ void cell_eval_points(const WalkArgs &a, CellWarpSmem &q,
                                                  const CellTarget &t, CellSums &s, uint32_t k) {
   __syncwarp();
-  float px = 0.f, py = 0.f;
-#pragma unroll 1  // a compact loop: the walk is sensitive to instruction-cache misses
-  for (uint32_t j = 0; j < k; j++) {
-    const uint32_t e = (s.ph + j) & (kCellRing - 1);
-    const float4 p = q.pPos[e];
-    const float2 mr = q.pMR[e];
-    const uint32_t u = q.pV[e];
-    const float dx = (p.x - t.vxh) + (p.z - t.vxl);
-    const float dy = (p.y - t.vyh) + (p.w - t.vyl);
-    const float d2 = dx * dx + dy * dy;
-    const bool doForce = t.has && u != t.v;
-    float fx = 0.f, fy = 0.f;
-    if (__any_sync(0xffffffffu, doForce && !(d2 > 0.0f))) {  // coincident points: rare
-      if (doForce)
-        rep_term<MODEL, OVERLAP>(dx, dy, d2, t.mv, mr.x, t.rv + mr.y, a.num, a.overlapC, t.v,
-                                 u, fx, fy);
-    } else if (doForce) {
-      rep_term_apart<MODEL, OVERLAP>(dx, dy, d2, t.mv, mr.x, t.rv + mr.y, a.num, a.overlapC,
-                                     fx, fy);
-    }
-    px += fx;
-    py += fy;
-    if (COUNT && doForce) s.nInter++;
-  }
+  float px, py;
+  cell_point_terms<MODEL, OVERLAP, false>(a, q, t, s, k, px, py);
+  if (__any_sync(0xffffffffu, t.has && !(isfinite(px) && isfinite(py))))
+    cell_point_terms<MODEL, OVERLAP, true>(a, q, t, s, k, px, py);
+  if (COUNT && t.has)
+    for (uint32_t j = 0; j < k; j++)
+      s.nInter += __float_as_uint(q.pMV[(s.ph + j) & (kCellRing - 1)].y) != t.v ? 1ull : 0ull;
   s.kx.add(px);
   s.ky.add(py);
   s.ph = (s.ph + k) & (kCellRing - 1);
   s.pn -= k;
   __syncwarp();
+}
+
+// The monopole terms of the first k listed cells and the network's correction
+// of each.
+template <int MODEL, bool OVERLAP, bool GUARDED>
+__device__ __forceinline__ void cell_cell_terms(const WalkArgs &a, const CellWarpSmem &q,
+                                                const CellTarget &t, const CellSums &s, uint32_t k,
+                                                float &px, float &py, float &cx, float &cy) {
+  px = py = 0.f;
+  cx = s.corrx;
+  cy = s.corry;
+#pragma unroll 4
+  for (uint32_t r = 0; r < k; r++) {
+    const uint32_t e = (s.ch + r) & (kCellRing - 1);
+    float fx, fy;
+    if (GUARDED && !t.has) continue;
+    cell_term<MODEL, OVERLAP, GUARDED>(a, t, q.cPos[e], q.cMN[e].x, 0.f, t.v, fx, fy);
+    px += fx;
+    py += fy;
+    far_apply(q.out[r], make_float2(fx, fy), cx, cy);
+  }
 }
 
 // The first k <= 16 listed cells: lane r < k builds row r (cell r seen from
@@ -1096,7 +1175,9 @@ __device__ __forceinline__ void cell_eval_cells(const WalkArgs &a, const FarCell
   __syncwarp();
   if (lane < k) {
     const uint32_t e = (s.ch + lane) & (kCellRing - 1);
-    const float4 p = q.cPos[e];
+    float4 p;
+    unpack2(q.cPos[e].x, p.x, p.y);
+    unpack2(q.cPos[e].y, p.z, p.w);
     const uint32_t node = __float_as_uint(q.cMN[e].y);
     const float4 c0 = __ldg(reinterpret_cast<const float4 *>(cells + node));
     const uint4 c1 = __ldg(reinterpret_cast<const uint4 *>(cells + node) + 1);
@@ -1119,32 +1200,18 @@ __device__ __forceinline__ void cell_eval_cells(const WalkArgs &a, const FarCell
   __syncwarp();
   mlp_forward_tile<true>(W, q.gx, MLP_XS, reinterpret_cast<float *>(q.out));
   __syncwarp();
-  float px = 0.f, py = 0.f;
-#pragma unroll 1  // a compact loop: the walk is sensitive to instruction-cache misses
-  for (uint32_t r = 0; r < k; r++) {
-    const uint32_t e = (s.ch + r) & (kCellRing - 1);
-    const float4 p = q.cPos[e];
-    const float m = q.cMN[e].x;
-    const float dx = (p.x - t.vxh) + (p.z - t.vxl);
-    const float dy = (p.y - t.vyh) + (p.w - t.vyl);
-    const float d2 = dx * dx + dy * dy;
-    float fx = 0.f, fy = 0.f;
-    if (__any_sync(0xffffffffu, t.has && !(d2 > 0.0f))) {
-      if (t.has)
-        rep_term<MODEL, OVERLAP>(dx, dy, d2, t.mv, m, t.rv, a.num, a.overlapC, t.v, t.v, fx, fy);
-    } else if (t.has) {
-      rep_term_apart<MODEL, OVERLAP>(dx, dy, d2, t.mv, m, t.rv, a.num, a.overlapC, fx, fy);
-    }
-    px += fx;
-    py += fy;
-    if (t.has) {
-      far_apply(q.out[r], make_float2(fx, fy), s.corrx, s.corry);
-      if (COUNT) s.nInter++;
-    }
-  }
+  float px, py, cx, cy;
+  cell_cell_terms<MODEL, OVERLAP, false>(a, q, t, s, k, px, py, cx, cy);
+  if (__any_sync(0xffffffffu, t.has && !(isfinite(px) && isfinite(py))))
+    cell_cell_terms<MODEL, OVERLAP, true>(a, q, t, s, k, px, py, cx, cy);
+  s.corrx = cx;
+  s.corry = cy;
   s.kx.add(px);
   s.ky.add(py);
-  if (COUNT) s.nRows += k;
+  if (COUNT) {
+    s.nRows += k;
+    if (t.has) s.nInter += k;
+  }
   s.ch = (s.ch + k) & (kCellRing - 1);
   s.cn -= k;
   __syncwarp();
@@ -1211,23 +1278,26 @@ __global__ __launch_bounds__(kCellThreads, kCellBlocksPerSM) void k_walk_f32_cel
     if (a.active && a.active[gr] == 0u) continue;
     const uint32_t root = a.graphBase[gr];
     const uint32_t end = min(root + a.rootT[gr], a.maxNodes);
-    t.vxh = t.vxl = t.vyh = t.vyl = t.mv = t.rv = 0.f;
+    float vxh = 0.f, vxl = 0.f, vyh = 0.f, vyl = 0.f;
+    t.mv = t.rv = 0.f;
     double2 pv = make_double2(0.0, 0.0);
     if (t.has) {
       pv = a.pos[t.v];
-      ds_split(pv.x, t.vxh, t.vxl);
-      ds_split(pv.y, t.vyh, t.vyl);
+      ds_split(pv.x, vxh, vxl);
+      ds_split(pv.y, vyh, vyl);
       t.mv = a.massF[t.v];
       if (OVERLAP) t.rv = a.radiusF[t.v];
     }
+    t.nh = pack2(-vxh, -vyh);
+    t.nl = pack2(-vxl, -vyl);
     CellGroup g;
     float wr2;
-    group_centroid<32, OVERLAP>(t.has, pv, t.vxh, t.vxl, t.vyh, t.vyl, t.rv, g.wxh, g.wxl,
-                                g.wyh, g.wyl, wr2, g.wrv);
-    g.bx0 = warp_minf(t.has ? t.vxh : INFINITY);
-    g.bx1 = warp_maxf(t.has ? t.vxh : -INFINITY);
-    g.by0 = warp_minf(t.has ? t.vyh : INFINITY);
-    g.by1 = warp_maxf(t.has ? t.vyh : -INFINITY);
+    group_centroid<32, OVERLAP>(t.has, pv, vxh, vxl, vyh, vyl, t.rv, g.wxh, g.wxl, g.wyh, g.wyl,
+                                wr2, g.wrv);
+    g.bx0 = warp_minf(t.has ? vxh : INFINITY);
+    g.bx1 = warp_maxf(t.has ? vxh : -INFINITY);
+    g.by0 = warp_minf(t.has ? vyh : INFINITY);
+    g.by1 = warp_maxf(t.has ? vyh : -INFINITY);
     g.gx = G.x;
     g.gy = G.y;
     CellSums s;
@@ -1265,17 +1335,10 @@ __global__ __launch_bounds__(kCellThreads, kCellBlocksPerSM) void k_walk_f32_cel
           const uint32_t skip = min(max((uint32_t)__float_as_int(n1.z), cur + 1u), serEnd);
           if (COUNT) nVisit++;
           const int kind = cell_classify(g, cur, n0, n1);
-          if (kind == 1 && lane == 0) {
-            const uint32_t e = (s.ph + s.pn) & (kCellRing - 1);
-            q.pPos[e] = n0;
-            q.pMR[e] = make_float2(n1.x, n1.y);
-            q.pV[e] = (uint32_t)__float_as_int(n1.w);
-          }
-          if (kind == 2 && lane == 0) {
-            const uint32_t e = (s.ch + s.cn) & (kCellRing - 1);
-            q.cPos[e] = n0;
-            q.cMN[e] = make_float2(n1.x, __uint_as_float(cur));
-          }
+          if (kind == 1 && lane == 0)
+            put_point<MODEL, OVERLAP>(q, (s.ph + s.pn) & (kCellRing - 1), n0, n1);
+          if (kind == 2 && lane == 0)
+            put_accepted<MODEL, OVERLAP>(q, (s.ch + s.cn) & (kCellRing - 1), n0, n1, cur);
           s.pn += kind == 1 ? 1u : 0u;
           s.cn += kind == 2 ? 1u : 0u;
           serCur = kind == 3 ? cur + 1u : skip;
@@ -1324,19 +1387,13 @@ __global__ __launch_bounds__(kCellThreads, kCellBlocksPerSM) void k_walk_f32_cel
       }
       // points and accepted cells join their lists in lane order
       const uint32_t bP = __ballot_sync(0xffffffffu, kind == 1);
-      if (kind == 1) {
-        const uint32_t e = (s.ph + s.pn + __popc(bP & below)) & (kCellRing - 1);
-        q.pPos[e] = n0;
-        q.pMR[e] = make_float2(n1.x, n1.y);
-        q.pV[e] = (uint32_t)__float_as_int(n1.w);
-      }
+      if (kind == 1)
+        put_point<MODEL, OVERLAP>(q, (s.ph + s.pn + __popc(bP & below)) & (kCellRing - 1), n0, n1);
       s.pn += __popc(bP);
       const uint32_t bC = __ballot_sync(0xffffffffu, kind == 2);
-      if (kind == 2) {
-        const uint32_t e = (s.ch + s.cn + __popc(bC & below)) & (kCellRing - 1);
-        q.cPos[e] = n0;
-        q.cMN[e] = make_float2(n1.x, __uint_as_float(cur));
-      }
+      if (kind == 2)
+        put_accepted<MODEL, OVERLAP>(q, (s.ch + s.cn + __popc(bC & below)) & (kCellRing - 1), n0,
+                                     n1, cur);
       s.cn += __popc(bC);
       // opened cells push their children (lane order) while they fit; the
       // rest wait for the in-place walk
