@@ -120,11 +120,8 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_stats);
   dfree(h->d_lastStats);
   dfree(h->d_chunkStat);
-  dfree(h->d_status);
-  dfree(h->d_chunkBox);
+  dfree(h->d_zero);
   dfree(h->d_roots);
-  dfree(h->d_keyHi);
-  dfree(h->d_keyLo);
   dfree(h->d_ck);
   dfree(h->d_ckAlt);
   dfree(h->d_idx);
@@ -134,9 +131,6 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_flag);
   dfree(h->d_scan);
   dfree(h->d_deepRuns);
-  dfree(h->d_counts);
-  dfree(h->d_sortState);
-  dfree(h->d_scanState);
   dfree(h->d_bHi);
   dfree(h->d_bLo);
   dfree(h->d_bGid);
@@ -161,7 +155,6 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_bCnt);
   dfree(h->d_bT);
   dfree(h->d_rootNode);
-  dfree(h->d_rootT);
   dfree(h->d_graphBase);
   dfree(h->d_nodes);
   dfree(h->d_kids);
@@ -691,11 +684,31 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   rc |= dalloc(h, &h->d_stats, (size_t)GVIZ_STATS_CAP * G * 5);
   rc |= dalloc(h, &h->d_lastStats, G * 5);
   rc |= dalloc(h, &h->d_chunkStat, C);
-  rc |= dalloc(h, &h->d_status, 1);
-  rc |= dalloc(h, &h->d_chunkBox, C);
+  {
+    size_t bytes = 0;
+    auto part = [&bytes](size_t count, size_t size) {
+      const size_t at = bytes;
+      bytes += (count * size + 15) & ~(size_t)15;
+      return at;
+    };
+    const size_t atStatus = part(1, 4), atCounts = part(8, 4), atBox = part(4 * G, 8),
+                 atRootT = part(G, 4), atScan = part(scan_state_entries(std::max(Vs, G)), 8),
+                 atSort = part(sort_state_entries(Vs), 4);
+    char *zero = nullptr;
+    rc |= dalloc(h, &zero, bytes);
+    h->d_zero = zero;
+    h->zeroBytes = bytes;
+    if (zero) {
+      h->d_status = reinterpret_cast<uint32_t *>(zero + atStatus);
+      h->d_counts = reinterpret_cast<uint32_t *>(zero + atCounts);
+      h->d_box = reinterpret_cast<unsigned long long *>(zero + atBox);
+      h->d_rootT = reinterpret_cast<uint32_t *>(zero + atRootT);
+      h->d_scanState = reinterpret_cast<uint64_t *>(zero + atScan);
+      h->d_sortState = reinterpret_cast<uint32_t *>(zero + atSort);
+      if (cudaMemset(zero, 0, bytes) != cudaSuccess) rc |= GVIZ_CUDA_ERR_CUDA;
+    }
+  }
   rc |= dalloc(h, &h->d_roots, G);
-  rc |= dalloc(h, &h->d_keyHi, Vs);
-  rc |= dalloc(h, &h->d_keyLo, Vs);
   rc |= dalloc(h, &h->d_ck, Vs);
   rc |= dalloc(h, &h->d_ckAlt, Vs);
   rc |= dalloc(h, &h->d_idx, Vs);
@@ -705,9 +718,6 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   rc |= dalloc(h, &h->d_flag, Vs);
   rc |= dalloc(h, &h->d_scan, Vs);
   rc |= dalloc(h, &h->d_deepRuns, 2 * Vs);
-  rc |= dalloc(h, &h->d_counts, 8);
-  rc |= dalloc(h, &h->d_sortState, sort_state_entries(Vs));
-  rc |= dalloc(h, &h->d_scanState, scan_state_entries(2 * Vs + G));
   rc |= dalloc(h, &h->d_bHi, Vs);
   rc |= dalloc(h, &h->d_bLo, Vs);
   rc |= dalloc(h, &h->d_bGid, Vs);
@@ -732,7 +742,6 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   rc |= dalloc(h, &h->d_bCnt, Vs);
   rc |= dalloc(h, &h->d_bT, Vs);
   rc |= dalloc(h, &h->d_rootNode, G);
-  rc |= dalloc(h, &h->d_rootT, G);
   rc |= dalloc(h, &h->d_graphBase, G);
   rc |= dalloc(h, &h->d_nodes, h->maxNodes * sizeof(NodeD));
   rc |= dalloc(h, &h->d_kids, h->maxNodes);

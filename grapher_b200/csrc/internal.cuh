@@ -11,6 +11,7 @@
 #define GVIZ_LEAF_BIT 0x80000000u
 #define GVIZ_MAX_NODES_PER_CELL 256
 #define GVIZ_CHUNK 2048          // vertices per reduction chunk
+#define GVIZ_SCAN_TILE 2048      // entries per tile of the single-pass scans
 #define GVIZ_FIX_MAX 4096        // largest deep run sorted in shared memory
 #define GVIZ_DIR_TABLE 256       // coincident-direction table entries
 #define GVIZ_STATS_CAP 4096      // stat rows kept per graph (ring)
@@ -160,15 +161,18 @@ struct gvizCudaForce {
 
   // --- tree build scratch (device) ---
   size_t maxNodes = 0;
-  double4 *d_chunkBox = nullptr;
+  // one buffer zeroed at the start of every build, and its parts: status and
+  // counts, the graphs' boxes, the roots' subtree sizes, scan and sort state
+  void *d_zero = nullptr;
+  size_t zeroBytes = 0;
+  unsigned long long *d_box = nullptr;  // per graph: see k_bbox_chunks
   GraphRoot *d_roots = nullptr;
-  uint64_t *d_keyHi = nullptr, *d_keyLo = nullptr;  // per vertex
   uint64_t *d_ck = nullptr, *d_ckAlt = nullptr;     // composite sort keys
   uint32_t *d_idx = nullptr, *d_idxAlt = nullptr;   // sorted vertex ids
   uint64_t *d_sHi = nullptr, *d_sLo = nullptr;      // full keys, sorted order
   uint32_t *d_flag = nullptr, *d_scan = nullptr;    // V-sized
   uint32_t *d_deepRuns = nullptr;
-  uint32_t *d_counts = nullptr;  // [0]=runs [1]=deep runs [2]=buckets [3]=nodes
+  uint32_t *d_counts = nullptr;  // [1]=deep runs [2]=buckets [3]=nodes
   uint32_t *d_sortState = nullptr;  // radix sort: look-back status, digit counts, tickets
   uint64_t *d_scanState = nullptr;  // scan: ticket and look-back status
   uint64_t *d_bHi = nullptr, *d_bLo = nullptr;
@@ -294,6 +298,7 @@ void radix_sort_pairs(gvizCudaForce *h, uint64_t *keys, uint32_t *vals,
 void scan_exclusive(gvizCudaForce *h, const uint32_t *in, uint32_t *out,
                     size_t n, uint32_t *total);
 size_t sort_state_entries(size_t n);
+uint32_t *sort_digit_counts(gvizCudaForce *h);
 size_t scan_state_entries(size_t n);
 
 // tree.cu

@@ -10,8 +10,8 @@
 // it; it publishes its count (flag AGGREGATE), then adds the counts of the
 // tiles before it, walking back until one has published its inclusive
 // prefix (flag PREFIX), and publishes its own prefix (decoupled look-back).
-// The first pass's digit counts come from one read of the keys; each pass
-// counts the next pass's digits of the keys it holds.
+// The first pass's digit counts come from the kernel that makes the keys; each
+// pass counts the next pass's digits of the keys it holds.
 // Status words are 64 bits in the scan (flag in the high half, count in the
 // low half) and 32 bits in the sort, written and read with single relaxed
 // accesses; a wait that outlasts its iteration limit sets GVIZ_ST_TREE and
@@ -19,37 +19,25 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "scan.cuh"
 
 namespace {
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;  // 2048
+static_assert(kScanThreads * kScanItems == GVIZ_SCAN_TILE, "the scan state is sized by it");
+constexpr int kScanTile = GVIZ_SCAN_TILE;
 constexpr int kTopThreads = 1024;
 
 constexpr int kLookbackWidth = 8;
 constexpr int kSortThreads = 512;
-constexpr int kHistThreads = 256;
 constexpr int kSortPasses = (64 - GVIZ_SORT_SKIP_BITS) / 8;
 static_assert(kSortPasses % 2 == 0, "the sorted pairs must end in the input buffers");
 
-constexpr uint64_t kFlagAggregate = 1ull << 32;
-constexpr uint64_t kFlagPrefix = 2ull << 32;
 // the sort's status words: flag in the top two bits, count below (n < 2^30)
 constexpr uint32_t kAggregate32 = 1u << 30;
 constexpr uint32_t kPrefix32 = 1u << 31;
 constexpr uint32_t kCount32 = kAggregate32 - 1u;
-constexpr uint32_t kLookbackSpin = 1u << 22;  // reads of a status word before giving up
-
-__device__ __forceinline__ uint64_t ld_status(const uint64_t *p) {
-  uint64_t v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_status(uint64_t *p, uint64_t v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 
 __device__ __forceinline__ uint32_t ld_status32(const uint32_t *p) {
   uint32_t v;
@@ -94,78 +82,13 @@ __device__ __forceinline__ uint32_t lookback_digit(const uint32_t *st, uint32_t 
   return excl;
 }
 
-// The scan's look-back by one warp: lane l reads the word of the l-th tile
-// before, so a step covers 32 tiles; the result is in every lane.
-__device__ __forceinline__ uint32_t lookback_warp(const uint64_t *st, uint32_t tile,
-                                                  uint32_t *status) {
-  const uint32_t lane = lane_id();
-  uint32_t excl = 0;
-  uint32_t spins = 0;
-  for (int64_t p = (int64_t)tile - 1; p >= 0; p -= 32) {
-    uint64_t w = p - lane >= 0 ? ld_status(st + (size_t)(p - lane)) : kFlagPrefix;
-    uint32_t have;
-    for (;;) {
-      // enough once every word up to the nearest prefix is published
-      have = __ballot_sync(0xffffffffu, (w >> 32) != 0);
-      const uint32_t pre = __ballot_sync(0xffffffffu, (w & ~0xffffffffull) == kFlagPrefix);
-      const uint32_t need = pre ? (pre ^ (pre - 1u)) : 0xffffffffu;
-      if ((have & need) == need) {
-        uint32_t c = (need >> lane) & 1u ? (uint32_t)w : 0u;
-        excl += __reduce_add_sync(0xffffffffu, c);
-        if (pre) return excl;
-        break;
-      }
-      if (++spins > kLookbackSpin) {
-        if (lane == 0) atomicOr(status, GVIZ_ST_TREE);
-        return excl;
-      }
-      if ((w >> 32) == 0) w = ld_status(st + (size_t)(p - lane));
-    }
-  }
-  return excl;
-}
-
-// Block-wide exclusive scan of one value per thread; returns the block total.
-template <int THREADS>
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v,
-                                                         uint32_t &excl) {
-  __shared__ uint32_t warpTot[THREADS / 32];
-  const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  uint32_t inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= (unsigned)o) inc += t;
-  }
-  if (lane == 31) warpTot[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    uint32_t t = lane < THREADS / 32 ? warpTot[lane] : 0;
-    uint32_t ti = t;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t u = __shfl_up_sync(0xffffffffu, ti, o);
-      if (lane >= (unsigned)o) ti += u;
-    }
-    if (lane < THREADS / 32) warpTot[lane] = ti - t;  // exclusive warp offsets
-  }
-  __syncthreads();
-  excl = warpTot[w] + inc - v;
-  __shared__ uint32_t blockTot;
-  if (threadIdx.x == THREADS - 1) blockTot = excl + v;
-  __syncthreads();
-  uint32_t bt = blockTot;
-  __syncthreads();
-  return bt;
-}
-
 // Single-pass exclusive scan: tile = ticket, 2048 entries per tile.
 // state: [0] ticket, [1 + t] status of tile t.
 __global__ __launch_bounds__(kScanThreads) void k_scan_onepass(
     const uint32_t *in, uint32_t *out, uint32_t n, uint64_t *state, uint32_t *total,
     uint32_t *status) {
-  __shared__ uint32_t sTile, sExcl;
-  if (threadIdx.x == 0) sTile = atomicAdd(reinterpret_cast<unsigned long long *>(state), 1ull);
+  __shared__ uint32_t sTile;
+  if (threadIdx.x == 0) sTile = scan_ticket(state);
   __syncthreads();
   const uint32_t tile = sTile;
   const uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
@@ -179,19 +102,7 @@ __global__ __launch_bounds__(kScanThreads) void k_scan_onepass(
   }
   uint32_t excl;
   const uint32_t tot = block_exclusive_scan<kScanThreads>(s, excl);
-  uint64_t *st = state + 1;
-  if (threadIdx.x < 32) {
-    if (tile != 0 && threadIdx.x == 0) st_status(st + tile, kFlagAggregate | tot);
-    const uint32_t before = lookback_warp(st, tile, status);
-    if (threadIdx.x == 0) {
-      st_status(st + tile, kFlagPrefix | (before + tot));
-      sExcl = before;
-      const uint32_t nTiles = (n + kScanTile - 1) / kScanTile;
-      if (total && tile == nTiles - 1) *total = before + tot;
-    }
-  }
-  __syncthreads();
-  excl += sExcl;
+  excl += scan_publish(state, tile, tot, (n + kScanTile - 1) / kScanTile, total, status);
 #pragma unroll
   for (int j = 0; j < kScanItems; j++) {
     const uint32_t i = base + j;
@@ -224,21 +135,6 @@ __global__ __launch_bounds__(kTopThreads) void k_scan_single(
     }
   }
   if (threadIdx.x == 0 && total) *total = tot;
-}
-
-// Digit counts of the first sort pass (each later pass counts the digit of
-// the pass after it while it scatters).
-__global__ __launch_bounds__(kHistThreads) void k_radix_hist0(
-    const uint64_t *__restrict__ keys, uint32_t n, uint32_t *ghist) {
-  __shared__ uint32_t sh[256];
-  sh[threadIdx.x] = 0u;
-  __syncthreads();
-  const uint32_t stride = gridDim.x * kHistThreads;
-  for (uint32_t i = blockIdx.x * kHistThreads + threadIdx.x; i < n; i += stride)
-    atomicAdd(&sh[(uint32_t)(keys[i] >> GVIZ_SORT_SKIP_BITS) & 255u], 1u);
-  __syncthreads();
-  const uint32_t c = sh[threadIdx.x];
-  if (c) atomicAdd(ghist + threadIdx.x, c);
 }
 
 // The lanes holding valid keys of the same 8-bit digit d: eight ballots, one
@@ -400,10 +296,14 @@ static size_t sort_tiles(size_t n) {
 
 size_t sort_state_entries(size_t n) {
   const size_t tiles = sort_tiles(n);
-  // per pass: tiles * 256 status words; then the global counts and the
-  // tickets (all 32 bits)
+  // per pass the global counts of 256 digits and a ticket, then per pass and
+  // tile 256 status words (all 32 bits)
   return (size_t)kSortPasses * (256 * (tiles ? tiles : 1) + 256 + 1);
 }
+
+// Where the caller counts the first sorted digit (GVIZ_SORT_SKIP_BITS up) of
+// the keys before radix_sort_pairs, in the zeroed sort state.
+uint32_t *sort_digit_counts(gvizCudaForce *h) { return h->d_sortState; }
 
 // Exclusive scan of n uint32 (n <= 2^31); in == out allowed. total may be
 // nullptr or a device pointer receiving the sum.
@@ -425,7 +325,8 @@ void scan_exclusive(gvizCudaForce *h, const uint32_t *in, uint32_t *out,
 
 // Stable sort by the key bits above GVIZ_SORT_SKIP_BITS (an even number of
 // 8-bit passes, so the result ends in (keys, vals)); keys equal in those bits
-// keep their input order.
+// keep their input order. The sort state is zero but for the first digit's
+// counts.
 // The scatter's shared memory exceeds the default per-block budget: opted
 // into once per device, at handle creation (outside any stream capture).
 void sort_set_smem_limits() {
@@ -439,15 +340,9 @@ void radix_sort_pairs(gvizCudaForce *h, uint64_t *keys, uint32_t *vals,
   if (n <= 1) return;
   const SortShape shape = sort_shape(n);
   const uint32_t tiles = (uint32_t)sort_tiles(n);
-  uint32_t *state = h->d_sortState;
-  uint32_t *ghist = state + (size_t)kSortPasses * 256 * tiles;
+  uint32_t *ghist = sort_digit_counts(h);
   uint32_t *tickets = ghist + kSortPasses * 256;
-  cudaMemsetAsync(state, 0, sort_state_entries(n) * sizeof(uint32_t), h->stream);
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const uint32_t hb = std::min<uint32_t>(tiles * 4u, (uint32_t)(sms > 0 ? sms : 1) * 2u);
-  k_radix_hist0<<<hb, kHistThreads, 0, h->stream>>>(keys, (uint32_t)n, ghist);
+  uint32_t *state = tickets + kSortPasses;
   uint64_t *ka = keys, *kb = keysAlt;
   uint32_t *va = vals, *vb = valsAlt;
   for (int pass = 0; pass < kSortPasses; pass++) {

@@ -3,9 +3,10 @@
 // sets of the reference's leaves.
 //
 // Pipeline (one launch each, no host synchronisation):
-//   bbox per chunk -> square root box per graph (gvizQuadtree.c:165-178)
-//   per point: quadrant path by replaying the reference's FP64 descent
-//     (QuadrantFor :65-73 against centres cx +/- halfSize/2, Subdivide :75-92)
+//   bounding box per graph (gvizQuadtree.c:165-178)
+//   per point: root box and quadrant path by replaying the reference's FP64
+//     descent (QuadrantFor :65-73 against centres cx +/- halfSize/2,
+//     Subdivide :75-92)
 //   stable radix sort of (graph, path) -> fix-up sort of equal-prefix runs
 //   buckets = identical full paths -> Karras binary radix tree (2012)
 //   binary nodes merged into quadtree nodes (two path bits per level)
@@ -31,6 +32,7 @@
 #include <cuda/atomic>
 
 #include "internal.cuh"
+#include "scan.cuh"
 
 namespace {
 
@@ -41,19 +43,39 @@ constexpr int kThreads = 256;
 // bounding boxes and roots
 // ---------------------------------------------------------------------------
 
+// A double as an unsigned integer of the same order, for atomic min and max.
+__device__ __forceinline__ uint64_t ordered_bits(double x) {
+  const uint64_t b = (uint64_t)__double_as_longlong(x);
+  return b >> 63 ? ~b : b | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double from_ordered_bits(uint64_t u) {
+  return __longlong_as_double((long long)(u >> 63 ? u ^ 0x8000000000000000ull : ~u));
+}
+
+// Bounding box of every graph: box[4g..] = the largest ordered bits of -min x,
+// max x, -min y, max y over its points (zero at the start: below every
+// double's). Minimum and maximum are order-free, so the box is exact however
+// the chunks' atomics interleave.
 __global__ __launch_bounds__(kThreads) void k_bbox_chunks(
     const double2 *__restrict__ pos, const uint32_t *__restrict__ cb,
-    const uint32_t *__restrict__ ce, double4 *box, uint32_t *status) {
+    const uint32_t *__restrict__ ce, const uint32_t *__restrict__ cg, unsigned long long *box,
+    uint32_t *status) {
   const uint32_t b = cb[blockIdx.x], e = ce[blockIdx.x];
   double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
   int bad = 0;
-  for (uint32_t i = b + threadIdx.x; i < e; i += kThreads) {
-    double2 p = pos[i];
-    if (!isfinite(p.x) || !isfinite(p.y)) bad = 1;
-    mnx = fmin(mnx, p.x);
-    mxx = fmax(mxx, p.x);
-    mny = fmin(mny, p.y);
-    mxy = fmax(mxy, p.y);
+  double2 p[GVIZ_CHUNK / kThreads];  // the chunk's loads, all in flight at once
+#pragma unroll
+  for (int r = 0; r < GVIZ_CHUNK / kThreads; r++) {
+    const uint32_t i = b + r * kThreads + threadIdx.x;
+    p[r] = pos[min(i, e - 1u)];
+  }
+#pragma unroll
+  for (int r = 0; r < GVIZ_CHUNK / kThreads; r++) {
+    if (!isfinite(p[r].x) || !isfinite(p[r].y)) bad = 1;
+    mnx = fmin(mnx, p[r].x);
+    mxx = fmax(mxx, p[r].x);
+    mny = fmin(mny, p[r].y);
+    mxy = fmax(mxy, p[r].y);
   }
   for (int o = 16; o > 0; o >>= 1) {
     mnx = fmin(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
@@ -65,180 +87,177 @@ __global__ __launch_bounds__(kThreads) void k_bbox_chunks(
   if (lane_id() == 0) wb[threadIdx.x >> 5] = make_double4(mnx, mxx, mny, mxy);
   if (bad) atomicOr(status, GVIZ_ST_NONFINITE);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double4 r = wb[0];
-    for (int w = 1; w < kThreads / 32; w++) {
-      r.x = fmin(r.x, wb[w].x);
-      r.y = fmax(r.y, wb[w].y);
-      r.z = fmin(r.z, wb[w].z);
-      r.w = fmax(r.w, wb[w].w);
-    }
-    box[blockIdx.x] = r;
+  if (threadIdx.x < 4) {
+    const double *w = reinterpret_cast<const double *>(wb) + threadIdx.x;
+    double r = w[0];
+    for (int k = 1; k < kThreads / 32; k++)
+      r = (threadIdx.x & 1u) ? fmax(r, w[4 * k]) : fmin(r, w[4 * k]);
+    atomicMax(box + 4 * (size_t)cg[blockIdx.x] + threadIdx.x,
+              (unsigned long long)ordered_bits((threadIdx.x & 1u) ? r : -r));
   }
 }
 
-// One block per graph: min/max over the graph's chunk boxes (order-free, so
-// exact), then the root box of gvizQuadtreeBuild.
-__global__ __launch_bounds__(kThreads) void k_graph_roots(
-    const double4 *__restrict__ box, const uint32_t *__restrict__ gcb,
-    const uint32_t *__restrict__ gce, GraphRoot *roots, uint32_t G,
-    uint32_t *status) {
-  const uint32_t g = blockIdx.x;
-  double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
-  for (uint32_t c = gcb[g] + threadIdx.x; c < gce[g]; c += kThreads) {
-    double4 r = box[c];
-    mnx = fmin(mnx, r.x);
-    mxx = fmax(mxx, r.y);
-    mny = fmin(mny, r.z);
-    mxy = fmax(mxy, r.w);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    mnx = fmin(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-    mxx = fmax(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-    mny = fmin(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-    mxy = fmax(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-  }
-  __shared__ double4 wb[kThreads / 32];
-  if (lane_id() == 0) wb[threadIdx.x >> 5] = make_double4(mnx, mxx, mny, mxy);
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int w = 1; w < kThreads / 32; w++) {
-    mnx = fmin(mnx, wb[w].x);
-    mxx = fmax(mxx, wb[w].y);
-    mny = fmin(mny, wb[w].z);
-    mxy = fmax(mxy, wb[w].w);
-  }
-  mnx = fmin(mnx, wb[0].x);
-  mxx = fmax(mxx, wb[0].y);
-  mny = fmin(mny, wb[0].z);
-  mxy = fmax(mxy, wb[0].w);
+// The root box of gvizQuadtreeBuild (src/ds/gvizQuadtree.c:165-178) from a
+// graph's bounding box. D, the first depth whose half size is at most 1e-9,
+// follows from the exponents (halving is exact).
+__device__ __forceinline__ GraphRoot graph_root(const unsigned long long *box) {
+  const double mnx = -from_ordered_bits(box[0]), mxx = from_ordered_bits(box[1]);
+  const double mny = -from_ordered_bits(box[2]), mxy = from_ordered_bits(box[3]);
   GraphRoot R;
-  if (!(mnx <= mxx)) {  // empty graph
-    R.cx = 0.0;
-    R.cy = 0.0;
-    R.h0 = 1.0;
-    R.D = 0;
-    R.capped = 0;
-    roots[g] = R;
-    return;
-  }
-  double sx = mxx - mnx, sy = mxy - mny;
-  double span = sx > sy ? sx : sy;
+  R.cx = R.cy = 0.0;
+  R.h0 = 1.0;
+  R.D = R.capped = 0;
+  if (!(mnx <= mxx)) return R;  // every position NaN: an error that the status reports
+  const double sx = mxx - mnx, sy = mxy - mny;
+  const double span = sx > sy ? sx : sy;
   R.h0 = span > 0.0 ? span / 2.0 : 1.0;
   R.cx = (mnx + mxx) / 2.0;
   R.cy = (mny + mxy) / 2.0;
-  double h = R.h0;
-  int d = 0;
-  while (h > 1e-9 && d < 64) {
-    h = h / 2.0;
-    d++;
-  }
-  R.D = d;
-  R.capped = h > 1e-9 ? 1 : 0;
-  if (R.capped) atomicOr(status, GVIZ_ST_DEPTH_CAP);
-  roots[g] = R;
+  const long long hb = __double_as_longlong(R.h0), lb = __double_as_longlong(1e-9);
+  const int up = (int)(hb >> 52) - (int)(lb >> 52);  // h0 > 0: no sign bit
+  const int d = up + ((hb & 0xfffffffffffffll) > (lb & 0xfffffffffffffll) ? 1 : 0);
+  R.D = min(max(d, 0), 64);
+  R.capped = d > 64 ? 1 : 0;
+  return R;
 }
 
-// Quadrant path of every point: digit = (north ? 0 : 2) + (east ? 1 : 0),
-// i.e. NW=0 NE=1 SW=2 SE=3 (include/ds/gvizQuadtree.h:11-17), so sorted
-// paths are the reference's depth-first NW,NE,SW,SE order.
+// Sixteen levels (or n < 16) of the descent from centre (cx, cy) and half
+// size h: the digits of 16 levels, the first in the top bits. The sign of
+// p - c, which is exact, gives the side: QuadrantFor's p >= c is its clear
+// sign bit; c moves by h / 2 with that sign. Halving subtracts one from h's
+// exponent (h > 1e-9 here).
+__device__ __forceinline__ uint32_t path_digits(double2 p, double &cx, double &cy, double &h,
+                                                int n) {
+  uint32_t w = 0;
+  auto level = [&]() {
+    const uint32_t tx = (uint32_t)__double2hiint(p.x - cx);
+    const uint32_t ty = (uint32_t)__double2hiint(p.y - cy);
+    const uint32_t hh = (uint32_t)__double2hiint(h) - 0x00100000u;
+    const int hl = __double2loint(h);
+    w = __funnelshift_l(ty, w, 1);  // south
+    w = __funnelshift_l(tx, w, 1);  // west
+    cx += __hiloint2double((int)(hh | (tx & 0x80000000u)), hl);
+    cy += __hiloint2double((int)(hh | (ty & 0x80000000u)), hl);
+    h = __hiloint2double((int)hh, hl);
+  };
+  if (n >= 16) {
+#pragma unroll
+    for (int d = 0; d < 16; d++) level();
+    return w ^ 0x55555555u;  // west to east
+  }
+#pragma unroll 1
+  for (int d = 0; d < n; d++) level();
+  return n > 0 ? (w ^ (0x55555555u >> (32 - 2 * n))) << (32 - 2 * n) : 0u;
+}
+
+// Quadrant path of a point: digit = (north ? 0 : 2) + (east ? 1 : 0), i.e.
+// NW=0 NE=1 SW=2 SE=3 (include/ds/gvizQuadtree.h:11-17), so sorted paths are
+// the reference's depth-first NW,NE,SW,SE order. lo is the digits of levels
+// 33 to 64 (FULL only).
+template <bool FULL>
+__device__ __forceinline__ uint64_t quadrant_path(double2 p, const GraphRoot &R, uint64_t &lo) {
+  double cx = R.cx, cy = R.cy, h = R.h0;
+  const uint32_t w0 = path_digits(p, cx, cy, h, R.D);
+  const uint32_t w1 = path_digits(p, cx, cy, h, R.D - 16);
+  if (FULL) {
+    const uint32_t w2 = path_digits(p, cx, cy, h, R.D - 32);
+    const uint32_t w3 = path_digits(p, cx, cy, h, R.D - 48);
+    lo = ((uint64_t)w2 << 32) | w3;
+  }
+  return ((uint64_t)w0 << 32) | w1;
+}
+
+// Composite sort key (graph, quadrant path) of every point, and the counts of
+// the first sorted digit. Only the first 32 levels are descended here: the
+// sort orders the top 48 bits, and the few points whose sorted bits meet
+// another's take their whole path in k_runs. The descent replays the
+// reference's FP64 steps, 9 instructions per level, four of them FP64. Eight
+// blocks per SM stride over the points: a block's 256 counts go to the same
+// few cache lines as every other's, and 4,096 blocks of one point per thread
+// spend 16 us on them. 23 us at 1,048,576 points; all levels at 35
+// instructions each, and the counts in a pass of their own, 60.
 __global__ __launch_bounds__(kThreads) void k_keys(
     const double2 *__restrict__ pos, const uint32_t *__restrict__ gid,
-    const GraphRoot *__restrict__ roots, uint64_t *keyHi, uint64_t *keyLo,
-    uint64_t *ck, uint32_t *idx, uint32_t V, int gbits) {
-  uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= V) return;
-  const uint32_t g = gid ? gid[i] : 0u;
-  const GraphRoot R = roots[g];
-  const double2 p = pos[i];
-  double cx = R.cx, cy = R.cy, h = R.h0;
-  uint64_t hi = 0, lo = 0;
-  for (int d = 1; d <= R.D; d++) {
-    const bool east = p.x >= cx;
-    const bool north = p.y >= cy;
-    const uint64_t q = (north ? 0ull : 2ull) | (east ? 1ull : 0ull);
-    const double quarter = h / 2.0;
-    cx = east ? cx + quarter : cx + (-quarter);
-    cy = north ? cy + quarter : cy + (-quarter);
-    h = quarter;
-    if (d <= 32)
-      hi |= q << (64 - 2 * d);
-    else
-      lo |= q << (128 - 2 * d);
+    const unsigned long long *__restrict__ box, GraphRoot *roots, uint64_t *ck, uint32_t *idx,
+    uint32_t *digits, uint32_t *status, uint32_t V, int gbits) {
+  __shared__ uint32_t cnt[256];
+  static_assert(kThreads == 256, "one thread per digit");
+  cnt[threadIdx.x] = 0u;
+  __syncthreads();
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < V; i += gridDim.x * kThreads) {
+    const uint32_t g = gid ? gid[i] : 0u;
+    const double2 p = pos[i];
+    const GraphRoot R = graph_root(box + 4 * (size_t)g);
+    if (i == 0 || (gid && gid[i - 1] != g)) {  // the graph's first point
+      roots[g] = R;
+      if (R.capped) atomicOr(status, GVIZ_ST_DEPTH_CAP);
+    }
+    uint64_t lo;
+    const uint64_t hi = quadrant_path<false>(p, R, lo);
+    const uint64_t key = gbits ? (((uint64_t)g << (64 - gbits)) | (hi >> gbits)) : hi;
+    ck[i] = key;
+    idx[i] = i;
+    atomicAdd(&cnt[(uint32_t)(key >> GVIZ_SORT_SKIP_BITS) & 255u], 1u);
   }
-  keyHi[i] = hi;
-  keyLo[i] = lo;
-  ck[i] = gbits ? (((uint64_t)g << (64 - gbits)) | (hi >> gbits)) : hi;
-  idx[i] = i;
-}
-
-// The sorted points' full paths, and the starts of runs of equal composite
-// keys (the sorted bits of the composite key).
-__global__ __launch_bounds__(kThreads) void k_gather_keys(
-    const uint32_t *__restrict__ idx, const uint64_t *__restrict__ keyHi,
-    const uint64_t *__restrict__ keyLo, const uint64_t *__restrict__ ck, uint64_t *sHi,
-    uint64_t *sLo, uint32_t *flag, uint32_t V) {
-  uint32_t s = blockIdx.x * kThreads + threadIdx.x;
-  if (s >= V) return;
-  uint32_t i = idx[s];
-  sHi[s] = keyHi[i];
-  sLo[s] = keyLo[i];
-  flag[s] = (s == 0 || (ck[s] >> GVIZ_SORT_SKIP_BITS) !=
-                           (ck[s - 1] >> GVIZ_SORT_SKIP_BITS)) ? 1u : 0u;
+  __syncthreads();
+  if (cnt[threadIdx.x]) atomicAdd(digits + threadIdx.x, cnt[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------------------
 // runs of equal composite keys
 // ---------------------------------------------------------------------------
 
-// Runs of equal composite keys (equal sorted prefixes). The thread at a
-// run's start finds its end, the first later key whose sorted prefix
-// differs, by a galloping search over the sorted keys (most runs are one
-// key long, found by the first probe). Runs longer than the leaf capacity k
-// need their deeper digits sorted; runs of 2..k points lie in one leaf, so
-// their keys are cut to the common prefix (the leaf keeps them in vertex
-// order, as the reference does).
+// The sorted points' paths, from the composite keys themselves. A point whose
+// sorted bits (the top 48) differ from its neighbours' needs no more than
+// the key holds. Runs of equal sorted bits of 2..k points lie in one leaf:
+// their paths are cut to the common prefix (the leaf keeps them in vertex
+// order, as the reference does). The points of longer runs take their whole
+// path from the descent, and the run's first point lists the run, whose end
+// it finds by a galloping search, for k_sort_runs. One pass over keys in
+// order, 28 B per point, no gathers but those points'.
 __global__ __launch_bounds__(kThreads) void k_runs(
-    const uint64_t *__restrict__ ck, const uint32_t *__restrict__ flag, uint32_t *counts,
+    const uint64_t *__restrict__ ck, const uint32_t *__restrict__ idx,
+    const double2 *__restrict__ pos, const GraphRoot *__restrict__ roots, uint32_t *counts,
     uint32_t *deep, uint64_t *sHi, uint64_t *sLo, uint32_t V, uint32_t k, int gbits) {
-  const uint32_t start = blockIdx.x * kThreads + threadIdx.x;
-  if (start >= V || !flag[start]) return;
-  const uint64_t key = ck[start] >> GVIZ_SORT_SKIP_BITS;
-  uint32_t end = start + 1u;
-  if (end < V && (ck[end] >> GVIZ_SORT_SKIP_BITS) == key) {
-    uint32_t lo = end, hi = V;  // ck[lo] is in the run, the end is in (lo, hi]
-    for (uint32_t step = 1u;; step <<= 1) {
-      const uint32_t probe = lo + step;
-      if (probe >= V || probe < lo) break;
-      if ((ck[probe] >> GVIZ_SORT_SKIP_BITS) != key) {
-        hi = probe;
-        break;
+  const uint32_t s = blockIdx.x * kThreads + threadIdx.x;
+  if (s >= V) return;
+  const uint64_t full = ck[s];
+  const uint64_t key = full >> GVIZ_SORT_SKIP_BITS;
+  uint64_t hi = full << gbits, lo = 0;
+  uint32_t back = 0, fwd = 0;  // equal keys before and after, counted to k
+  while (back < k && back < s && (ck[s - back - 1u] >> GVIZ_SORT_SKIP_BITS) == key) back++;
+  while (back + fwd < k && s + fwd + 1u < V && (ck[s + fwd + 1u] >> GVIZ_SORT_SKIP_BITS) == key)
+    fwd++;
+  if (back + fwd >= k) {  // more than k points
+    const uint32_t g = gbits ? (uint32_t)(full >> (64 - gbits)) : 0u;
+    hi = quadrant_path<true>(pos[idx[s]], roots[g], lo);
+    if (back == 0) {
+      uint32_t last = s + fwd, hiS = V;  // the run's end is in (last, hiS]
+      for (uint32_t step = 1u;; step <<= 1) {
+        const uint32_t probe = last + step;
+        if (probe >= V || probe < last) break;
+        if ((ck[probe] >> GVIZ_SORT_SKIP_BITS) != key) {
+          hiS = probe;
+          break;
+        }
+        last = probe;
       }
-      lo = probe;
+      while (hiS - last > 1u) {
+        const uint32_t mid = last + (hiS - last) / 2u;
+        if ((ck[mid] >> GVIZ_SORT_SKIP_BITS) == key)
+          last = mid;
+        else
+          hiS = mid;
+      }
+      const uint32_t slot = atomicAdd(&counts[1], 1u);
+      deep[2 * slot] = s;
+      deep[2 * slot + 1] = hiS - s;
     }
-    while (hi - lo > 1u) {
-      const uint32_t mid = lo + (hi - lo) / 2u;
-      if ((ck[mid] >> GVIZ_SORT_SKIP_BITS) == key)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    end = hi;
+  } else if (back + fwd > 0) {
+    hi = (key << GVIZ_SORT_SKIP_BITS) << gbits;
   }
-  const uint32_t len = end - start;
-  if (len > k) {
-    uint32_t slot = atomicAdd(&counts[1], 1u);
-    deep[2 * slot] = start;
-    deep[2 * slot + 1] = len;
-  } else if (len >= 2) {
-    // path bits covered by the sorted prefix of the composite key
-    const int covered = 64 - GVIZ_SORT_SKIP_BITS - gbits;
-    const uint64_t mask = covered >= 64 ? ~0ull : (~0ull << (64 - covered));
-    for (uint32_t j = start; j < end; j++) {
-      sHi[j] &= mask;
-      sLo[j] = 0;
-    }
-  }
+  sHi[s] = hi;
+  sLo[s] = lo;
 }
 
 __device__ __forceinline__ bool key_less(uint64_t ah, uint64_t al, uint32_t av,
@@ -318,34 +337,60 @@ __global__ __launch_bounds__(512) void k_sort_runs(
 // buckets (identical full paths) and the binary radix tree
 // ---------------------------------------------------------------------------
 
-__global__ __launch_bounds__(kThreads) void k_bucket_flags(
+// Buckets, the runs of identical full paths, numbered by a single-pass scan
+// (sort.cu): a warp takes 256 consecutive sorted points in rounds of 32, the
+// ballot of bucket starts gives each its number in the warp.
+__global__ __launch_bounds__(kThreads) void k_buckets(
     const uint64_t *__restrict__ sHi, const uint64_t *__restrict__ sLo,
-    const uint32_t *__restrict__ idx, const uint32_t *__restrict__ gid,
-    uint32_t *flag, uint32_t V) {
-  uint32_t s = blockIdx.x * kThreads + threadIdx.x;
-  if (s >= V) return;
-  uint32_t f = 1;
-  if (s > 0) {
-    f = (sHi[s] != sHi[s - 1] || sLo[s] != sLo[s - 1]) ? 1u : 0u;
-    if (!f && gid) f = gid[idx[s]] != gid[idx[s - 1]];
+    const uint64_t *__restrict__ ck, uint32_t *bStart, uint64_t *bHi, uint64_t *bLo,
+    uint32_t *bGid, uint2 *upLeaf, uint64_t *state, uint32_t *total, uint32_t *status, uint32_t V,
+    int gbits) {
+  constexpr int kRounds = GVIZ_SCAN_TILE / kThreads;
+  __shared__ uint32_t sTile;
+  if (threadIdx.x == 0) sTile = scan_ticket(state);
+  __syncthreads();
+  const uint32_t tile = sTile;
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  const uint32_t s0 = tile * GVIZ_SCAN_TILE + w * (32u * kRounds) + lane;
+  uint64_t hi[kRounds], lo[kRounds];
+  uint32_t starts[kRounds], g[kRounds];
+  uint32_t count = 0;
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    const uint32_t s = min(s0 + 32u * r, V - 1u);
+    hi[r] = sHi[s];
+    lo[r] = sLo[s];
+    g[r] = gbits ? (uint32_t)(ck[s] >> (64 - gbits)) : 0u;
   }
-  flag[s] = f;
-}
-
-__global__ __launch_bounds__(kThreads) void k_bucket_fill(
-    const uint32_t *__restrict__ flag, const uint32_t *__restrict__ scan,
-    const uint64_t *__restrict__ sHi, const uint64_t *__restrict__ sLo,
-    const uint32_t *__restrict__ idx, const uint32_t *__restrict__ gid,
-    uint32_t *bStart, uint64_t *bHi, uint64_t *bLo, uint32_t *bGid,
-    uint2 *upLeaf, uint32_t V) {
-  uint32_t s = blockIdx.x * kThreads + threadIdx.x;
-  if (s >= V || !flag[s]) return;
-  uint32_t b = scan[s];
-  bStart[b] = s;
-  bHi[b] = sHi[s];
-  bLo[b] = sLo[s];
-  bGid[b] = gid ? gid[idx[s]] : 0u;
-  upLeaf[b] = make_uint2(GVIZ_NONE, 0u);
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    const uint32_t s = s0 + 32u * r;
+    uint64_t ph = __shfl_up_sync(0xffffffffu, hi[r], 1);
+    uint64_t pl = __shfl_up_sync(0xffffffffu, lo[r], 1);
+    uint32_t pg = __shfl_up_sync(0xffffffffu, g[r], 1);
+    if (lane == 0 && s > 0 && s < V) {
+      ph = sHi[s - 1u];
+      pl = sLo[s - 1u];
+      pg = gbits ? (uint32_t)(ck[s - 1u] >> (64 - gbits)) : 0u;
+    }
+    const bool start = s < V && (s == 0 || ph != hi[r] || pl != lo[r] || pg != g[r]);
+    starts[r] = __ballot_sync(0xffffffffu, start);
+    count += __popc(starts[r]);
+  }
+  uint32_t b = scan_tile_prefix<kThreads>(state, tile, count, (V + GVIZ_SCAN_TILE - 1u) / GVIZ_SCAN_TILE,
+                                          total, status);
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    if ((starts[r] >> lane) & 1u) {
+      const uint32_t at = b + __popc(starts[r] & ((1u << lane) - 1u));
+      bStart[at] = s0 + 32u * r;
+      bHi[at] = hi[r];
+      bLo[at] = lo[r];
+      bGid[at] = g[r];
+      upLeaf[at] = make_uint2(GVIZ_NONE, 0u);
+    }
+    b += __popc(starts[r]);
+  }
 }
 
 // Common-prefix length in bits of the composite keys (graph id:32,
@@ -1430,37 +1475,26 @@ inline uint32_t blocks_for(size_t n) {
 void enqueue_tree_build(gvizCudaForce *h) {
   const uint32_t V = (uint32_t)h->V;
   cudaStream_t st = h->stream;
-  cudaMemsetAsync(h->d_counts, 0, 8 * sizeof(uint32_t), st);
-  // graphs without vertices get no root: their subtree size must read 0
-  cudaMemsetAsync(h->d_rootT, 0, h->G * sizeof(uint32_t), st);
-  k_bbox_chunks<<<h->nChunks, kThreads, 0, st>>>(h->d_pos, h->d_chunkBegin,
-                                                  h->d_chunkEnd, h->d_chunkBox,
-                                                  h->d_status);
-  k_graph_roots<<<(uint32_t)h->G, kThreads, 0, st>>>(
-      h->d_chunkBox, h->d_gChunkBegin, h->d_gChunkEnd, h->d_roots,
-      (uint32_t)h->G, h->d_status);
-  k_keys<<<blocks_for(V), kThreads, 0, st>>>(h->d_pos, h->d_gid, h->d_roots,
-                                             h->d_keyHi, h->d_keyLo, h->d_ck,
-                                             h->d_idx, V, h->gbits);
+  // status, counters, boxes, subtree sizes (a graph without vertices gets no
+  // root: its size must read 0), the scan's and the sort's state
+  cudaMemsetAsync(h->d_zero, 0, h->zeroBytes, st);
+  k_bbox_chunks<<<h->nChunks, kThreads, 0, st>>>(h->d_pos, h->d_chunkBegin, h->d_chunkEnd,
+                                                  h->d_chunkGraph, h->d_box, h->d_status);
+  k_keys<<<std::min(blocks_for(V), 148u * 8u), kThreads, 0, st>>>(h->d_pos, h->d_gid, h->d_box, h->d_roots, h->d_ck,
+                                             h->d_idx, sort_digit_counts(h), h->d_status, V,
+                                             h->gbits);
   prof_mark(h, "tree_keys");
   radix_sort_pairs(h, h->d_ck, h->d_idx, h->d_ckAlt, h->d_idxAlt, V);
-  k_gather_keys<<<blocks_for(V), kThreads, 0, st>>>(h->d_idx, h->d_keyHi, h->d_keyLo,
-                                                    h->d_ck, h->d_sHi, h->d_sLo,
-                                                    h->d_flag, V);
-  k_runs<<<blocks_for(V), kThreads, 0, st>>>(h->d_ck, h->d_flag, h->d_counts, h->d_deepRuns,
-                                             h->d_sHi, h->d_sLo, V, h->params.nodesPerCell,
-                                             h->gbits);
+  k_runs<<<blocks_for(V), kThreads, 0, st>>>(h->d_ck, h->d_idx, h->d_pos, h->d_roots, h->d_counts,
+                                             h->d_deepRuns, h->d_sHi, h->d_sLo, V,
+                                             h->params.nodesPerCell, h->gbits);
   const size_t fixSmem = (size_t)GVIZ_FIX_MAX * 20;
   k_sort_runs<<<148, 512, fixSmem, st>>>(h->d_sHi, h->d_sLo, h->d_idx,
                                           h->d_deepRuns, h->d_counts,
                                           h->d_status);
-  k_bucket_flags<<<blocks_for(V), kThreads, 0, st>>>(h->d_sHi, h->d_sLo,
-                                                     h->d_idx, h->d_gid,
-                                                     h->d_flag, V);
-  scan_exclusive(h, h->d_flag, h->d_scan, V, h->d_counts + 2);
-  k_bucket_fill<<<blocks_for(V), kThreads, 0, st>>>(
-      h->d_flag, h->d_scan, h->d_sHi, h->d_sLo, h->d_idx, h->d_gid,
-      h->d_bStart, h->d_bHi, h->d_bLo, h->d_bGid, h->d_upLeaf, V);
+  k_buckets<<<(V + GVIZ_SCAN_TILE - 1) / GVIZ_SCAN_TILE, kThreads, 0, st>>>(
+      h->d_sHi, h->d_sLo, h->d_ck, h->d_bStart, h->d_bHi, h->d_bLo, h->d_bGid, h->d_upLeaf,
+      h->d_scanState, h->d_counts + 2, h->d_status, V, h->gbits);
   prof_mark(h, "tree_buckets");
   k_karras<<<blocks_for(V), kThreads, 0, st>>>(
       h->d_bHi, h->d_bLo, h->G > 1 ? h->d_bGid : nullptr, h->d_counts, h->d_nLeft, h->d_nRight,
