@@ -76,6 +76,7 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_judgeExact);
   dfree(h->d_judgeOut);
   dfree(h->d_judgeRep);
+  dfree(h->d_judgePart);
   dfree(h->d_rowOff);
   dfree(h->d_cols);
   dfree(h->d_degree);
@@ -417,9 +418,11 @@ static int far_judge(gvizCudaForce *h) {
     dfree(h->d_judgeIdx);
     dfree(h->d_judgeExact);
     dfree(h->d_judgeOut);
+    dfree(h->d_judgePart);
     h->judgeN = 0;
     int rc = dalloc(h, &h->d_judgeIdx, n) | dalloc(h, &h->d_judgeExact, n) |
-             dalloc(h, &h->d_judgeOut, 2 * (size_t)n);
+             dalloc(h, &h->d_judgeOut, 2 * (size_t)n) |
+             dalloc(h, &h->d_judgePart, (size_t)exact_judge_splits(h->V, n) * n);
     if (!h->d_judgeRep) rc |= dalloc(h, &h->d_judgeRep, h->V);
     if (rc) return set_err(h, GVIZ_CUDA_ERR_ALLOC);
     const std::vector<uint32_t> idx = judge_sample(h->V, n, h->judgeSeed);
@@ -428,7 +431,7 @@ static int far_judge(gvizCudaForce *h) {
     h->judgeN = n;
   }
   cudaMemsetAsync(h->d_status, 0, 4, h->stream);
-  enqueue_exact_judge(h, h->d_judgeIdx, n, h->d_judgeExact);
+  enqueue_exact_judge(h, h->d_judgeIdx, n, h->d_judgeExact, h->d_judgePart);
   judge_eval(h, h->d_judgeOut);  // the learned walk as configured
   const gvizCudaForceParams saved = h->params;
   const bool savedSide = h->farSide;
@@ -1305,17 +1308,19 @@ int gvizCudaForceExactRepulsion(gvizCudaForce *h, const uint32_t *targets,
     if (targets[i] >= h->V) return set_err(h, GVIZ_CUDA_ERR_ARG);
   DeviceGuard guard(h->device);
   uint32_t *dt = nullptr;
-  double2 *dout = nullptr;
-  int rc = dalloc(h, &dt, n) | dalloc(h, &dout, n);
+  double2 *dout = nullptr, *part = nullptr;
+  int rc = dalloc(h, &dt, n) | dalloc(h, &dout, n) |
+           dalloc(h, &part, (size_t)exact_judge_splits(h->V, n) * n);
   if (!rc) {
     cudaMemcpy(dt, targets, n * 4, cudaMemcpyHostToDevice);
-    enqueue_exact_judge(h, dt, n, dout);
+    enqueue_exact_judge(h, dt, n, dout, part);
     rc = sync_and_check(h);
     if (!rc && cudaMemcpy(out, dout, n * 16, cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = set_err(h, GVIZ_CUDA_ERR_CUDA);
   }
   dfree(dt);
   dfree(dout);
+  dfree(part);
   return rc;
 }
 

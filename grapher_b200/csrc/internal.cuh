@@ -225,6 +225,7 @@ struct gvizCudaForce {
   uint32_t *d_judgeIdx = nullptr;  // sampled vertices, ascending
   double2 *d_judgeExact = nullptr, *d_judgeOut = nullptr;  // n; 2n (learned, plain)
   double2 *d_judgeRep = nullptr;   // V: repulsion of one evaluation
+  double2 *d_judgePart = nullptr;  // split sums of the exact repulsion
 
   // --- CUDA graph of one step ---
   cudaGraphExec_t stepExec = nullptr;
@@ -328,4 +329,5 @@ void enqueue_walk_f64(gvizCudaForce *h);
 void enqueue_exact_f64(gvizCudaForce *h);
 void enqueue_fa2(gvizCudaForce *h);
 void enqueue_exact_judge(gvizCudaForce *h, const uint32_t *d_targets,
-                         size_t n, double2 *d_out);
+                         size_t n, double2 *d_out, double2 *partial);
+uint32_t exact_judge_splits(size_t V, size_t n);
