@@ -121,6 +121,7 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_stats);
   dfree(h->d_lastStats);
   dfree(h->d_chunkStat);
+  dfree(h->d_chunksDone);
   dfree(h->d_zero);
   dfree(h->d_roots);
   dfree(h->d_ck);
@@ -191,19 +192,24 @@ int upload_radius(gvizCudaForce *h) {
 
 void enqueue_step(gvizCudaForce *h) {
   cudaStream_t st = h->stream;
-  cudaMemsetAsync(h->d_status, 0, sizeof(uint32_t), st);
-  cudaMemcpyAsync(h->d_sfOld, h->d_sf, h->V * sizeof(double2),
-                  cudaMemcpyDeviceToDevice, st);
   const bool f64 = h->params.precision == GVIZ_CUDA_FP64;
   const bool bh = h->params.barnesHutEnabled != 0;
+  if (!bh) cudaMemsetAsync(h->d_status, 0, sizeof(uint32_t), st);  // a tree build zeroes it
+  // the old force is copied aside: reading it from where the walk writes the
+  // new one, in path order, takes 1.20 instead of 0.71 ms at 1,048,576
+  // vertices (reads of sectors half written)
+  const auto keep_old_force = [h](cudaStream_t s) {
+    cudaMemcpyAsync(h->d_sfOld, h->d_sf, h->V * sizeof(double2), cudaMemcpyDeviceToDevice, s);
+  };
   // attraction reads positions only and its forces are first read by the
-  // repulsion pass: with a tree to build it runs on the side stream,
+  // repulsion pass: with a tree to build it (and the copy) runs on the side stream,
   // overlapping the build (in order while profiling, so that each kernel
   // keeps its own time)
   const bool overlap = bh && h->side && !h->profiling;
   if (overlap) {
     cudaEventRecord(h->evFork, st);
     cudaStreamWaitEvent(h->side, h->evFork, 0);
+    keep_old_force(h->side);
     h->stream = h->side;
     if (f64)
       enqueue_attraction_f64(h);
@@ -214,6 +220,7 @@ void enqueue_step(gvizCudaForce *h) {
     enqueue_tree_build(h);
     cudaStreamWaitEvent(st, h->evJoin, 0);
   } else {
+    keep_old_force(st);
     if (bh) enqueue_tree_build(h);
     if (f64)
       enqueue_attraction_f64(h);
@@ -687,6 +694,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   rc |= dalloc(h, &h->d_stats, (size_t)GVIZ_STATS_CAP * G * 5);
   rc |= dalloc(h, &h->d_lastStats, G * 5);
   rc |= dalloc(h, &h->d_chunkStat, C);
+  rc |= dalloc(h, &h->d_chunksDone, G);
   {
     size_t bytes = 0;
     auto part = [&bytes](size_t count, size_t size) {
@@ -795,6 +803,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   up(h->d_hubChunkE0, hcE0.data(), hcE0.size() * 4);
   up(h->d_hubChunkE1, hcE1.data(), hcE1.size() * 4);
   ok = ok && cudaMemset(h->d_nCounter, 0, Vs * 4) == cudaSuccess;
+  ok = ok && cudaMemset(h->d_chunksDone, 0, G * 4) == cudaSuccess;
   ok = ok && cudaMemset(h->d_pos, 0, Vs * 16) == cudaSuccess;
   ok = ok && cudaMemset(h->d_counters, 0, 64) == cudaSuccess;
   if (!ok || upload_dir_table(h) || upload_radius(h)) {

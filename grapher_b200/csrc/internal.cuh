@@ -157,6 +157,7 @@ struct gvizCudaForce {
   uint32_t walkStackCap = 0;  // FP32 walks: the caller's stack entries per warp (0: not set)
   uint32_t walkTunedCap = 0;  // plain walk: the autotuner's stack entries (0: not tuned)
   ChunkStat *d_chunkStat = nullptr;
+  uint32_t *d_chunksDone = nullptr;  // per graph: chunks that finished a sum
   uint32_t *d_status = nullptr;
 
   // --- tree build scratch (device) ---

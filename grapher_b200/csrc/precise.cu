@@ -14,6 +14,8 @@
 
 #include <algorithm>
 
+#include <cuda/atomic>
+
 #include "epilogue.cuh"
 #include "internal.cuh"
 
@@ -377,6 +379,7 @@ struct Fa2Args {
   const double2 *disp;
   double2 *pos, *applied;
   ChunkStat *chunkStat;
+  uint32_t *chunksDone;  // per graph, zero between kernels
   double *speed, *eff, *stats, *lastStats;
   uint32_t *active, *anyActive;
   uint64_t *iter, *runLeft;
@@ -410,30 +413,25 @@ __device__ __forceinline__ double block_max(double v, double *sh) {
   return r;
 }
 
-__global__ __launch_bounds__(kThreads) void k_fa2_chunks(Fa2Args a) {
-  __shared__ double sh[kThreads / 32];
-  const uint32_t c = blockIdx.x;
-  const uint32_t g = a.chunkGraph[c];
-  if (!a.active[g]) return;
-  double sw = 0.0, tr = 0.0;
-  for (uint32_t v = a.chunkBegin[c] + threadIdx.x; v < a.chunkEnd[c]; v += kThreads) {
-    sw += a.swing[v];
-    tr += a.trac[v];
-  }
-  sw = block_sum(sw, sh);
-  tr = block_sum(tr, sh);
+// Whether this block is the last of its graph's chunks to get here: its
+// chunk's sums are visible to that block, and the counter is zero again for
+// the next kernel. For the whole block, after thread 0 wrote the sums.
+__device__ __forceinline__ bool last_chunk(const Fa2Args &a, uint32_t g) {
+  __shared__ uint32_t sLast;
   if (threadIdx.x == 0) {
-    a.chunkStat[c].a = sw;
-    a.chunkStat[c].b = tr;
+    cuda::atomic_ref<uint32_t, cuda::thread_scope_device> done(a.chunksDone[g]);
+    const uint32_t n = a.gChunkEnd[g] - a.gChunkBegin[g];
+    sLast = done.fetch_add(1u, cuda::memory_order_acq_rel) == n - 1u;
+    if (sLast) done.store(0u, cuda::memory_order_relaxed);
   }
+  __syncthreads();
+  return sLast != 0u;
 }
 
-// updateGlobalSpeed, src/embedders/gvizForceEmbedder.c:140-185, per graph
-// One block per graph; thread 0 applies the rule to the block's sums.
-__global__ __launch_bounds__(kThreads) void k_fa2_speed(Fa2Args a) {
-  __shared__ double sh[kThreads / 32];
-  const uint32_t g = blockIdx.x;
-  if (!a.active[g]) return;
+// updateGlobalSpeed, src/embedders/gvizForceEmbedder.c:140-185, per graph:
+// thread 0 applies the rule to the block's sums of the graph's chunks (or,
+// strict, to the vertices in order).
+__device__ void fa2_speed(const Fa2Args &a, uint32_t g, double *sh) {
   double totalSwing = 0.0, totalTraction = 0.0;
   if (a.strict) {
     if (threadIdx.x == 0)
@@ -443,8 +441,8 @@ __global__ __launch_bounds__(kThreads) void k_fa2_speed(Fa2Args a) {
       }
   } else {
     for (uint32_t c = a.gChunkBegin[g] + threadIdx.x; c < a.gChunkEnd[g]; c += kThreads) {
-      totalSwing += a.chunkStat[c].a;
-      totalTraction += a.chunkStat[c].b;
+      totalSwing += __ldcg(&a.chunkStat[c].a);
+      totalTraction += __ldcg(&a.chunkStat[c].b);
     }
     totalSwing = block_sum(totalSwing, sh);
     totalTraction = block_sum(totalTraction, sh);
@@ -478,42 +476,42 @@ __global__ __launch_bounds__(kThreads) void k_fa2_speed(Fa2Args a) {
   a.eff[g] = eff;
 }
 
-// applySpeedRange (:187-197) + position update and stat partials (:467-477)
-__global__ __launch_bounds__(kThreads) void k_fa2_apply(Fa2Args a) {
+// Swing and traction sums of every chunk; the last chunk of a graph to finish
+// adds them up and applies the speed rule. A chunk's loads are all in flight
+// at once (a serial chain of them is what a block would otherwise take its
+// time with); every sum keeps its fixed order: strided per-thread partials,
+// the block's tree, the chunks in order.
+__global__ __launch_bounds__(kThreads) void k_fa2_speed(Fa2Args a) {
   __shared__ double sh[kThreads / 32];
   const uint32_t c = blockIdx.x;
   const uint32_t g = a.chunkGraph[c];
   if (!a.active[g]) return;
-  const double speed = a.speed[g];
-  double mx = 0.0, sAtt = 0.0, sRep = 0.0;
-  for (uint32_t v = a.chunkBegin[c] + threadIdx.x; v < a.chunkEnd[c]; v += kThreads) {
-    const double factor = speed / (1.0 + sqrt(speed * a.swing[v]));
-    const double2 f = a.disp[v];
-    const double2 o = make_double2(f.x * factor, f.y * factor);
-    a.applied[v] = o;
-    const double nrm = sqrt(o.x * o.x + o.y * o.y);
-    mx = fmax(mx, nrm);
-    sAtt += a.att[v];
-    sRep += a.rep[v];
-    double2 p = a.pos[v];
-    p.x += o.x;
-    p.y += o.y;
-    a.pos[v] = p;
+  constexpr int kItems = GVIZ_CHUNK / kThreads;
+  const uint32_t v0 = a.chunkBegin[c] + threadIdx.x, v1 = a.chunkEnd[c];
+  double swing[kItems], trac[kItems];
+#pragma unroll
+  for (int r = 0; r < kItems; r++) {
+    const uint32_t v = v0 + r * kThreads;
+    swing[r] = v < v1 ? a.swing[v] : 0.0;
+    trac[r] = v < v1 ? a.trac[v] : 0.0;
   }
-  mx = block_max(mx, sh);
-  sAtt = block_sum(sAtt, sh);
-  sRep = block_sum(sRep, sh);
+  double sw = 0.0, tr = 0.0;
+#pragma unroll
+  for (int r = 0; r < kItems; r++) {
+    sw += swing[r];  // (adding zeros past the end changes nothing)
+    tr += trac[r];
+  }
+  sw = block_sum(sw, sh);
+  tr = block_sum(tr, sh);
   if (threadIdx.x == 0) {
-    a.chunkStat[c].a = mx;
-    a.chunkStat[c].b = sAtt;
-    a.chunkStat[c].c = sRep;
+    a.chunkStat[c].a = sw;
+    a.chunkStat[c].b = tr;
   }
+  if (last_chunk(a, g)) fa2_speed(a, g, sh);
 }
 
-__global__ __launch_bounds__(kThreads) void k_fa2_stats(Fa2Args a) {
-  __shared__ double sh[kThreads / 32];
-  const uint32_t g = blockIdx.x;
-  if (!a.active[g]) return;
+// The step tail's statistics of graph g (:478-492) and its Run bookkeeping.
+__device__ void fa2_stats(const Fa2Args &a, uint32_t g, double *sh) {
   double mx = 0.0, sAtt = 0.0, sRep = 0.0;
   if (a.strict) {
     if (threadIdx.x == 0)
@@ -526,9 +524,9 @@ __global__ __launch_bounds__(kThreads) void k_fa2_stats(Fa2Args a) {
       }
   } else {
     for (uint32_t c = a.gChunkBegin[g] + threadIdx.x; c < a.gChunkEnd[g]; c += kThreads) {
-      mx = fmax(mx, a.chunkStat[c].a);
-      sAtt += a.chunkStat[c].b;
-      sRep += a.chunkStat[c].c;
+      mx = fmax(mx, __ldcg(&a.chunkStat[c].a));
+      sAtt += __ldcg(&a.chunkStat[c].b);
+      sRep += __ldcg(&a.chunkStat[c].c);
     }
     mx = block_max(mx, sh);
     sAtt = block_sum(sAtt, sh);
@@ -553,6 +551,68 @@ __global__ __launch_bounds__(kThreads) void k_fa2_stats(Fa2Args a) {
   }
 }
 
+// applySpeedRange (:187-197), position update and the statistics' chunk sums
+// (:467-477); the last chunk of a graph to finish adds those up.
+__global__ __launch_bounds__(kThreads) void k_fa2_apply(Fa2Args a) {
+  __shared__ double sh[kThreads / 32];
+  const uint32_t c = blockIdx.x;
+  const uint32_t g = a.chunkGraph[c];
+  if (!a.active[g]) return;
+  const double speed = a.speed[g];
+  const uint32_t v0 = a.chunkBegin[c] + threadIdx.x, v1 = a.chunkEnd[c];
+  double mx = 0.0, sAtt = 0.0, sRep = 0.0;
+  constexpr int kItems = 4;  // a thread's loads in flight at once
+#pragma unroll
+  for (int b = 0; b < GVIZ_CHUNK / kThreads; b += kItems) {
+    double swing[kItems], att[kItems], rep[kItems];
+    double2 f[kItems], p[kItems];
+#pragma unroll
+    for (int r = 0; r < kItems; r++) {
+      const uint32_t v = v0 + (b + r) * kThreads;
+      if (v < v1) {
+        swing[r] = a.swing[v];
+        f[r] = a.disp[v];
+        att[r] = a.att[v];
+        rep[r] = a.rep[v];
+        p[r] = a.pos[v];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kItems; r++) {
+      const uint32_t v = v0 + (b + r) * kThreads;
+      if (v < v1) {
+        const double factor = speed / (1.0 + sqrt(speed * swing[r]));
+        const double2 o = make_double2(f[r].x * factor, f[r].y * factor);
+        a.applied[v] = o;
+        const double nrm = sqrt(o.x * o.x + o.y * o.y);
+        mx = fmax(mx, nrm);
+        sAtt += att[r];
+        sRep += rep[r];
+        a.pos[v] = make_double2(p[r].x + o.x, p[r].y + o.y);
+      }
+    }
+  }
+  mx = block_max(mx, sh);
+  sAtt = block_sum(sAtt, sh);
+  sRep = block_sum(sRep, sh);
+  if (threadIdx.x == 0) {
+    a.chunkStat[c].a = mx;
+    a.chunkStat[c].b = sAtt;
+    a.chunkStat[c].c = sRep;
+  }
+  if (last_chunk(a, g) && !a.strict) fa2_stats(a, g, sh);
+}
+
+// Strict reductions: one block per graph, thread 0 sums the vertices in order.
+__global__ __launch_bounds__(kThreads) void k_fa2_speed_strict(Fa2Args a) {
+  __shared__ double sh[kThreads / 32];
+  if (a.active[blockIdx.x]) fa2_speed(a, blockIdx.x, sh);
+}
+__global__ __launch_bounds__(kThreads) void k_fa2_stats_strict(Fa2Args a) {
+  __shared__ double sh[kThreads / 32];
+  if (a.active[blockIdx.x]) fa2_stats(a, blockIdx.x, sh);
+}
+
 inline uint32_t blocks(size_t n, int t) { return (uint32_t)((n + t - 1) / t); }
 
 Fa2Args make_fa2(gvizCudaForce *h) {
@@ -572,6 +632,7 @@ Fa2Args make_fa2(gvizCudaForce *h) {
   a.pos = h->d_pos;
   a.applied = h->d_applied;
   a.chunkStat = h->d_chunkStat;
+  a.chunksDone = h->d_chunksDone;
   a.speed = h->d_speed;
   a.eff = h->d_eff;
   a.stats = h->d_stats;
@@ -693,10 +754,13 @@ void enqueue_exact_judge(gvizCudaForce *h, const uint32_t *d_targets, size_t n,
 void enqueue_fa2(gvizCudaForce *h) {
   Fa2Args a = make_fa2(h);
   const uint32_t G = (uint32_t)h->G;
-  if (!h->params.strictReductions)
-    k_fa2_chunks<<<h->nChunks, kThreads, 0, h->stream>>>(a);
-  k_fa2_speed<<<G, kThreads, 0, h->stream>>>(a);
-  k_fa2_apply<<<h->nChunks, kThreads, 0, h->stream>>>(a);
-  k_fa2_stats<<<G, kThreads, 0, h->stream>>>(a);
+  if (a.strict) {
+    k_fa2_speed_strict<<<G, kThreads, 0, h->stream>>>(a);
+    k_fa2_apply<<<h->nChunks, kThreads, 0, h->stream>>>(a);
+    k_fa2_stats_strict<<<G, kThreads, 0, h->stream>>>(a);
+  } else {
+    k_fa2_speed<<<h->nChunks, kThreads, 0, h->stream>>>(a);
+    k_fa2_apply<<<h->nChunks, kThreads, 0, h->stream>>>(a);
+  }
   prof_mark(h, "fa2_update");
 }
