@@ -103,6 +103,7 @@ struct gvizCudaForce {
   // host copies
   uint64_t *h_graphOff = nullptr;  // G+1
   double *h_meanDegPlusOne = nullptr;
+  double *h_tail = nullptr;  // pinned: d_lastStats, then the status (finish_step)
   uint32_t nChunks = 0;
 
   // --- structure (device) ---
