@@ -131,7 +131,7 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_sHi);
   dfree(h->d_sLo);
   dfree(h->d_flag);
-  dfree(h->d_scan);
+  dfree(h->d_pre);
   dfree(h->d_deepRuns);
   dfree(h->d_bHi);
   dfree(h->d_bLo);
@@ -715,7 +715,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
       return at;
     };
     const size_t atStatus = part(1, 4), atCounts = part(8, 4), atBox = part(4 * G, 8),
-                 atRootT = part(G, 4), atScan = part(scan_state_entries(std::max(Vs, G)), 8),
+                 atRootT = part(G, 4), atTop = part(top_count_entries(Vs), 4), atScan = part(scan_state_entries(std::max(Vs, G)), 8),
                  atSort = part(sort_state_entries(Vs), 4);
     char *zero = nullptr;
     rc |= dalloc(h, &zero, bytes);
@@ -726,6 +726,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
       h->d_counts = reinterpret_cast<uint32_t *>(zero + atCounts);
       h->d_box = reinterpret_cast<unsigned long long *>(zero + atBox);
       h->d_rootT = reinterpret_cast<uint32_t *>(zero + atRootT);
+      h->d_topCount = reinterpret_cast<uint32_t *>(zero + atTop);
       h->d_scanState = reinterpret_cast<uint64_t *>(zero + atScan);
       h->d_sortState = reinterpret_cast<uint32_t *>(zero + atSort);
       if (cudaMemset(zero, 0, bytes) != cudaSuccess) rc |= GVIZ_CUDA_ERR_CUDA;
@@ -739,7 +740,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   rc |= dalloc(h, &h->d_sHi, Vs);
   rc |= dalloc(h, &h->d_sLo, Vs);
   rc |= dalloc(h, &h->d_flag, Vs);
-  rc |= dalloc(h, &h->d_scan, Vs);
+  rc |= dalloc(h, &h->d_pre, Vs);
   rc |= dalloc(h, &h->d_deepRuns, 2 * Vs);
   rc |= dalloc(h, &h->d_bHi, Vs);
   rc |= dalloc(h, &h->d_bLo, Vs);
@@ -815,6 +816,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   up(h->d_hubChunkE0, hcE0.data(), hcE0.size() * 4);
   up(h->d_hubChunkE1, hcE1.data(), hcE1.size() * 4);
   ok = ok && cudaMemset(h->d_nCounter, 0, Vs * 4) == cudaSuccess;
+  ok = ok && cudaMemset(h->d_graphBase, 0, G * 4) == cudaSuccess;
   ok = ok && cudaMemset(h->d_chunksDone, 0, G * 4) == cudaSuccess;
   ok = ok && cudaMemset(h->d_pos, 0, Vs * 16) == cudaSuccess;
   ok = ok && cudaMemset(h->d_counters, 0, 64) == cudaSuccess;

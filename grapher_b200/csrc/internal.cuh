@@ -172,7 +172,9 @@ struct gvizCudaForce {
   uint64_t *d_ck = nullptr, *d_ckAlt = nullptr;     // composite sort keys
   uint32_t *d_idx = nullptr, *d_idxAlt = nullptr;   // sorted vertex ids
   uint64_t *d_sHi = nullptr, *d_sLo = nullptr;      // full keys, sorted order
-  uint32_t *d_flag = nullptr, *d_scan = nullptr;    // V-sized
+  uint32_t *d_flag = nullptr;      // V: level-1 lists of the nodes above blocks
+  uint2 *d_pre = nullptr;          // V: their places, then preorder positions (k_top)
+  uint32_t *d_topCount = nullptr;  // per super-range: nodes listed (part of d_zero)
   uint32_t *d_deepRuns = nullptr;
   uint32_t *d_counts = nullptr;  // [1]=deep runs [2]=buckets [3]=nodes
   uint32_t *d_sortState = nullptr;  // radix sort: look-back status, digit counts, tickets
@@ -305,6 +307,7 @@ uint32_t *sort_digit_counts(gvizCudaForce *h);
 size_t scan_state_entries(size_t n);
 
 // tree.cu
+size_t top_count_entries(size_t V);
 void enqueue_tree_build(gvizCudaForce *h);
 void enqueue_tree_export(gvizCudaForce *h, int32_t *leafDepth);
 void enqueue_group_export(gvizCudaForce *h, uint32_t *groupOf);

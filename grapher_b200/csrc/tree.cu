@@ -10,12 +10,12 @@
 //   stable radix sort of (graph, path) -> fix-up sort of equal-prefix runs
 //   buckets = identical full paths -> Karras binary radix tree (2012)
 //   binary nodes merged into quadtree nodes (two path bits per level)
-//   bottom-up mass / centre-of-mass / subtree sizes (arrival counters):
-//     inside blocks of 256 buckets through shared memory, then the few
-//     nodes spanning blocks on a persistent grid
-//   preorder index of the spanning nodes by walking up weighted parent
-//   links, then every node record, its own walk up stopping at the first
-//   spanning ancestor
+//   bottom-up mass / centre-of-mass / subtree sizes (arrival counters)
+//     through shared memory: blocks of 256 buckets, then blocks of 4,096 for
+//     the few nodes spanning those, then one block for the rest; the last two
+//     also give those nodes' preorder positions
+//   every node record at its preorder position, its own walk up weighted
+//   parent links stopping at the first ancestor above blocks
 //
 // Why the compressed tree walks like the reference's: a chain of single-child
 // nodes shares one point set, hence one mass and centre of mass; the
@@ -33,6 +33,15 @@
 
 #include "internal.cuh"
 #include "scan.cuh"
+
+// Super-ranges such that neither level's lists outgrow k_top's shared memory:
+// about 8 nodes span a block's edge, so 2^12, 2^14 and 2^16 buckets have
+// level-1 lists of ~120, ~500 and ~2,000 nodes, and level 2 has as many per
+// 16, 64 and 256 super-ranges.
+static int super_bits(size_t V) { return V <= (1u << 17) ? 12 : (V <= (1u << 21) ? 14 : 16); }
+
+// super-ranges of the tree build's nodes above blocks (see node_level)
+size_t top_count_entries(size_t V) { return (V >> super_bits(V)) + 1; }
 
 namespace {
 
@@ -425,31 +434,38 @@ __device__ __forceinline__ int bdelta(int a, int b, const KarrasKeys &k) {
   return 160;
 }
 
-// Karras, "Maximizing parallelism in the construction of BVHs, octrees and
-// k-d trees" (HPG 2012), algorithm of section 4 over unique bucket keys.
-// Block j finds nodes [256 j, 256 j + 256); the keys of the 256 buckets on
-// either side are staged in shared memory first, where most of the
-// searches stay.
-__global__ __launch_bounds__(kThreads) void k_karras(
-    const uint64_t *__restrict__ bHi, const uint64_t *__restrict__ bLo,
-    const uint32_t *__restrict__ bGid, const uint32_t *__restrict__ counts,
-    uint32_t *nLeft, uint32_t *nRight, uint32_t *nFirst, uint32_t *nLast,
-    int32_t *nDelta, uint2 *upInt, uint2 *upLeaf) {
-  __shared__ uint64_t sHi[kKarrasTile], sLo[kKarrasTile];
-  const int U = (int)counts[2];
-  const int B0 = (int)(blockIdx.x * kThreads);
-  if (B0 >= U - 1) return;
-  KarrasKeys k{bHi, bLo, bGid, sHi, sLo, B0 - kThreads, U};
-  for (int j = threadIdx.x; j < kKarrasTile; j += kThreads) {
-    const int b = k.T0 + j;
-    if (b >= 0 && b < U) {
-      sHi[j] = bHi[b];
-      sLo[j] = bLo[b];
-    }
-  }
-  __syncthreads();
-  const int i = B0 + threadIdx.x;
-  if (i >= U - 1) return;
+// A node's sums are made by the smallest unit that holds all its buckets:
+// level 0, a block of k_bottom_up (256 buckets); level 1, a block of k_top
+// over a super-range of 2^superBits buckets; level 2, k_top's single block for
+// the rest. Nodes that join graphs (a common prefix inside the graph id) are
+// of no level. A Karras node is one end of its own range, so its index places
+// it.
+__device__ __forceinline__ int node_level(uint32_t p, int delta, uint32_t first, uint32_t last,
+                                          uint32_t U, int superBits) {
+  if (delta < 32) return 0;
+  const uint32_t B0 = p & ~(uint32_t)(kThreads - 1);
+  if (first >= B0 && last < min(B0 + kThreads, U)) return 0;
+  return (first >> superBits) == (last >> superBits) ? 1 : 2;
+}
+
+// The listed nodes: those of level 1 by super-range (its list starts at its
+// first bucket's index), those of level 2; and per node {kPreLocal, -} or,
+// until k_top replaces it by the node's preorder position, {kPreListed +
+// level, its place in its list}.
+struct TopLists {
+  uint32_t *list1, *count1, *list2, *count2;
+  uint2 *pre;
+  int superBits;
+};
+constexpr uint32_t kPreLocal = 0xFFFFFFFEu;
+constexpr uint32_t kPreListed = 0xFFFFFF00u;  // + level
+
+// Node i of the binary radix tree (Karras 2012, algorithm of section 4);
+// returns its level (node_level).
+__device__ __forceinline__ int karras_node(int i, const KarrasKeys &k, uint32_t *nLeft,
+                                           uint32_t *nRight, uint32_t *nFirst, uint32_t *nLast,
+                                           int32_t *nDelta, uint2 *upInt, uint2 *upLeaf,
+                                           int superBits) {
   const int dir = (bdelta(i, i + 1, k) - bdelta(i, i - 1, k)) >= 0 ? 1 : -1;
   const int dmin = bdelta(i, i - dir, k);
   int lmax = 2;
@@ -490,8 +506,55 @@ __global__ __launch_bounds__(kThreads) void k_karras(
   nLast[i] = (uint32_t)last;
   nDelta[i] = dnode;
   if (i == 0) upInt[0].x = GVIZ_NONE;
+  return node_level((uint32_t)i, dnode, (uint32_t)first, (uint32_t)last, (uint32_t)k.U,
+                    superBits);
 }
 
+// Karras, "Maximizing parallelism in the construction of BVHs, octrees and
+// k-d trees" (HPG 2012), algorithm of section 4 over unique bucket keys.
+// Block j finds nodes [256 j, 256 j + 256); the keys of the 256 buckets on
+// either side are staged in shared memory first, where most of the
+// searches stay.
+__global__ __launch_bounds__(kThreads) void k_karras(
+    const uint64_t *__restrict__ bHi, const uint64_t *__restrict__ bLo,
+    const uint32_t *__restrict__ bGid, const uint32_t *__restrict__ counts,
+    uint32_t *nLeft, uint32_t *nRight, uint32_t *nFirst, uint32_t *nLast,
+    int32_t *nDelta, uint2 *upInt, uint2 *upLeaf, TopLists top) {
+  __shared__ uint64_t sHi[kKarrasTile], sLo[kKarrasTile];
+  __shared__ uint32_t sCount[2], sBase[2];
+  const int U = (int)counts[2];
+  const int B0 = (int)(blockIdx.x * kThreads);
+  if (B0 >= U - 1) return;
+  if (threadIdx.x < 2) sCount[threadIdx.x] = 0u;
+  KarrasKeys k{bHi, bLo, bGid, sHi, sLo, B0 - kThreads, U};
+  for (int j = threadIdx.x; j < kKarrasTile; j += kThreads) {
+    const int b = k.T0 + j;
+    if (b >= 0 && b < U) {
+      sHi[j] = bHi[b];
+      sLo[j] = bLo[b];
+    }
+  }
+  __syncthreads();
+  const int i = B0 + threadIdx.x;
+  int level = 0;
+  if (i < U - 1)
+    level = karras_node(i, k, nLeft, nRight, nFirst, nLast, nDelta, upInt, upLeaf, top.superBits);
+  // the block's nodes above blocks join their level's list
+  uint32_t at = 0;
+  if (level > 0) at = atomicAdd(&sCount[level - 1], 1u);
+  __syncthreads();
+  if (threadIdx.x < 2 && sCount[threadIdx.x])
+    sBase[threadIdx.x] = atomicAdd(threadIdx.x ? top.count2 : top.count1 + (B0 >> top.superBits),
+                                   sCount[threadIdx.x]);
+  __syncthreads();
+  if (level > 0) {
+    at += sBase[level - 1];
+    (level == 1 ? top.list1 + ((B0 >> top.superBits) << top.superBits) : top.list2)[at] = (uint32_t)i;
+    top.pre[i] = make_uint2(kPreListed + (uint32_t)level, at);
+  } else if (i < U - 1) {
+    top.pre[i] = make_uint2(kPreLocal, 0u);
+  }
+}
 struct BU {
   const uint32_t *idx, *bStart, *bGid, *counts, *nLeft, *nRight, *nFirst, *nLast;
   const int32_t *nDelta;
@@ -504,11 +567,17 @@ struct BU {
   // second central moments {Qxx, Qxy, Qyy, -}, or null: summed and shifted
   // in FP64, stored in FP32 (they only feed FP32 features)
   float4 *bQ, *nQ;
-  // nodes spanning blocks whose children are both summed when k_bottom_up
-  // ends (counts[4] of them)
-  uint32_t *ready;
+  TopLists top;
+  uint32_t *total;  // single graph: the number of records (else null)
   uint32_t V, k;
 };
+
+// x is its graph's root: T records
+__device__ __forceinline__ void put_root(const BU &a, uint32_t g, uint32_t x, uint32_t T) {
+  a.rootNode[g] = x;
+  a.rootT[g] = T;
+  if (a.total) *a.total = T;
+}
 
 // second central moments of a child about its own centre of mass
 __device__ __forceinline__ float4 child_q(const BU &a, uint32_t c) {
@@ -557,48 +626,70 @@ __device__ __forceinline__ uint2 *up_of(const BU &a, uint32_t c) {
   return (c & GVIZ_LEAF_BIT) ? a.upLeaf + (c & ~GVIZ_LEAF_BIT) : a.upInt + c;
 }
 
-// Node p from its children l, r (left first: fixed order, deterministic
+// A node from its children's sums (left first: fixed order, deterministic
 // sums): mass, mass-weighted position sums, point count, subtree size in
-// emitted records, the absorbed (p shares its quadtree level with its parent
-// pp) and collapsed (a capacity leaf) flags and its children's preorder link
-// weights; with kQ the second moments about p's centre of mass.
+// emitted records, the absorbed and collapsed (a capacity leaf) flags and its
+// children's preorder link weights wl, wr; with kQ the second moments about
+// its centre of mass.
+struct TopSums {
+  double M, SX, SY;
+  uint32_t cnt, T;
+  float4 q;
+};
+
+struct Combined {
+  TopSums s;
+  uint32_t flag, wl, wr;
+};
+
 template <bool kQ>
-__device__ __forceinline__ void combine(const BU &a, uint32_t p, int dp, uint32_t pp, int dpp,
-                                        uint32_t l, uint32_t r, double Ml, double SXl,
-                                        double SYl, uint32_t cl, uint32_t Tl, float4 ql,
-                                        double Mr, double SXr, double SYr, uint32_t cr,
-                                        uint32_t Tr, float4 qr, double &M, double &SX,
-                                        double &SY, uint32_t &cnt, uint32_t &T,
-                                        float4 &q) {
-  M = Ml + Mr;
-  SX = SXl + SXr;
-  SY = SYl + SYr;
-  cnt = cl + cr;
-  const bool absorbed = pp != GVIZ_NONE && dpp >= 32 && ((dp - 32) >> 1) == ((dpp - 32) >> 1);
-  const bool collapsed = !absorbed && cnt <= a.k;
-  T = absorbed ? Tl + Tr : (collapsed ? 1u + cnt : 1u + Tl + Tr);
+__device__ __forceinline__ Combined combined(const BU &a, bool absorbed, const TopSums &L,
+                                             const TopSums &R) {
+  Combined c;
+  c.s.M = L.M + R.M;
+  c.s.SX = L.SX + R.SX;
+  c.s.SY = L.SY + R.SY;
+  c.s.cnt = L.cnt + R.cnt;
+  const bool collapsed = !absorbed && c.s.cnt <= a.k;
+  c.s.T = absorbed ? L.T + R.T : (collapsed ? 1u + c.s.cnt : 1u + L.T + R.T);
+  c.s.q = make_float4(0.f, 0.f, 0.f, 0.f);
   if (kQ) {
     double px = 0.0, py = 0.0;
-    if (M > 1e-9 || M < -1e-9) {
-      const double im = __drcp_rn(M);  // one reciprocal on the serial climb
-      px = SX * im;
-      py = SY * im;
+    if (c.s.M > 1e-9 || c.s.M < -1e-9) {
+      const double im = __drcp_rn(c.s.M);  // one reciprocal on the serial climb
+      px = c.s.SX * im;
+      py = c.s.SY * im;
     }
-    q = make_float4(0.f, 0.f, 0.f, 0.f);
-    add_shifted(q, ql, Ml, SXl, SYl, px, py);
-    add_shifted(q, qr, Mr, SXr, SYr, px, py);
-    a.nQ[p] = q;
+    add_shifted(c.s.q, L.q, L.M, L.SX, L.SY, px, py);
+    add_shifted(c.s.q, R.q, R.M, R.SX, R.SY, px, py);
   }
-  a.nM[p] = M;
-  a.nSX[p] = SX;
-  a.nSY[p] = SY;
-  a.nCnt[p] = cnt;
-  a.nT[p] = T;
-  a.nFlag[p] = (absorbed ? 1u : 0u) | (collapsed ? 2u : 0u);
+  c.flag = (absorbed ? 1u : 0u) | (collapsed ? 2u : 0u);
   const uint32_t base = absorbed ? 0u : 1u;
   const uint32_t dead = collapsed ? 0x80000000u : 0u;
-  up_of(a, l)->y = base | dead;
-  up_of(a, r)->y = (base + Tl) | dead;
+  c.wl = base | dead;
+  c.wr = (base + L.T) | dead;
+  return c;
+}
+
+// c to global memory: node p's sums and flags and its children's link weights
+template <bool kQ>
+__device__ __forceinline__ void put_combined(const BU &a, uint32_t p, uint32_t l, uint32_t r,
+                                             const Combined &c) {
+  if (kQ) a.nQ[p] = c.s.q;
+  a.nM[p] = c.s.M;
+  a.nSX[p] = c.s.SX;
+  a.nSY[p] = c.s.SY;
+  a.nCnt[p] = c.s.cnt;
+  a.nT[p] = c.s.T;
+  a.nFlag[p] = c.flag;
+  up_of(a, l)->y = c.wl;
+  up_of(a, r)->y = c.wr;
+}
+
+// p, of delta dp, shares its quadtree level with its binary parent, of delta
+// dpp (none: dpp < 32): two path bits per level
+__device__ __forceinline__ bool is_absorbed(int dp, int dpp) {
+  return dpp >= 32 && ((dp - 32) >> 1) == ((dpp - 32) >> 1);
 }
 
 // Per-block shared state of k_bottom_up: the sums of the block's buckets
@@ -622,11 +713,8 @@ struct BUShared {
 // whose buckets all belong to this block has both children summed by
 // threads of this block: its arrivals meet in shared memory with block-scope
 // ordering and its children's sums are read from shared memory. A climb
-// stops at the first node spanning blocks: its arrivals use a device-scope
-// counter, and the second one lists the node for k_bottom_up_top. (A block
-// that carried its climbs to the root stayed resident for ~20 device-scope
-// steps, and the kernel ran in several such waves.) Every node's sums also
-// go to global memory (k_emit reads them).
+// stops at the first node spanning blocks, which k_top sums. Every node's
+// sums also go to global memory (k_emit reads them).
 template <bool kQ>
 __global__ __launch_bounds__(kThreads) void k_bottom_up(BU a) {
   __shared__ BUShared<kQ> s;
@@ -703,20 +791,11 @@ __global__ __launch_bounds__(kThreads) void k_bottom_up(BU a) {
     const bool pin = p >= B0 && p < B1;  // false for GVIZ_NONE
     const int dp = p == GVIZ_NONE ? 0 : (pin ? s.delta[p - B0] : a.nDelta[p]);
     if (p == GVIZ_NONE || dp < 32) {
-      a.rootNode[g] = x;
-      a.rootT[g] = T;
+      put_root(a, g, x, T);
       *up_of(a, x) = make_uint2(GVIZ_NONE, 0u);
       return;
     }
-    if (!pin || s.first[p - B0] < B0 || s.last[p - B0] >= B1) {
-      // a node spanning blocks: k_bottom_up_top sums it once both children
-      // are summed
-      cuda::atomic_ref<uint32_t, cuda::thread_scope_device> arrivals(a.nCounter[p]);
-      if (arrivals.fetch_add(1u, cuda::memory_order_acq_rel) == 0u) return;
-      a.nCounter[p] = 0u;
-      a.ready[atomicAdd(const_cast<uint32_t *>(a.counts) + 4, 1u)] = p;
-      return;
-    }
+    if (!pin || s.first[p - B0] < B0 || s.last[p - B0] >= B1) return;  // spans blocks
     const uint32_t l = s.left[p - B0], r = s.right[p - B0], pp = s.up[p - B0];
     const int dpp = pp == GVIZ_NONE ? 0
                     : ((pp >= B0 && pp < B1) ? s.delta[pp - B0] : a.nDelta[pp]);
@@ -725,115 +804,272 @@ __global__ __launch_bounds__(kThreads) void k_bottom_up(BU a) {
     // children lie in [B0, B1) and were summed by this block)
     cuda::atomic_ref<uint32_t, cuda::thread_scope_block> arrivals(s.arrive[p - B0]);
     if (arrivals.fetch_add(1u, cuda::memory_order_acq_rel) == 0u) return;
-    double Ml, SXl, SYl, Mr, SXr, SYr;
-    uint32_t cl, Tl, cr, Tr;
-    float4 ql = make_float4(0.f, 0.f, 0.f, 0.f), qr = ql;
-    if (l & GVIZ_LEAF_BIT) {
-      const uint32_t c = (l & ~GVIZ_LEAF_BIT) - B0;
-      Ml = s.lM[c], SXl = s.lSX[c], SYl = s.lSY[c], cl = s.lCnt[c], Tl = s.lT[c];
-      if (kQ) ql = s.lQ[c];
-    } else {
-      const uint32_t c = l - B0;
-      Ml = s.iM[c], SXl = s.iSX[c], SYl = s.iSY[c], cl = s.iCnt[c], Tl = s.iT[c];
-      if (kQ) ql = s.iQ[c];
-    }
-    if (r & GVIZ_LEAF_BIT) {
-      const uint32_t c = (r & ~GVIZ_LEAF_BIT) - B0;
-      Mr = s.lM[c], SXr = s.lSX[c], SYr = s.lSY[c], cr = s.lCnt[c], Tr = s.lT[c];
-      if (kQ) qr = s.lQ[c];
-    } else {
-      const uint32_t c = r - B0;
-      Mr = s.iM[c], SXr = s.iSX[c], SYr = s.iSY[c], cr = s.iCnt[c], Tr = s.iT[c];
-      if (kQ) qr = s.iQ[c];
-    }
-    float4 q;
-    combine<kQ>(a, p, dp, pp, dpp, l, r, Ml, SXl, SYl, cl, Tl, ql, Mr, SXr, SYr, cr, Tr, qr,
-                M, SX, SY, cnt, T, q);
+    auto child = [&](uint32_t x) {
+      TopSums t;
+      const uint32_t c = (x & ~GVIZ_LEAF_BIT) - B0;
+      t.q = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (x & GVIZ_LEAF_BIT) {
+        t.M = s.lM[c], t.SX = s.lSX[c], t.SY = s.lSY[c], t.cnt = s.lCnt[c], t.T = s.lT[c];
+        if (kQ) t.q = s.lQ[c];
+      } else {
+        t.M = s.iM[c], t.SX = s.iSX[c], t.SY = s.iSY[c], t.cnt = s.iCnt[c], t.T = s.iT[c];
+        if (kQ) t.q = s.iQ[c];
+      }
+      return t;
+    };
+    const Combined z = combined<kQ>(a, is_absorbed(dp, dpp), child(l), child(r));
+    put_combined<kQ>(a, p, l, r, z);
     const uint32_t c = p - B0;  // an in-block parent reads the sums from here
-    s.iM[c] = M;
-    s.iSX[c] = SX;
-    s.iSY[c] = SY;
-    s.iCnt[c] = cnt;
-    s.iT[c] = T;
-    if (kQ) s.iQ[c] = q;
+    s.iM[c] = z.s.M;
+    s.iSX[c] = z.s.SX;
+    s.iSY[c] = z.s.SY;
+    s.iCnt[c] = z.s.cnt;
+    s.iT[c] = T = z.s.T;
+    if (kQ) s.iQ[c] = z.s.q;
     x = p;
     p = pp;
   }
 }
 
-// The nodes spanning blocks, from those whose children k_bottom_up summed:
-// each thread takes one listed node, sums it from its children's sums and
-// climbs on while it arrives second (device-scope counters; the first
-// arrival may have come from k_bottom_up). The climb's critical path is the
-// tree's depth above the blocks (~20 levels at 1M points), so each level
-// issues the next level's shape loads before its arrival and reads only
-// the sibling's sums (the climbing child's are in registers). A persistent
-// grid: the list is short (~3 % of the nodes at 1M points).
+// Sums and preorder positions of the nodes of one level's list, by one block:
+// level 1, block s the list of super-range s; level 2, one block. A listed
+// node's children are listed themselves or were summed by an earlier kernel.
+// The block keeps the list's sums, links and arrivals in shared memory and
+// climbs there: nodes without listed children are combined first, and the
+// second listed child to be combined goes on with its parent. Then every
+// node adds the link weights up to the last ancestor in the list: up to the
+// graph's root that is its preorder position (without the graph base), below
+// a node of level 2 it is relative to that last ancestor, which k_emit adds.
+// A list above kTopCap nodes is worked off by the same block in global memory.
+// Bound by latency: five dependent loads to fill a list, then one chain of
+// shared-memory steps as deep as the tree above the blocks (15 to 26 levels
+// here). One device-scope climb through those levels, a fence, an arrival and
+// a reload of ~3 us each, took 59 us at 65,537 vertices and 71 at 1,048,576,
+// and the positions 7 and 19 more; both kernels together take 23 and 47.
+template <bool kQ, int CAP>
+struct __align__(16) TopShared {
+  double2 s0[CAP];        // M, SX
+  double sy[CAP];
+  uint2 ct[CAP];          // cnt, T
+  uint4 node[CAP];        // children's places, absorbed, parent's place (kTop*)
+  float4 q[kQ ? CAP : 1];
+  uint32_t id[CAP], lc[CAP], rc[CAP];  // node ids: its own, its children's
+  uint32_t w[CAP];            // weight (and dead bit) of the link to the parent
+  uint32_t wl[CAP], wr[CAP];  // and of the links to the children
+  uint32_t arrive[CAP];
+  uint8_t listed[CAP];        // listed children: 0, 1, 2
+};
+constexpr uint32_t kTopRoot = 0xFFFFFFFFu;  // parent: none, the node is a graph's root
+constexpr uint32_t kTopOut = 0xFFFFFFFEu;   // parent: of a higher level
+constexpr uint32_t kTopTwo = 0x80000000u;   // parent's place: both its children are listed
+
 template <bool kQ>
-__global__ __launch_bounds__(kThreads) void k_bottom_up_top(BU a) {
-  const uint32_t nReady = a.counts[4];
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < nReady;
-       i += gridDim.x * kThreads) {
-    uint32_t p = a.ready[i];
-    // p's shape (p is no root sentinel: k_bottom_up checked it)
-    int dp = a.nDelta[p];
-    uint32_t l = a.nLeft[p], r = a.nRight[p], pp = a.upInt[p].x;
-    int dpp = pp == GVIZ_NONE ? 0 : a.nDelta[pp];
-    // the climbing child's sums (none for a listed node: both are read)
-    uint32_t x = GVIZ_NONE, T = 0, cnt = 0;
-    double M = 0.0, SX = 0.0, SY = 0.0;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+__device__ __forceinline__ TopSums summed_child(const BU &a, uint32_t c) {
+  TopSums s;
+  child_vals(a, c, s.M, s.SX, s.SY, s.cnt, s.T);
+  s.q = kQ ? child_q(a, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return s;
+}
+
+__device__ __forceinline__ int level_of(const BU &a, uint32_t p, uint32_t U) {
+  return node_level(p, a.nDelta[p], a.nFirst[p], a.nLast[p], U, a.top.superBits);
+}
+
+// A list too long for shared memory: the same climb and positions over the
+// nodes' global sums, links and counters (block scope: no other block
+// touches these nodes).
+template <bool kQ>
+__device__ void top_in_global(const BU &a, const uint32_t *list, uint32_t n, int level,
+                              uint32_t U) {
+  auto listed = [&](uint32_t c) {
+    return !(c & GVIZ_LEAF_BIT) && level_of(a, c, U) == level;
+  };
+  for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
+    uint32_t p = list[e];
+    if (listed(a.nLeft[p]) || listed(a.nRight[p])) continue;
     for (int guard = 0;; guard++) {
       if (guard > GVIZ_MAX_CLIMB) {
         atomicOr(a.status, GVIZ_ST_TREE);
         break;
       }
-      // the next level's shape, fetched while this level waits
-      const bool nextIn = pp != GVIZ_NONE && dpp >= 32;
-      uint32_t l2 = 0, r2 = 0, ppp = GVIZ_NONE;
-      if (nextIn) {
-        l2 = a.nLeft[pp];
-        r2 = a.nRight[pp];
-        ppp = a.upInt[pp].x;
-      }
-      if (x != GVIZ_NONE) {
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> arrivals(a.nCounter[p]);
-        if (arrivals.fetch_add(1u, cuda::memory_order_acq_rel) == 0u) break;
-        a.nCounter[p] = 0u;
-      }
-      double Ml, SXl, SYl, Mr, SXr, SYr;
-      uint32_t cl, Tl, cr, Tr;
-      float4 ql = make_float4(0.f, 0.f, 0.f, 0.f), qr = ql;
-      if (x == l) {
-        Ml = M, SXl = SX, SYl = SY, cl = cnt, Tl = T, ql = q;
-      } else {
-        child_vals(a, l, Ml, SXl, SYl, cl, Tl);
-        if (kQ) ql = child_q(a, l);
-      }
-      if (x == r) {
-        Mr = M, SXr = SX, SYr = SY, cr = cnt, Tr = T, qr = q;
-      } else {
-        child_vals(a, r, Mr, SXr, SYr, cr, Tr);
-        if (kQ) qr = child_q(a, r);
-      }
-      combine<kQ>(a, p, dp, pp, dpp, l, r, Ml, SXl, SYl, cl, Tl, ql, Mr, SXr, SYr, cr, Tr, qr,
-                  M, SX, SY, cnt, T, q);
-      x = p;
-      if (!nextIn) {  // x is its graph's root
-        const uint32_t g = a.bGid[a.nFirst[x]];
-        a.rootNode[g] = x;
-        a.rootT[g] = T;
-        *up_of(a, x) = make_uint2(GVIZ_NONE, 0u);
+      const uint32_t l = a.nLeft[p], r = a.nRight[p], pp = a.upInt[p].x;
+      const int dpp = pp == GVIZ_NONE ? 0 : a.nDelta[pp];
+      const Combined z = combined<kQ>(a, is_absorbed(a.nDelta[p], dpp), summed_child<kQ>(a, l),
+                                      summed_child<kQ>(a, r));
+      put_combined<kQ>(a, p, l, r, z);
+      if (dpp < 32) {
+        put_root(a, a.bGid[a.nFirst[p]], p, z.s.T);
+        *up_of(a, p) = make_uint2(GVIZ_NONE, 0u);
         break;
       }
+      if (level_of(a, pp, U) != level) break;
+      cuda::atomic_ref<uint32_t, cuda::thread_scope_block> arrivals(a.nCounter[pp]);
+      const uint32_t need = (listed(a.nLeft[pp]) ? 1u : 0u) + (listed(a.nRight[pp]) ? 1u : 0u);
+      if (arrivals.fetch_add(1u, cuda::memory_order_acq_rel) + 1u < need) break;
+      a.nCounter[pp] = 0u;
       p = pp;
-      dp = dpp;
-      l = l2;
-      r = r2;
-      pp = ppp;
-      dpp = pp == GVIZ_NONE ? 0 : a.nDelta[pp];
     }
   }
+  __syncthreads();
+  for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
+    uint32_t x = list[e], pre = 0, dead = 0;
+    uint2 u = a.upInt[x];
+    for (int guard = 0; u.x != GVIZ_NONE && level_of(a, u.x, U) == level; guard++) {
+      if (guard > GVIZ_MAX_CLIMB) {
+        dead = 1;
+        break;
+      }
+      pre += u.y & 0x7fffffffu;
+      dead |= u.y >> 31;
+      x = u.x;
+      u = a.upInt[x];
+    }
+    a.top.pre[list[e]] = make_uint2(dead ? GVIZ_NONE : pre, u.x == GVIZ_NONE ? GVIZ_NONE : x);
+  }
+}
+
+template <bool kQ, int LEVEL, int CAP, int THREADS>
+__global__ __launch_bounds__(THREADS) void k_top(BU a) {
+  extern __shared__ __align__(16) unsigned char topDyn[];
+  TopShared<kQ, CAP> &s = *reinterpret_cast<TopShared<kQ, CAP> *>(topDyn);
+  const uint32_t n = LEVEL == 1 ? a.top.count1[blockIdx.x] : *a.top.count2;
+  const uint32_t *list = LEVEL == 1 ? a.top.list1 + ((size_t)blockIdx.x << a.top.superBits) : a.top.list2;
+  if (n > (uint32_t)CAP) {
+    top_in_global<kQ>(a, list, n, LEVEL, a.counts[2]);
+    return;
+  }
+  auto hold = [&](uint32_t e, const TopSums &c) {
+    s.s0[e] = make_double2(c.M, c.SX);
+    s.sy[e] = c.SY;
+    s.ct[e] = make_uint2(c.cnt, c.T);
+    if (kQ) s.q[e] = c.q;
+  };
+  auto held = [&](uint32_t e) {
+    TopSums c;
+    const double2 m = s.s0[e];
+    const uint2 k = s.ct[e];
+    c.M = m.x;
+    c.SX = m.y;
+    c.SY = s.sy[e];
+    c.cnt = k.x;
+    c.T = k.y;
+    c.q = kQ ? s.q[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    return c;
+  };
+  // every entry's shape, and the sums of the children summed before: of one
+  // such child they are held in the entry's own place until it is combined,
+  // an entry with two is combined right away
+  for (uint32_t e = threadIdx.x; e < n; e += THREADS) {
+    const uint32_t p = list[e];
+    const uint32_t l = a.nLeft[p], r = a.nRight[p], pp = a.upInt[p].x;
+    const int dp = a.nDelta[p], dpp = pp == GVIZ_NONE ? 0 : a.nDelta[pp];
+    const uint2 none = make_uint2(kPreLocal, 0u);
+    const uint2 tl = (l & GVIZ_LEAF_BIT) ? none : a.top.pre[l];
+    const uint2 tr = (r & GVIZ_LEAF_BIT) ? none : a.top.pre[r];
+    const uint2 tp = pp == GVIZ_NONE ? none : a.top.pre[pp];
+    const bool inL = tl.x == kPreListed + LEVEL, inR = tr.x == kPreListed + LEVEL;
+    const bool absorbed = is_absorbed(dp, dpp);
+    const uint32_t par = dpp < 32 ? kTopRoot : (tp.x == kPreListed + LEVEL ? tp.y : kTopOut);
+    s.node[e] = make_uint4(inL ? tl.y : e, inR ? tr.y : e, absorbed ? 1u : 0u, par);
+    s.id[e] = p;
+    s.lc[e] = l;
+    s.rc[e] = r;
+    s.arrive[e] = 0u;
+    s.listed[e] = (inL ? 1 : 0) + (inR ? 1 : 0);
+    if (!inL && !inR) {
+      const Combined z =
+          combined<kQ>(a, absorbed, summed_child<kQ>(a, l), summed_child<kQ>(a, r));
+      hold(e, z.s);
+      s.wl[e] = z.wl;
+      s.wr[e] = z.wr;
+    } else if (!inL || !inR) {
+      hold(e, summed_child<kQ>(a, inL ? r : l));
+    }
+  }
+  __syncthreads();
+  for (uint32_t e = threadIdx.x; e < n; e += THREADS) {  // (places, or kTopOut and above)
+    const uint32_t par = s.node[e].w;
+    if (par < kTopOut && s.listed[par] == 2) s.node[e].w = par | kTopTwo;
+  }
+  __syncthreads();
+  for (uint32_t e0 = threadIdx.x; e0 < n; e0 += THREADS) {
+    if (s.listed[e0]) continue;
+    uint32_t par = s.node[e0].w;
+    for (int guard = 0; par < kTopOut; guard++) {
+      if (guard > GVIZ_MAX_CLIMB) {
+        atomicOr(a.status, GVIZ_ST_TREE);
+        break;
+      }
+      const uint32_t e = par & ~kTopTwo;
+      if (par & kTopTwo) {
+        // release this child's sums, acquire the other's (both in shared memory)
+        __threadfence_block();
+        if (atomicAdd(&s.arrive[e], 1u) == 0u) break;
+        __threadfence_block();
+      }
+      const uint4 nd = s.node[e];
+      const Combined z = combined<kQ>(a, nd.z != 0u, held(nd.x), held(nd.y));
+      hold(e, z.s);
+      s.wl[e] = z.wl;
+      s.wr[e] = z.wr;
+      par = nd.w;
+    }
+  }
+  __syncthreads();
+  // each entry tells its listed children their links' weights
+  for (uint32_t e = threadIdx.x; e < n; e += THREADS) {
+    const uint4 nd = s.node[e];
+    if (nd.x != e) s.w[nd.x] = s.wl[e];
+    if (nd.y != e) s.w[nd.y] = s.wr[e];
+  }
+  __syncthreads();
+  for (uint32_t e = threadIdx.x; e < n; e += THREADS) {
+    const uint32_t p = s.id[e];
+    const uint4 nd = s.node[e];
+    Combined z;
+    z.s = held(e);
+    z.flag = nd.z | (nd.z == 0u && z.s.cnt <= a.k ? 2u : 0u);
+    z.wl = s.wl[e];
+    z.wr = s.wr[e];
+    put_combined<kQ>(a, p, s.lc[e], s.rc[e], z);
+    if (nd.w == kTopRoot) {
+      put_root(a, a.bGid[a.nFirst[p]], p, z.s.T);
+      *up_of(a, p) = make_uint2(GVIZ_NONE, 0u);
+    }
+    uint32_t x = e, par = nd.w, pre = 0, dead = 0;
+    for (int guard = 0; par < kTopOut; guard++) {
+      if (guard > GVIZ_MAX_CLIMB) {
+        dead = 1;
+        break;
+      }
+      pre += s.w[x] & 0x7fffffffu;
+      dead |= s.w[x] >> 31;
+      x = par & ~kTopTwo;
+      par = s.node[x].w;
+    }
+    a.top.pre[p] = make_uint2(dead ? GVIZ_NONE : pre, par == kTopOut ? s.id[x] : GVIZ_NONE);
+  }
+}
+
+constexpr int kTopCap = 2048;  // 156 KB of shared memory, 188 with second moments
+constexpr int kTop1Threads = 512, kTop2Threads = 1024;
+
+template <bool kQ>
+void launch_top(const BU &bu, uint32_t V, cudaStream_t st) {
+  constexpr size_t smem = sizeof(TopShared<kQ, kTopCap>);
+  const uint32_t supers = (uint32_t)top_count_entries(V);
+  k_top<kQ, 1, kTopCap, kTop1Threads><<<supers, kTop1Threads, smem, st>>>(bu);
+  // a layout of one super-range has no nodes above it
+  if (supers > 1) k_top<kQ, 2, kTopCap, kTop2Threads><<<1, kTop2Threads, smem, st>>>(bu);
+}
+
+template <bool kQ>
+void top_smem_limits() {
+  constexpr int smem = (int)sizeof(TopShared<kQ, kTopCap>);
+  cudaFuncSetAttribute(k_top<kQ, 1, kTopCap, kTop1Threads>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_top<kQ, 2, kTopCap, kTop2Threads>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
 // preorder position (without the graph base) and whether any ancestor is a
@@ -873,9 +1109,7 @@ struct EM {
   uint32_t *leafPre;
   uint32_t *cellCnt;  // per record: points below it, 1 for a point (null unless requested)
   uint4 *kids;        // per cell: its children's preorder slots (null unless requested)
-  // per internal node (k_pre_top): its preorder position without the graph
-  // base if it spans blocks of k_bottom_up, else kPreLocal
-  const uint32_t *preTop;
+  const uint2 *pre;  // per internal node: see k_top
 };
 
 __device__ __forceinline__ void put_count(const EM &a, uint32_t at, uint32_t c) {
@@ -1119,41 +1353,29 @@ __device__ void emit_bucket(const EM &a, uint32_t U, uint32_t b, uint32_t pre, u
 }
 
 // A node's preorder position relative to its graph's base is the sum of the
-// link weights up to the graph's root. k_pre_top stores it for every internal
-// node spanning blocks (GVIZ_NONE below a capacity leaf) and kPreLocal for
-// the others, so a walk up stops at the first ancestor spanning blocks.
-constexpr uint32_t kPreLocal = 0xFFFFFFFEu;
+// link weights up to the graph's root; k_top gives it for the nodes above
+// blocks (kPreLocal: not one), so a walk up stops at the first of them.
 
-__device__ __forceinline__ bool spans_blocks(uint32_t p, uint32_t first, uint32_t last,
-                                             uint32_t U) {
-  const uint32_t B0 = p & ~(uint32_t)(kThreads - 1);
-  return first < B0 || last >= min(B0 + kThreads, U);
-}
-
-__global__ __launch_bounds__(kThreads) void k_pre_top(const EM a) {
-  const uint32_t U = a.counts[2];
-  const uint32_t p = blockIdx.x * kThreads + threadIdx.x;
-  if (p + 1 >= U) return;  // internal nodes are [0, U - 1)
-  if (a.nDelta[p] < 32 || !spans_blocks(p, a.nFirst[p], a.nLast[p], U)) {
-    const_cast<uint32_t *>(a.preTop)[p] = kPreLocal;
-    return;
-  }
-  uint32_t pre, dead;
-  walk_up(a.upInt[p], a.upInt, pre, dead);  // its ancestors all span blocks
-  const_cast<uint32_t *>(a.preTop)[p] = dead ? GVIZ_NONE : pre;
-}
-
-// Shared by the threads of one k_emit block: parent links and k_pre_top's
-// entries of the internal nodes [C0, C0 + kEmitSpan).
+// Shared by the threads of one k_emit block: parent links and k_top's entries
+// of the internal nodes [C0, C0 + kEmitSpan).
 constexpr uint32_t kEmitSpan = kThreads / 2;
 struct EmitShared {
-  uint2 up[kEmitSpan];
-  uint32_t pre[kEmitSpan];
+  uint2 up[kEmitSpan], pre[kEmitSpan];
 };
 
+// k_top's position of a node above blocks (t, its entry): below a node of
+// level 2 it is relative to the last ancestor of level 1, t.y.
+__device__ __forceinline__ uint32_t top_pre(const EM &a, uint2 t, bool &dead) {
+  dead = t.x == GVIZ_NONE;
+  if (t.y == GVIZ_NONE) return t.x;
+  const uint2 u = a.upInt[t.y];
+  const uint32_t above = a.pre[u.x].x;
+  dead = dead || (u.y >> 31) || above == GVIZ_NONE;
+  return t.x + u.y + above;
+}
+
 // Preorder position (without the graph base) of the node whose parent link
-// is u: the link weights summed up to the first ancestor spanning blocks,
-// whose own position k_pre_top wrote. dead: an ancestor is a capacity leaf.
+// is u. dead: an ancestor is a capacity leaf.
 __device__ __forceinline__ uint32_t emit_pre(const EM &a, const EmitShared &s, uint32_t C0,
                                              uint2 u, bool &dead) {
   uint32_t pre = 0;
@@ -1166,11 +1388,8 @@ __device__ __forceinline__ uint32_t emit_pre(const EM &a, const EmitShared &s, u
     pre += u.y;
     const uint32_t x = u.x;
     const bool cached = x - C0 < kEmitSpan;
-    const uint32_t t = cached ? s.pre[x - C0] : a.preTop[x];
-    if (t != kPreLocal) {
-      if (t == GVIZ_NONE) dead = true;
-      return pre + t;
-    }
+    const uint2 t = cached ? s.pre[x - C0] : a.pre[x];
+    if (t.x != kPreLocal) return pre + top_pre(a, t, dead);
     u = cached ? s.up[x - C0] : a.upInt[x];
   }
   return pre;
@@ -1188,7 +1407,7 @@ __global__ __launch_bounds__(kThreads) void k_emit(EM a) {
   const uint32_t t = C0 + i;
   if (threadIdx.x < kEmitSpan && t < nInt) {
     s.up[i] = a.upInt[t];
-    s.pre[i] = a.preTop[t];
+    s.pre[i] = a.pre[t];
   }
   __syncthreads();
   // each record's inputs are loaded before the walk up, whose end (the
@@ -1201,11 +1420,8 @@ __global__ __launch_bounds__(kThreads) void k_emit(EM a) {
       const uint32_t g = a.bGid[fb];
       const uint32_t base = a.graphBase[g];
       bool dead;
-      uint32_t pre = s.pre[i];
-      if (pre == kPreLocal)
-        pre = emit_pre(a, s, C0, s.up[i], dead);
-      else
-        dead = pre == GVIZ_NONE;
+      const uint32_t pre = s.pre[i].x == kPreLocal ? emit_pre(a, s, C0, s.up[i], dead)
+                                                   : top_pre(a, s.pre[i], dead);
       if (!dead) emit_internal(a, U, t, pre + base, fb, g, M, SX, SY, T);
     }
   } else if (t < U) {
@@ -1462,7 +1678,7 @@ EM make_em(gvizCudaForce *h) {
   a.nLeft = h->d_nLeft;
   a.nRight = h->d_nRight;
   a.kids = a.f64 ? nullptr : h->d_kids;  // the FP32 walks expand cells by them
-  a.preTop = nullptr;
+  a.pre = h->d_pre;
   return a;
 }
 
@@ -1496,9 +1712,16 @@ void enqueue_tree_build(gvizCudaForce *h) {
       h->d_sHi, h->d_sLo, h->d_ck, h->d_bStart, h->d_bHi, h->d_bLo, h->d_bGid, h->d_upLeaf,
       h->d_scanState, h->d_counts + 2, h->d_status, V, h->gbits);
   prof_mark(h, "tree_buckets");
+  TopLists top;
+  top.list1 = h->d_flag;  // V entries, free after the sort
+  top.list2 = h->d_deepRuns;
+  top.count1 = h->d_topCount;
+  top.count2 = h->d_counts + 4;
+  top.pre = h->d_pre;
+  top.superBits = super_bits(V);
   k_karras<<<blocks_for(V), kThreads, 0, st>>>(
       h->d_bHi, h->d_bLo, h->G > 1 ? h->d_bGid : nullptr, h->d_counts, h->d_nLeft, h->d_nRight,
-      h->d_nFirst, h->d_nLast, h->d_nDelta, h->d_upInt, h->d_upLeaf);
+      h->d_nFirst, h->d_nLast, h->d_nDelta, h->d_upInt, h->d_upLeaf, top);
   BU bu;
   bu.idx = h->d_idx;
   bu.bStart = h->d_bStart;
@@ -1532,22 +1755,18 @@ void enqueue_tree_build(gvizCudaForce *h) {
   bu.k = h->params.nodesPerCell;
   bu.bQ = h->farSide ? h->d_bQ : nullptr;
   bu.nQ = h->farSide ? h->d_nQ : nullptr;
-  // free after the buckets: the list of nodes spanning blocks, and the
-  // preorder positions of k_pre_top
-  bu.ready = h->d_flag;
-  // the nodes spanning blocks are a few percent of the buckets: one wave
-  const uint32_t topBlocks = std::max(1u, std::min<uint32_t>(blocks_for(V), 148u * 4u));
+  bu.top = top;
+  bu.total = h->G == 1 ? h->d_counts + 3 : nullptr;
   if (bu.bQ) {
     k_bottom_up<true><<<blocks_for(V), kThreads, 0, st>>>(bu);
-    k_bottom_up_top<true><<<topBlocks, kThreads, 0, st>>>(bu);
+    launch_top<true>(bu, V, st);
   } else {
     k_bottom_up<false><<<blocks_for(V), kThreads, 0, st>>>(bu);
-    k_bottom_up_top<false><<<topBlocks, kThreads, 0, st>>>(bu);
+    launch_top<false>(bu, V, st);
   }
-  scan_exclusive(h, h->d_rootT, h->d_graphBase, h->G, h->d_counts + 3);
+  // (a single graph starts at slot 0, and its root told the total)
+  if (h->G > 1) scan_exclusive(h, h->d_rootT, h->d_graphBase, h->G, h->d_counts + 3);
   EM em = make_em(h);
-  em.preTop = h->d_scan;
-  k_pre_top<<<blocks_for(V), kThreads, 0, st>>>(em);
   k_emit<<<(uint32_t)((V + kEmitSpan - 1) / kEmitSpan), kThreads, 0, st>>>(em);
   if (em.cellCnt && !em.f64) {
     GroupArgs ga;
@@ -1584,6 +1803,8 @@ void enqueue_group_export(gvizCudaForce *h, uint32_t *groupOf) {
 void tree_set_smem_limits() {
   cudaFuncSetAttribute(k_sort_runs, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        GVIZ_FIX_MAX * 20);
+  top_smem_limits<false>();
+  top_smem_limits<true>();
 }
 
 // Inspection: every cell of the compressed tree (branching nodes and
