@@ -5,8 +5,9 @@
 // exact kernel and the FA2 arithmetic reproduce the reference's rounding.
 //
 //  * k_attr_f64  : src/embedders/gvizForceEmbedder.c:93-100 in CSR order
-//  * k_walk_f64  : bhAccumulateRepulsion (:35-74), warp-shared traversal as in
-//                  forces.cu, terms summed in the reference's DFS order
+//  * k_walk_f64  : bhAccumulateRepulsion (:35-74), a warp steps through the
+//                  union of its targets' nodes, terms summed in the
+//                  reference's DFS order
 //  * k_exact_f64 : the BH-off loop (:104-115), j ascending, j != i
 //  * k_fa2_*     : swing/traction sums, updateGlobalSpeed (:140-185),
 //                  applySpeedRange (:187-197), step tail (:467-492)
@@ -49,36 +50,94 @@ constexpr int kExactTile = 256;
 constexpr uint32_t kInf = 0xffffffffu;
 
 struct Attr64Args {
-  const uint32_t *rowOff, *cols, *gid, *active;
+  const uint32_t *rowOff, *cols, *gid, *active, *list;
   const double2 *pos;
   double2 *out;
   double k;
-  uint32_t V;
+  uint32_t n;  // entries of list
 };
 
+// one attraction term of the vertex at p towards q; false: no term
+template <int MODEL>
+__device__ __forceinline__ bool attr_term64(double2 p, double2 q, double k, double &tx,
+                                            double &ty) {
+  const double dx = q.x - p.x;
+  const double dy = q.y - p.y;
+  const double dist = sqrt(dx * dx + dy * dy);
+  if (dist < 1e-9) return false;
+  double s;
+  if (MODEL == GVIZ_CUDA_MODEL_FR)
+    s = dist / k;
+  else
+    s = log(1.0 + dist) / dist;
+  tx = s * dx;
+  ty = s * dy;
+  return true;
+}
+
+// Vertices with at most GVIZ_HEAVY_DEGREE neighbours: one thread each.
 template <int MODEL>
 __global__ __launch_bounds__(kThreads) void k_attr_f64(Attr64Args a) {
-  const uint32_t v = blockIdx.x * kThreads + threadIdx.x;
-  if (v >= a.V) return;
+  const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= a.n) return;
+  const uint32_t v = a.list[i];
   if (a.active && !a.active[a.gid ? a.gid[v] : 0u]) return;
   const double2 p = a.pos[v];
   double ax = 0.0, ay = 0.0;
   const uint32_t e1 = a.rowOff[v + 1];
   for (uint32_t e = a.rowOff[v]; e < e1; e++) {
-    const double2 q = a.pos[a.cols[e]];
-    const double dx = q.x - p.x;
-    const double dy = q.y - p.y;
-    const double dist = sqrt(dx * dx + dy * dy);
-    if (dist < 1e-9) continue;
-    double s;
-    if (MODEL == GVIZ_CUDA_MODEL_FR)
-      s = dist / a.k;
-    else
-      s = log(1.0 + dist) / dist;
-    ax += s * dx;
-    ay += s * dy;
+    double tx, ty;
+    if (attr_term64<MODEL>(p, a.pos[a.cols[e]], a.k, tx, ty)) {
+      ax += tx;
+      ay += ty;
+    }
   }
   a.out[v] = make_double2(ax, ay);
+}
+
+// The others: one warp each. The lanes compute 32 terms of the row side by
+// side (the gather, square root, logarithm and division of a term take a
+// thousand cycles one after the other) and lanes 0 and 1 add their x and y in
+// row order, so the sums are the serial loop's bit for bit. The next terms'
+// positions are on their way meanwhile. A row of 1,000 entries set the
+// kernel's time: 281 us at 20,000 vertices (LinLog, highest degree ~800),
+// now 36.
+constexpr int kHeavyThreads = 128;
+
+template <int MODEL>
+__global__ __launch_bounds__(kHeavyThreads) void k_attr_f64_heavy(Attr64Args a) {
+  __shared__ double term[kHeavyThreads / 32][2][32];
+  const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t i = blockIdx.x * (kHeavyThreads / 32) + w;
+  if (i >= a.n) return;  // the whole warp
+  const uint32_t v = a.list[i];
+  if (a.active && !a.active[a.gid ? a.gid[v] : 0u]) return;
+  const double2 p = a.pos[v];
+  const uint32_t e0 = a.rowOff[v], e1 = a.rowOff[v + 1];
+  double sum = 0.0;  // lane 0: x, lane 1: y
+  double2 q = p;
+  if (e0 + lane < e1) q = a.pos[a.cols[e0 + lane]];
+  for (uint32_t e = e0; e < e1; e += 32u) {
+    double2 next = p;
+    if (e + 32u + lane < e1) next = a.pos[a.cols[e + 32u + lane]];
+    double tx = 0.0, ty = 0.0;
+    const bool has = e + lane < e1 && attr_term64<MODEL>(p, q, a.k, tx, ty);
+    const uint32_t mask = __ballot_sync(0xffffffffu, has);
+    term[w][0][lane] = tx;
+    term[w][1][lane] = ty;
+    __syncwarp();
+    if (lane < 2u) {
+#pragma unroll 8
+      for (int j = 0; j < 32; j++) {
+        const double t = term[w][lane][j];
+        if ((mask >> j) & 1u) sum += t;
+      }
+    }
+    __syncwarp();
+    q = next;
+  }
+  const double sy = __shfl_sync(0xffffffffu, sum, 1);
+  if (lane == 0u) a.out[v] = make_double2(sum, sy);
 }
 
 // FR / LinLog repulsion term added to (ax, ay) with the reference's
@@ -124,15 +183,29 @@ struct Walk64Args {
   const double *mass, *radius;
   const double2 *attD;
   EpiArgs epi;
-  double kk, overlapC, theta;
+  double kk, overlapC, theta, theta2;
   uint32_t V, maxNodes;
+  uint32_t targets;  // per warp
 };
+
+struct NodeRec {
+  double2 n0, n1;
+  int4 n2;
+};
+
+__device__ __forceinline__ NodeRec load_node(const Walk64Args &a, uint32_t i) {
+  NodeRec r;
+  r.n0 = __ldg(reinterpret_cast<const double2 *>(a.nodes + i));
+  r.n1 = __ldg(reinterpret_cast<const double2 *>(a.nodes + i) + 1);
+  r.n2 = __ldg(reinterpret_cast<const int4 *>(a.nodes + i) + 2);
+  return r;
+}
 
 template <int MODEL>
 __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
   const unsigned lane = threadIdx.x & 31u;
-  const uint32_t s = ((blockIdx.x * kWalkThreads + threadIdx.x) >> 5) * 32u + lane;
-  const bool valid = s < a.V;
+  const uint32_t s = ((blockIdx.x * kWalkThreads + threadIdx.x) >> 5) * a.targets + lane;
+  const bool valid = lane < a.targets && s < a.V;
   const uint32_t v = valid ? a.idx[s] : 0u;
   const uint32_t g = (valid && a.gid) ? a.gid[v] : 0u;
   const bool act = valid && (a.active == nullptr || a.active[g] != 0u);
@@ -150,10 +223,17 @@ __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
   double ax = 0.0, ay = 0.0;
   uint32_t nxt = resume < myEnd ? resume : kInf;
   uint32_t cur = __reduce_min_sync(0xffffffffu, nxt);
+  // The walk is a chain of node records. The one after `cur` is cur + 1 where
+  // a lane opens it, else (every other lane waits at the end of a subtree
+  // around it) the one behind its subtree: both are on their way while this
+  // one is worked on.
+  NodeRec n = cur != kInf ? load_node(a, cur) : NodeRec();
   while (cur != kInf) {
-    const double2 n0 = __ldg(reinterpret_cast<const double2 *>(a.nodes + cur));
-    const double2 n1 = __ldg(reinterpret_cast<const double2 *>(a.nodes + cur) + 1);
-    const int4 n2 = __ldg(reinterpret_cast<const int4 *>(a.nodes + cur) + 2);
+    const NodeRec in = load_node(a, min(cur + 1u, a.maxNodes - 1u));
+    const uint32_t behind = max((uint32_t)n.n2.x, cur + 1u);
+    const NodeRec out = load_node(a, min(behind, a.maxNodes - 1u));
+    const double2 n0 = n.n0, n1 = n.n1;
+    const int4 n2 = n.n2;
     const bool active = cur >= resume && cur < myEnd;
     const bool isLeaf = n2.y >= 0;
     const bool massOk = n1.x != 0.0;
@@ -164,20 +244,31 @@ __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
           rep_term64<MODEL>(vx, vy, n0.x, n0.y, mv, n1.x, rv + n1.y, a.kk,
                             a.overlapC, v, (uint32_t)n2.y, ax, ay);
       } else {
+        // the reference's test, 2h / dist < theta, settled by its squares
+        // wherever those are further apart than any rounding of either
         const double dx = n0.x - vx;
         const double dy = n0.y - vy;
-        const double dist = sqrt(dx * dx + dy * dy);
-        const double ratio = (2.0 * n1.y) / dist;
-        if (ratio < a.theta)
+        const double d2 = dx * dx + dy * dy;
+        const double lhs = 4.0 * n1.y * n1.y, rhs = a.theta2 * d2;
+        bool accept = lhs < rhs * (1.0 - 1e-12);
+        if (!accept && !(lhs > rhs * (1.0 + 1e-12))) accept = (2.0 * n1.y) / sqrt(d2) < a.theta;
+        if (accept)
           rep_term64<MODEL>(vx, vy, n0.x, n0.y, mv, n1.x, rv, a.kk,
                             a.overlapC, v, v, ax, ay);
         else
           open = true;
       }
     }
-    if (active) resume = open ? cur + 1u : max((uint32_t)n2.x, cur + 1u);
+    if (active) resume = open ? cur + 1u : behind;
     nxt = resume < myEnd ? resume : kInf;
+    const uint32_t last = cur;
     cur = __reduce_min_sync(0xffffffffu, nxt);
+    if (cur == last + 1u)
+      n = in;
+    else if (cur == behind)
+      n = out;
+    else if (cur != kInf)  // the next graph's tree
+      n = load_node(a, cur);
   }
   if (!act) return;
   const double2 at = a.attD[v];
@@ -669,6 +760,21 @@ Exact64Args make_exact64(gvizCudaForce *h) {
 
 }  // namespace
 
+template <int MODEL>
+static void launch_attraction_f64(gvizCudaForce *h, Attr64Args a) {
+  const uint32_t *const lists[3] = {h->d_attrLight, h->d_attrHeavy, h->d_hubV};
+  const uint32_t counts[3] = {h->nAttrLight, h->nAttrHeavy, h->nHubs};
+  for (int l = 2; l >= 0; l--) {  // the longest rows first
+    if (!counts[l]) continue;
+    a.list = lists[l];
+    a.n = counts[l];
+    if (l == 0)
+      k_attr_f64<MODEL><<<blocks(a.n, kThreads), kThreads, 0, h->stream>>>(a);
+    else
+      k_attr_f64_heavy<MODEL><<<blocks(a.n, kHeavyThreads / 32), kHeavyThreads, 0, h->stream>>>(a);
+  }
+}
+
 void enqueue_attraction_f64(gvizCudaForce *h) {
   Attr64Args a;
   a.rowOff = h->d_rowOff;
@@ -678,12 +784,23 @@ void enqueue_attraction_f64(gvizCudaForce *h) {
   a.pos = h->d_pos;
   a.out = h->d_attD;
   a.k = h->params.edgeLength;
-  a.V = (uint32_t)h->V;
   if (h->model == GVIZ_CUDA_MODEL_FR)
-    k_attr_f64<GVIZ_CUDA_MODEL_FR><<<blocks(h->V, kThreads), kThreads, 0, h->stream>>>(a);
+    launch_attraction_f64<GVIZ_CUDA_MODEL_FR>(h, a);
   else
-    k_attr_f64<GVIZ_CUDA_MODEL_LINLOG><<<blocks(h->V, kThreads), kThreads, 0, h->stream>>>(a);
+    launch_attraction_f64<GVIZ_CUDA_MODEL_LINLOG>(h, a);
   prof_mark(h, "attraction_f64");
+}
+
+// Targets per warp of the FP64 walk: 32 path-sorted targets share a walk, but
+// below 148 SMs x 20 warps the walk's latency counts, not the work, and
+// fewer targets per warp make more and shorter walks. A target's sum does not
+// depend on it. Walk in us with 32 / 16 / 8 / 4 targets: 700 vertices 129 /
+// 102 / 82 / 70, 9,000 199 / 154 / 128 / 117, 20,000 205 / 168 / 154 / 217,
+// 40,000 221 / 204 / 280 / 371, 80,000 264 / 355 / 465 / 729.
+static uint32_t walk64_targets(size_t V) {
+  uint32_t t = 4;
+  while (t < 32 && V > (size_t)t * 148 * 20) t *= 2;
+  return t;
 }
 
 void enqueue_walk_f64(gvizCudaForce *h) {
@@ -702,9 +819,11 @@ void enqueue_walk_f64(gvizCudaForce *h) {
   a.kk = h->params.edgeLength * h->params.edgeLength;
   a.overlapC = h->params.overlapConstant;
   a.theta = h->params.theta;
+  a.theta2 = a.theta * a.theta;
+  a.targets = walk64_targets(h->V);
   a.V = (uint32_t)h->V;
   a.maxNodes = (uint32_t)h->maxNodes;
-  const uint32_t grid = blocks(((h->V + 31) / 32) * 32, kWalkThreads);
+  const uint32_t grid = blocks(((h->V + a.targets - 1) / a.targets) * 32, kWalkThreads);
   if (h->model == GVIZ_CUDA_MODEL_FR)
     k_walk_f64<GVIZ_CUDA_MODEL_FR><<<grid, kWalkThreads, 0, h->stream>>>(a);
   else
