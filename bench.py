@@ -883,7 +883,7 @@ def grip_bench(args):
         "e2e": {"value": n_e2e / e2e_s, "unit": "rounds/s", "h2d_bytes_per_step": 16 * GRIP_V,
                 "d2h_bytes_per_step": 16 * GRIP_V + 32, "steps": n_e2e,
                 "timer": "host wall clock around synchronous calls"},
-        "gpu_launches": 5 * args.steps, "kernels_per_step": 5,
+        "gpu_launches": 3 * args.steps, "kernels_per_step": 3,
         "roofline": {"kernel": "k_grip_pass1", "bound": "hbm", "achieved": achieved,
                      "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"],

@@ -8,16 +8,18 @@
 // FP64, compiled without fused multiply-add, every expression in the
 // reference's operation order: the per-vertex forces, heat and step are
 // bit-identical to the reference's. The sums over the layer (mean
-// displacement, centroid, angular momentum, inertia, round statistics) run
-// in one block: each thread sums a contiguous chunk in order and thread 0
-// adds the chunk sums in order, so they are deterministic; with
-// strictReductions one thread sums everything in the reference's serial
-// order and the round is bit-identical to the reference's. 2-D only.
+// displacement, centroid, angular momentum, inertia, round statistics) are
+// block partials of fixed shape that the last block of a kernel adds in a
+// fixed order, so they are deterministic; with strictReductions one thread
+// sums everything in the reference's serial order and the round is
+// bit-identical to the reference's. A round is three kernels. 2-D only.
 #include <math.h>
 #include <stdlib.h>
 
 #include <algorithm>
 #include <vector>
+
+#include <cuda/atomic>
 
 #include "gvizcuda.h"
 
@@ -31,9 +33,7 @@ constexpr double kS = 3;             // gvizGRIPs
 constexpr double kFrScale = 0.05;    // FR_SCALE_FACTOR
 constexpr double kEps = 1e-7;        // gvizNumericEpsilon
 constexpr int kThreads = 256;
-constexpr int kSumThreads = 1024;  // room of the partial kernels' staging
-constexpr int kPartThreads = 256;
-constexpr uint32_t kMaxParts = 592;  // 4 blocks per SM
+constexpr uint32_t kMaxParts = 592;  // blocks of the rotation and the move: 4 per SM
 
 struct GripArgs {
   const uint64_t *row;
@@ -43,230 +43,247 @@ struct GripArgs {
   const uint64_t *knnOff;   // list t (of work[t]) has knnOff[t+1] - knnOff[t] entries
   const uint64_t *warpBase; // lists of warp w start at warpBase[w]
   const uint32_t *knnV, *knnD;  // entry e of list 32w + l at warpBase[w] + 32e + l
-  double *part;             // per-block partial sums of the ordered reductions
+  double *part;             // per-block partial sums
   double2 *pos, *disp, *oldDisp;
   double *heat, *oldCos, *lastF, *nrm;
   uint8_t *calc;
   double *red;  // [0,1] mean disp, [2,3] centroid, [4] omega, [5] rotate, [6..9] stats
-  uint32_t n, layer, parts;  // parts: blocks of the partial-sum kernels
+  uint32_t *counter;  // blocks that wrote their partials, zero between kernels
+  uint32_t n, layer;
 };
 
-constexpr int kBatch = 8;
+// A warp takes kGroups vertices, kLanes lanes each: lane r of a group has the
+// entries r, r + kLanes, ... of its vertex's list, kBatch of them in flight,
+// and the group adds each kLanes terms in list order, so the sums are the
+// serial loop's bit for bit.
+constexpr int kLanes = 4;
+constexpr int kGroups = 32 / kLanes;
+constexpr int kBatch = 4;
+constexpr int kForceThreads = 128;
+constexpr int kForceVertices = kForceThreads / kLanes;  // per block
 
 // gvizVecAccKKForce (include/core/gvizVec.h:138-186) at L = dist * 10
-__device__ __forceinline__ void kk_term(double2 p, double2 q, uint32_t dist, double &fx,
-                                        double &fy) {
+__device__ __forceinline__ double2 kk_term(double2 p, double2 q, uint32_t dist) {
   const double L = (double)dist * kEdge;
-  if (L < 1e-9) return;
+  if (L < 1e-9) return make_double2(0.0, 0.0);
   const double dx = q.x - p.x, dy = q.y - p.y;
   const double s = sqrt(dx * dx + dy * dy) / L - 1.0;
-  fx += s * dx;
-  fy += s * dy;
+  return make_double2(s * dx, s * dy);
 }
 
 // gvizVecAccGRIPFRAttForce (include/core/gvizVec.h:115-180), frScale 0.05
-__device__ __forceinline__ void grip_att_term(double2 p, double2 q, double &fx, double &fy) {
+__device__ __forceinline__ double2 grip_att_term(double2 p, double2 q) {
   const double dx = p.x - q.x, dy = p.y - q.y;
   const double d2 = dx * dx + dy * dy;
-  if (d2 < 1e-18) return;
+  if (d2 < 1e-18) return make_double2(0.0, 0.0);
   const double s = kFrScale * (kEdge * kEdge) / d2;
-  fx += s * dx;
-  fy += s * dy;
+  return make_double2(s * dx, s * dy);
+}
+
+// GRIP's FR op along an edge
+__device__ __forceinline__ double2 grip_edge_term(double2 p, double2 q) {
+  const double dx = q.x - p.x, dy = q.y - p.y;
+  const double d2 = dx * dx + dy * dy;
+  if (d2 < 1e-18) return make_double2(0.0, 0.0);
+  const double s = d2 / (kEdge * kEdge);
+  return make_double2(s * dx, s * dy);
+}
+
+// f += the group's kLanes terms in lane order, in every lane of the group. (A
+// term that is left out is +0, which changes no sum: a sum is never -0.)
+__device__ __forceinline__ void add_in_order(double2 t, double &fx, double &fy) {
+#pragma unroll
+  for (int r = 0; r < kLanes; r++) {
+    fx += __shfl_sync(0xffffffffu, t.x, r, kLanes);
+    fy += __shfl_sync(0xffffffffu, t.y, r, kLanes);
+  }
+}
+
+// The fixed-shape sum of v over a block (warp trees, then the warps in order),
+// in thread 0; MAX the maximum.
+template <bool MAX>
+__device__ __forceinline__ double block_reduce(double v, double *sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = MAX ? fmax(v, w) : v + w;
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31u) == 0u) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double r = sh[0];
+  if (threadIdx.x == 0)
+    for (unsigned w = 1; w < blockDim.x / 32; w++) r = MAX ? fmax(r, sh[w]) : r + sh[w];
+  return r;
+}
+
+// Whether this block is the last of the grid to have written its partial sums
+// (visible to it then); leaves the counter at zero. For the whole block.
+__device__ __forceinline__ bool last_block(uint32_t *counter) {
+  __shared__ uint32_t sLast;
+  if (threadIdx.x == 0) {
+    cuda::atomic_ref<uint32_t, cuda::thread_scope_device> done(*counter);
+    sLast = done.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1u;
+    if (sLast) done.store(0u, cuda::memory_order_relaxed);
+  }
+  __syncthreads();
+  return sLast != 0u;
+}
+
+// sum k of the grid's partials (maximum: MAX), in thread 0
+template <bool MAX>
+__device__ __forceinline__ double sum_parts(const double *part, int stride, int k, double *sh) {
+  double v = 0.0;
+  for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+    const double x = __ldcg(part + (size_t)b * stride + k);
+    v = MAX ? fmax(v, x) : v + x;
+  }
+  return block_reduce<MAX>(v, sh);
 }
 
 // Spring forces (calculateSpringForces :892-934; the ops of
 // include/core/gvizVec.h:138-316 via src/embedders/gvizForceDirected.c:6-20),
 // then the heat update (:1071-1103 with updateLocalTemp :870-889) and the
-// heat-scaled step.
-__global__ __launch_bounds__(kThreads) void k_grip_pass1(GripArgs a) {
-  const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= a.n) return;
-  const uint32_t v = a.work[i];
-  const double2 prev = a.disp[v];
-  a.oldDisp[v] = prev;
-  const double2 p = a.pos[v];
+// heat-scaled step; SUMS: also the layer's sums of displacements and
+// positions (removeNetTranslation :1106-1121, the centroid of
+// removeNetRotation :1192-1203), block partials that the last block adds.
+// The gathers of 16 B per list entry bound it, by their latency: with a
+// thread per vertex and 8 gathers in flight (86 registers, 1.3 waves) the
+// kernel took 327 us for 100,000 vertices of 128 entries; four lanes per
+// vertex take 104, the whole round 124 instead of 379.
+template <bool SUMS>
+__global__ __launch_bounds__(kForceThreads) void k_grip_pass1(GripArgs a) {
+  const uint32_t r = threadIdx.x % kLanes;
+  const uint32_t i = blockIdx.x * kForceVertices + threadIdx.x / kLanes;
+  const bool has = i < a.n;
+  const uint32_t v = has ? a.work[i] : 0u;
+  const double2 p = has ? a.pos[v] : make_double2(0.0, 0.0);
   double fx = 0.0, fy = 0.0;
-  // this thread's list, stored warp-interleaved so that the lanes' loads of
-  // entry e are coalesced
-  const uint32_t len = (uint32_t)(a.knnOff[i + 1] - a.knnOff[i]);
-  const uint64_t k0 = a.warpBase[i >> 5] + (i & 31u);
-  const uint64_t k1 = k0 + 32ull * len;
-  // the list is walked in batches of kBatch entries: all their loads are
-  // issued first (the gathers are what bounds this kernel), then the terms
-  // are added in list order, as the reference adds them
+  if (a.layer == 0) {  // along edges
+    const uint64_t j0 = has ? a.row[v] : 0u;
+    const uint32_t len = has ? (uint32_t)(a.row[v + 1] - j0) : 0u;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, len);
+    for (uint32_t e = r; e < most + r; e += kLanes * kBatch) {
+      double2 q[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; b++)
+        q[b] = e + b * kLanes < len ? a.pos[a.col[j0 + e + b * kLanes]] : p;
+#pragma unroll
+      for (int b = 0; b < kBatch; b++) add_in_order(grip_edge_term(p, q[b]), fx, fy);
+    }
+  }
+  // the vertex's list, interleaved with those of the 32 vertices around it:
+  // a warp's lanes read whole sectors
+  const uint32_t len = has ? (uint32_t)(a.knnOff[i + 1] - a.knnOff[i]) : 0u;
+  const uint64_t k0 = has ? a.warpBase[i >> 5] + (i & 31u) : 0u;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, len);
   if (a.layer > 0) {
-    uint64_t e = k0;
-    for (; e + 32ull * (kBatch - 1) < k1; e += 32ull * kBatch) {  // KK springs
+    for (uint32_t e = r; e < most + r; e += kLanes * kBatch) {  // KK springs
       uint32_t dist[kBatch];
       double2 q[kBatch];
 #pragma unroll
-      for (int j = 0; j < kBatch; j++) dist[j] = a.knnD[e + 32ull * j];
+      for (int b = 0; b < kBatch; b++) {
+        const uint32_t at = e + b * kLanes;
+        dist[b] = at < len ? a.knnD[k0 + 32ull * at] : 0u;
+        q[b] = at < len ? a.pos[a.knnV[k0 + 32ull * at]] : p;
+      }
 #pragma unroll
-      for (int j = 0; j < kBatch; j++) q[j] = a.pos[a.knnV[e + 32ull * j]];
-#pragma unroll
-      for (int j = 0; j < kBatch; j++) kk_term(p, q[j], dist[j], fx, fy);
+      for (int b = 0; b < kBatch; b++) add_in_order(kk_term(p, q[b], dist[b]), fx, fy);
     }
-    for (; e < k1; e += 32) kk_term(p, a.pos[a.knnV[e]], a.knnD[e], fx, fy);
   } else {
-    const double lenSq = kEdge * kEdge;
-    for (uint64_t j = a.row[v]; j < a.row[v + 1]; j++) {  // along edges
-      const double2 q = a.pos[a.col[j]];
-      const double dx = q.x - p.x, dy = q.y - p.y;
-      const double d2 = dx * dx + dy * dy;
-      if (d2 < 1e-18) continue;
-      const double s = d2 / lenSq;
-      fx += s * dx;
-      fy += s * dy;
-    }
-    uint64_t e = k0;
-    for (; e + 32ull * (kBatch - 1) < k1; e += 32ull * kBatch) {  // from the k nearest
+    for (uint32_t e = r; e < most + r; e += kLanes * kBatch) {  // from the k nearest
       double2 q[kBatch];
 #pragma unroll
-      for (int j = 0; j < kBatch; j++) q[j] = a.pos[a.knnV[e + 32ull * j]];
+      for (int b = 0; b < kBatch; b++) {
+        const uint32_t at = e + b * kLanes;
+        q[b] = at < len ? a.pos[a.knnV[k0 + 32ull * at]] : p;
+      }
 #pragma unroll
-      for (int j = 0; j < kBatch; j++) grip_att_term(p, q[j], fx, fy);
+      for (int b = 0; b < kBatch; b++) add_in_order(grip_att_term(p, q[b]), fx, fy);
     }
-    for (; e < k1; e += 32) grip_att_term(p, a.pos[a.knnV[e]], fx, fy);
   }
-  double heat = a.heat[v], oc = a.oldCos[v];
-  if (!a.calc[v]) {
-    a.calc[v] = 1;
-    heat = kEdge / 6.0;
-  } else {
+  const bool owner = has && r == 0u;
+  if (owner) {
+    const double2 prev = a.disp[v];
+    a.oldDisp[v] = prev;
+    double heat = a.heat[v], oc = a.oldCos[v];
     const double nrm = sqrt(fx * fx + fy * fy);
-    const double oldNrm = sqrt(prev.x * prev.x + prev.y * prev.y);
-    if (!(fabs(nrm) < kEps || fabs(oldNrm) < kEps)) {
-      const double c = (fx * prev.x + fy * prev.y) / (nrm * oldNrm);
-      if (c > 0 && oc > 0)
-        heat *= (1 + c * kR * kS);
-      else
-        heat *= (1 + c * kR);
-      oc = c;
+    if (!a.calc[v]) {
+      a.calc[v] = 1;
+      heat = kEdge / 6.0;
+    } else {
+      const double oldNrm = sqrt(prev.x * prev.x + prev.y * prev.y);
+      if (!(fabs(nrm) < kEps || fabs(oldNrm) < kEps)) {
+        const double c = (fx * prev.x + fy * prev.y) / (nrm * oldNrm);
+        if (c > 0 && oc > 0)
+          heat *= (1 + c * kR * kS);
+        else
+          heat *= (1 + c * kR);
+        oc = c;
+      }
     }
+    heat = fmin(heat, kEdge * 10);
+    heat = fmax(heat, kEdge * 1e-4);
+    a.lastF[v] = nrm;
+    if (nrm > kEps) {
+      const double s = heat / nrm;
+      fx *= s;
+      fy *= s;
+    }
+    a.disp[v] = make_double2(fx, fy);
+    a.heat[v] = heat;
+    a.oldCos[v] = oc;
   }
-  heat = fmin(heat, kEdge * 10);
-  heat = fmax(heat, kEdge * 1e-4);
-  const double nrm = sqrt(fx * fx + fy * fy);
-  a.lastF[v] = nrm;
-  if (nrm > kEps) {
-    const double s = heat / nrm;
-    fx *= s;
-    fy *= s;
-  }
-  a.disp[v] = make_double2(fx, fy);
-  a.heat[v] = heat;
-  a.oldCos[v] = oc;
-}
-
-// Ordered sums over the layer in two launches. Partial: block b takes the
-// contiguous range of items [b*B, (b+1)*B); each thread sums a contiguous
-// chunk of it in order and thread 0 adds the chunk sums in order. Final:
-// one thread adds the block partials in order. Deterministic; with one block
-// of one thread (strict reductions) the whole sum runs in the reference's
-// serial order.
-template <int K>
-__device__ __forceinline__ void block_partial(double (&acc)[K], double *out,
-                                              double (*tmp)[K]) {
-  for (int k = 0; k < K; k++) tmp[threadIdx.x][k] = acc[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < K; k++) acc[k] = tmp[0][k];
-    for (unsigned t = 1; t < blockDim.x; t++)
-      for (int k = 0; k < K; k++) acc[k] += tmp[t][k];
-    for (int k = 0; k < K; k++) out[blockIdx.x * K + k] = acc[k];
+  if (!SUMS) return;
+  __shared__ double sh[kForceThreads / 32];
+  double sum[4] = {owner ? fx : 0.0, owner ? fy : 0.0, owner ? p.x : 0.0, owner ? p.y : 0.0};
+#pragma unroll
+  for (int k = 0; k < 4; k++) sum[k] = block_reduce<false>(sum[k], sh);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 4; k++) a.part[(size_t)blockIdx.x * 4 + k] = sum[k];
+  if (!last_block(a.counter)) return;
+  for (int k = 0; k < 4; k++) {
+    const double t = sum_parts<false>(a.part, 4, k, sh);
+    if (threadIdx.x == 0) a.red[k] = k < 2 ? t * (1.0 / (double)a.n) : t / (double)a.n;
   }
 }
 
-__device__ __forceinline__ void item_range(uint32_t n, uint32_t &b, uint32_t &e) {
-  const uint32_t per = (n + gridDim.x - 1) / gridDim.x;
-  const uint32_t lo = blockIdx.x * per, hi = min(lo + per, n);
-  const uint32_t c = (per + blockDim.x - 1) / blockDim.x;
-  b = min(lo + threadIdx.x * c, hi);
-  e = min(b + c, hi);
-}
-
-// sums of the displacements and the positions (removeNetTranslation
-// :1106-1121, the centroid of removeNetRotation :1192-1203)
-__global__ __launch_bounds__(kSumThreads) void k_grip_part1(GripArgs a) {
-  __shared__ double tmp[kSumThreads][4];
-  uint32_t b, e;
-  item_range(a.n, b, e);
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (uint32_t i = b; i < e; i++) {
-    const uint32_t v = a.active[i];
-    const double2 d = a.disp[v], p = a.pos[v];
-    acc[0] += 1.0 * d.x;
-    acc[1] += 1.0 * d.y;
-    acc[2] += p.x;
-    acc[3] += p.y;
-  }
-  block_partial<4>(acc, a.part, tmp);
-}
-
-// the block partials, loaded by the whole block into shared memory so that
-// one thread can add them in order without waiting on each load
-__device__ __forceinline__ const double *stage_parts(const GripArgs &a, double *sp) {
-  for (uint32_t j = threadIdx.x; j < a.parts * 4; j += blockDim.x) sp[j] = a.part[j];
-  __syncthreads();
-  return sp;
-}
-
-__global__ __launch_bounds__(kPartThreads) void k_grip_final1(GripArgs a) {
-  __shared__ double sp[kMaxParts * 4];
-  const double *part = stage_parts(a, sp);
-  if (threadIdx.x) return;
-  double acc[4];
-  for (int k = 0; k < 4; k++) acc[k] = part[k];
-  for (uint32_t b = 1; b < a.parts; b++)
-    for (int k = 0; k < 4; k++) acc[k] += part[b * 4 + k];
-  const double inv = 1.0 / (double)a.n;
-  a.red[0] = acc[0] * inv;
-  a.red[1] = acc[1] * inv;
-  a.red[2] = acc[2] / (double)a.n;
-  a.red[3] = acc[3] / (double)a.n;
-}
-
-// angular momentum of the translated displacements and the polar moment of
-// inertia about the centroid; omega = L / I (:1204-1252, dim 2)
-__global__ __launch_bounds__(kSumThreads) void k_grip_part2(GripArgs a) {
-  __shared__ double tmp[kSumThreads][2];
-  uint32_t b, e;
-  item_range(a.n, b, e);
+// Angular momentum of the translated displacements and the polar moment of
+// inertia about the centroid; omega = L / I (:1204-1252, dim 2), by the last
+// block.
+__global__ __launch_bounds__(kThreads) void k_grip_rotation(GripArgs a) {
+  __shared__ double sh[kThreads / 32];
   const double mx = a.red[0], my = a.red[1], cx = a.red[2], cy = a.red[3];
-  double acc[2] = {0.0, 0.0};
-  for (uint32_t i = b; i < e; i++) {
-    const uint32_t v = a.active[i];
+  double L = 0.0, I = 0.0;
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < a.n; i += gridDim.x * kThreads) {
+    const uint32_t v = a.work[i];
     const double2 p = a.pos[v];
     double2 d = a.disp[v];
     d.x += -1.0 * mx;
     d.y += -1.0 * my;
     const double rx = p.x - cx, ry = p.y - cy;
-    acc[0] += rx * d.y - ry * d.x;
-    acc[1] += rx * rx + ry * ry;
+    L += rx * d.y - ry * d.x;
+    I += rx * rx + ry * ry;
   }
-  block_partial<2>(acc, a.part, tmp);
-}
-
-__global__ __launch_bounds__(kPartThreads) void k_grip_final2(GripArgs a) {
-  __shared__ double sp[kMaxParts * 4];
-  const double *part = stage_parts(a, sp);
-  if (threadIdx.x) return;
-  double L = part[0], I = part[1];
-  for (uint32_t b = 1; b < a.parts; b++) {
-    L += part[b * 2];
-    I += part[b * 2 + 1];
+  L = block_reduce<false>(L, sh);
+  I = block_reduce<false>(I, sh);
+  if (threadIdx.x == 0) {
+    a.part[(size_t)blockIdx.x * 2] = L;
+    a.part[(size_t)blockIdx.x * 2 + 1] = I;
   }
+  if (!last_block(a.counter)) return;
+  L = sum_parts<false>(a.part, 2, 0, sh);
+  I = sum_parts<false>(a.part, 2, 1, sh);
+  if (threadIdx.x != 0) return;
   const bool rotate = a.n >= 3 && !(fabs(I) < kEps);
   a.red[4] = rotate ? L / I : 0.0;
   a.red[5] = rotate ? 1.0 : 0.0;
 }
 
-// remove the translation and the rotation, move (gvizEmbeddedGraphAdd-
-// VPosition, src/embedders/gvizEmbeddedGraph.c:400-404)
-__global__ __launch_bounds__(kThreads) void k_grip_apply(GripArgs a) {
-  const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-  if (i >= a.n) return;
-  const uint32_t v = a.active[i];
+// Removes the translation and the rotation of vertex v and moves it
+// (gvizEmbeddedGraphAddVPosition, src/embedders/gvizEmbeddedGraph.c:400-404);
+// returns the displacement's length.
+__device__ __forceinline__ double grip_move(const GripArgs &a, uint32_t v) {
   const double2 p = a.pos[v];
   double2 d = a.disp[v];
   d.x += -1.0 * a.red[0];
@@ -278,17 +295,83 @@ __global__ __launch_bounds__(kThreads) void k_grip_apply(GripArgs a) {
     d.y -= w * rx - 0.0 * 0.0;
   }
   a.disp[v] = d;
-  a.nrm[i] = sqrt(d.x * d.x + d.y * d.y);
   a.pos[v] = make_double2(p.x + 1.0 * d.x, p.y + 1.0 * d.y);
+  return sqrt(d.x * d.x + d.y * d.y);
 }
 
-// round statistics (:1302-1331): max and sums of |disp|, heat, force
-__global__ __launch_bounds__(kSumThreads) void k_grip_part3(GripArgs a) {
-  __shared__ double tmp[kSumThreads][4];
-  uint32_t b, e;
-  item_range(a.n, b, e);
+// The move, and the round's statistics (:1302-1331): maximum and sums of
+// |disp|, heat and force, by the last block.
+__global__ __launch_bounds__(kThreads) void k_grip_move(GripArgs a) {
+  __shared__ double sh[kThreads / 32];
+  double mx = 0.0, sum[3] = {0.0, 0.0, 0.0};
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < a.n; i += gridDim.x * kThreads) {
+    const uint32_t v = a.work[i];
+    const double nrm = grip_move(a, v);
+    mx = fmax(mx, nrm);
+    sum[0] += nrm;
+    sum[1] += a.heat[v];
+    sum[2] += a.lastF[v];
+  }
+  mx = block_reduce<true>(mx, sh);
+  for (int k = 0; k < 3; k++) sum[k] = block_reduce<false>(sum[k], sh);
+  if (threadIdx.x == 0) {
+    a.part[(size_t)blockIdx.x * 4] = mx;
+    for (int k = 0; k < 3; k++) a.part[(size_t)blockIdx.x * 4 + 1 + k] = sum[k];
+  }
+  if (!last_block(a.counter)) return;
+  mx = sum_parts<true>(a.part, 4, 0, sh);
+  if (threadIdx.x == 0) a.red[6] = mx;
+  for (int k = 0; k < 3; k++) {
+    const double t = sum_parts<false>(a.part, 4, 1 + k, sh);
+    if (threadIdx.x == 0) a.red[7 + k] = t / a.n;
+  }
+}
+
+// The layer's sums in the reference's serial order (strict reductions), by
+// one thread over the filtration order.
+__global__ void k_grip_serial1(GripArgs a) {
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (uint32_t i = 0; i < a.n; i++) {
+    const uint32_t v = a.active[i];
+    const double2 d = a.disp[v], p = a.pos[v];
+    acc[0] += 1.0 * d.x;
+    acc[1] += 1.0 * d.y;
+    acc[2] += p.x;
+    acc[3] += p.y;
+  }
+  const double inv = 1.0 / (double)a.n;
+  a.red[0] = acc[0] * inv;
+  a.red[1] = acc[1] * inv;
+  a.red[2] = acc[2] / (double)a.n;
+  a.red[3] = acc[3] / (double)a.n;
+}
+
+__global__ void k_grip_serial2(GripArgs a) {
+  const double mx = a.red[0], my = a.red[1], cx = a.red[2], cy = a.red[3];
+  double L = 0.0, I = 0.0;
+  for (uint32_t i = 0; i < a.n; i++) {
+    const uint32_t v = a.active[i];
+    const double2 p = a.pos[v];
+    double2 d = a.disp[v];
+    d.x += -1.0 * mx;
+    d.y += -1.0 * my;
+    const double rx = p.x - cx, ry = p.y - cy;
+    L += rx * d.y - ry * d.x;
+    I += rx * rx + ry * ry;
+  }
+  const bool rotate = a.n >= 3 && !(fabs(I) < kEps);
+  a.red[4] = rotate ? L / I : 0.0;
+  a.red[5] = rotate ? 1.0 : 0.0;
+}
+
+__global__ __launch_bounds__(kThreads) void k_grip_apply(GripArgs a) {
+  const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+  if (i < a.n) a.nrm[i] = grip_move(a, a.active[i]);
+}
+
+__global__ void k_grip_serial3(GripArgs a) {
   double acc[4] = {0.0, 0.0, 0.0, 0.0};  // max, sum disp, sum heat, sum force
-  for (uint32_t i = b; i < e; i++) {
+  for (uint32_t i = 0; i < a.n; i++) {
     const uint32_t v = a.active[i];
     const double nrm = a.nrm[i];
     if (nrm > acc[0]) acc[0] = nrm;
@@ -296,29 +379,23 @@ __global__ __launch_bounds__(kSumThreads) void k_grip_part3(GripArgs a) {
     acc[2] += a.heat[v];
     acc[3] += a.lastF[v];
   }
-  tmp[threadIdx.x][0] = acc[0];
-  __syncthreads();
-  double mx = acc[0];
-  if (threadIdx.x == 0)
-    for (unsigned t = 1; t < blockDim.x; t++) mx = fmax(mx, tmp[t][0]);
-  __syncthreads();
-  block_partial<4>(acc, a.part, tmp);
-  if (threadIdx.x == 0) a.part[blockIdx.x * 4] = mx;
+  a.red[6] = acc[0];
+  for (int k = 1; k < 4; k++) a.red[6 + k] = acc[k] / a.n;
 }
 
-__global__ __launch_bounds__(kPartThreads) void k_grip_final3(GripArgs a) {
-  __shared__ double sp[kMaxParts * 4];
-  const double *part = stage_parts(a, sp);
-  if (threadIdx.x) return;
-  double mx = part[0], acc[3] = {part[1], part[2], part[3]};
-  for (uint32_t b = 1; b < a.parts; b++) {
-    mx = fmax(mx, part[b * 4]);
-    for (int k = 0; k < 3; k++) acc[k] += part[b * 4 + 1 + k];
-  }
-  a.red[6] = mx;
-  a.red[7] = a.n ? acc[0] / a.n : 0.0;
-  a.red[8] = a.n ? acc[1] / a.n : 0.0;
-  a.red[9] = a.n ? acc[2] / a.n : 0.0;
+// positions between the caller's vertex order and the handle's labels (label
+// n is the caller's vertex perm[n])
+__global__ __launch_bounds__(kThreads) void k_grip_take(const double2 *__restrict__ xy,
+                                                        const uint32_t *__restrict__ perm,
+                                                        double2 *pos, uint32_t V) {
+  const uint32_t n = blockIdx.x * kThreads + threadIdx.x;
+  if (n < V) pos[n] = xy[perm[n]];
+}
+__global__ __launch_bounds__(kThreads) void k_grip_give(const double2 *__restrict__ pos,
+                                                        const uint32_t *__restrict__ perm,
+                                                        double2 *xy, uint32_t V) {
+  const uint32_t n = blockIdx.x * kThreads + threadIdx.x;
+  if (n < V) xy[perm[n]] = pos[n];
 }
 
 // clearDecorators (:936-951) for the vertices of the new layer
@@ -349,7 +426,10 @@ struct gvizCudaGrip {
   uint8_t *d_calc = nullptr;
   uint32_t *d_active = nullptr, *d_knnV = nullptr, *d_knnD = nullptr;
   uint64_t *d_knnOff = nullptr, *d_warpBase = nullptr;
-  double *d_part = nullptr;  // kMaxParts x 4 partial sums
+  double *d_part = nullptr;  // partial sums, four per block
+  uint32_t *d_counter = nullptr;
+  uint32_t *d_perm = nullptr;  // perm below
+  double2 *d_xy = nullptr;     // positions in the caller's order, on their way
   uint32_t *d_work = nullptr;
   size_t n = 0, knnCap = 0, layer = 0;
   bool hasLayer = false;
@@ -400,8 +480,7 @@ GripArgs grip_args(gvizCudaGrip *h) {
   a.red = h->d_red;
   a.n = (uint32_t)h->n;
   a.layer = (uint32_t)h->layer;
-  const uint32_t want = (uint32_t)((h->n + 1023) / 1024);
-  a.parts = h->strict ? 1u : (want < 1 ? 1u : (want > kMaxParts ? kMaxParts : want));
+  a.counter = h->d_counter;
   return a;
 }
 
@@ -421,6 +500,9 @@ void grip_free(gvizCudaGrip *h) {
   cudaFree(h->d_knnOff);
   cudaFree(h->d_warpBase);
   cudaFree(h->d_part);
+  cudaFree(h->d_counter);
+  cudaFree(h->d_perm);
+  cudaFree(h->d_xy);
   cudaFree(h->d_work);
   cudaFree(h->d_knnV);
   cudaFree(h->d_knnD);
@@ -465,7 +547,11 @@ int gvizCudaGripCreate(gvizCudaGrip **out, size_t vertexCount, const uint64_t *r
   if (!rc) rc |= galloc(&h->d_active, V);
   if (!rc) rc |= galloc(&h->d_knnOff, V + 1);
   if (!rc) rc |= galloc(&h->d_warpBase, V / 32 + 2);
-  if (!rc) rc |= galloc(&h->d_part, (size_t)kMaxParts * 4);
+  if (!rc)
+    rc |= galloc(&h->d_part, std::max<size_t>(kMaxParts, V / kForceVertices + 1) * 4);
+  if (!rc) rc |= galloc(&h->d_counter, 1);
+  if (!rc) rc |= galloc(&h->d_perm, V);
+  if (!rc) rc |= galloc(&h->d_xy, V);
   if (!rc) rc |= galloc(&h->d_work, V);
   if (rc) {
     grip_free(h);
@@ -518,7 +604,9 @@ int gvizCudaGripCreate(gvizCudaGrip **out, size_t vertexCount, const uint64_t *r
     cudaMemsetAsync(h->d_oldCos, 0, V * 8, h->stream);
     cudaMemsetAsync(h->d_lastF, 0, V * 8, h->stream);
     cudaMemsetAsync(h->d_calc, 0, V, h->stream);
+    cudaMemcpyAsync(h->d_perm, h->perm.data(), V * 4, cudaMemcpyHostToDevice, h->stream);
   }
+  cudaMemsetAsync(h->d_counter, 0, 4, h->stream);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
     grip_free(h);
     cudaStreamDestroy(h->stream);
@@ -548,15 +636,11 @@ int gvizCudaGripSetPositions(gvizCudaGrip *h, const double *xy) {
   if (!h || (h->V && !xy)) return GVIZ_CUDA_ERR_ARG;
   GripGuard guard(h->device);
   if (!h->V) return GVIZ_CUDA_OK;
-  std::vector<double> tmp(2 * h->V);
-  for (size_t n = 0; n < h->V; n++) {
-    tmp[2 * n] = xy[2 * (size_t)h->perm[n]];
-    tmp[2 * n + 1] = xy[2 * (size_t)h->perm[n] + 1];
-  }
-  if (cudaMemcpyAsync(h->d_pos, tmp.data(), h->V * 16, cudaMemcpyHostToDevice, h->stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(h->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(h->d_xy, xy, h->V * 16, cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
     return GVIZ_CUDA_ERR_CUDA;
+  k_grip_take<<<grid_for(h->V), kThreads, 0, h->stream>>>(h->d_xy, h->d_perm, h->d_pos,
+                                                           (uint32_t)h->V);
+  if (cudaStreamSynchronize(h->stream) != cudaSuccess) return GVIZ_CUDA_ERR_CUDA;
   return GVIZ_CUDA_OK;
 }
 
@@ -564,15 +648,11 @@ int gvizCudaGripGetPositions(gvizCudaGrip *h, double *xy) {
   if (!h || (h->V && !xy)) return GVIZ_CUDA_ERR_ARG;
   GripGuard guard(h->device);
   if (!h->V) return GVIZ_CUDA_OK;
-  std::vector<double> tmp(2 * h->V);
-  if (cudaMemcpyAsync(tmp.data(), h->d_pos, h->V * 16, cudaMemcpyDeviceToHost, h->stream) !=
-          cudaSuccess ||
+  k_grip_give<<<grid_for(h->V), kThreads, 0, h->stream>>>(h->d_pos, h->d_perm, h->d_xy,
+                                                           (uint32_t)h->V);
+  if (cudaMemcpyAsync(xy, h->d_xy, h->V * 16, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
       cudaStreamSynchronize(h->stream) != cudaSuccess)
     return GVIZ_CUDA_ERR_CUDA;
-  for (size_t n = 0; n < h->V; n++) {
-    xy[2 * (size_t)h->perm[n]] = tmp[2 * n];
-    xy[2 * (size_t)h->perm[n] + 1] = tmp[2 * n + 1];
-  }
   return GVIZ_CUDA_OK;
 }
 
@@ -653,16 +733,26 @@ int gvizCudaGripSetLayer(gvizCudaGrip *h, size_t layer, const uint32_t *active,
   return GVIZ_CUDA_OK;
 }
 
+static void grip_forces(gvizCudaGrip *h, const GripArgs &a) {
+  const uint32_t grid = (uint32_t)((h->n + kForceVertices - 1) / kForceVertices);
+  if (h->strict)
+    k_grip_pass1<false><<<grid, kForceThreads, 0, h->stream>>>(a);
+  else
+    k_grip_pass1<true><<<grid, kForceThreads, 0, h->stream>>>(a);
+}
+
 // everything of a round after the force kernel
-void grip_after_forces(gvizCudaGrip *h, const GripArgs &a) {
-  const uint32_t th = h->strict ? 1u : (uint32_t)kPartThreads;
-  k_grip_part1<<<a.parts, th, 0, h->stream>>>(a);
-  k_grip_final1<<<1, kPartThreads, 0, h->stream>>>(a);
-  k_grip_part2<<<a.parts, th, 0, h->stream>>>(a);
-  k_grip_final2<<<1, kPartThreads, 0, h->stream>>>(a);
-  k_grip_apply<<<grid_for(h->n), kThreads, 0, h->stream>>>(a);
-  k_grip_part3<<<a.parts, th, 0, h->stream>>>(a);
-  k_grip_final3<<<1, kPartThreads, 0, h->stream>>>(a);
+static void grip_after_forces(gvizCudaGrip *h, const GripArgs &a) {
+  if (h->strict) {
+    k_grip_serial1<<<1, 1, 0, h->stream>>>(a);
+    k_grip_serial2<<<1, 1, 0, h->stream>>>(a);
+    k_grip_apply<<<grid_for(h->n), kThreads, 0, h->stream>>>(a);
+    k_grip_serial3<<<1, 1, 0, h->stream>>>(a);
+    return;
+  }
+  const uint32_t grid = std::min(grid_for(h->n), kMaxParts);
+  k_grip_rotation<<<grid, kThreads, 0, h->stream>>>(a);
+  k_grip_move<<<grid, kThreads, 0, h->stream>>>(a);
 }
 
 int gvizCudaGripRefineRound(gvizCudaGrip *h, gvizCudaGripRoundStats *stats) {
@@ -672,7 +762,7 @@ int gvizCudaGripRefineRound(gvizCudaGrip *h, gvizCudaGripRoundStats *stats) {
   double red[16] = {0};
   if (h->n) {
     const GripArgs a = grip_args(h);
-    k_grip_pass1<<<grid_for(h->n), kThreads, 0, h->stream>>>(a);
+    grip_forces(h, a);
     grip_after_forces(h, a);
     if (cudaGetLastError() != cudaSuccess) return GVIZ_CUDA_ERR_CUDA;
     if (cudaMemcpyAsync(red, h->d_red, sizeof red, cudaMemcpyDeviceToHost, h->stream) !=
@@ -705,7 +795,7 @@ int gvizCudaGripTimeRounds(gvizCudaGrip *h, uint32_t rounds, float *totalMs, flo
     cudaEventRecord(ev[0], h->stream);
     for (uint32_t r = 0; r < rounds; r++) {
       cudaEventRecord(ev[2 + 2 * r], h->stream);
-      k_grip_pass1<<<grid_for(h->n), kThreads, 0, h->stream>>>(a);
+      grip_forces(h, a);
       cudaEventRecord(ev[3 + 2 * r], h->stream);
       grip_after_forces(h, a);
     }
