@@ -265,6 +265,102 @@ __global__ __launch_bounds__(THREADS) void k_radix_onesweep(
   }
 }
 
+// The whole sort of n <= THREADS * ROUNDS keys by one block: the pairs stay in
+// shared memory through all passes, so there are no launches, counts or
+// look-backs between them.
+template <int THREADS, int ROUNDS>
+struct SmallSortSmem {
+  uint64_t k[THREADS * ROUNDS];
+  uint32_t v[THREADS * ROUNDS];
+  uint32_t wcnt[THREADS / 32][256];
+  uint32_t start[256];
+};
+
+template <int THREADS, int ROUNDS>
+__global__ __launch_bounds__(THREADS) void k_radix_small(uint64_t *keys, uint32_t *vals,
+                                                         uint32_t n) {
+  constexpr int kWarps = THREADS / 32;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  SmallSortSmem<THREADS, ROUNDS> &s = *reinterpret_cast<SmallSortSmem<THREADS, ROUNDS> *>(dyn);
+  const unsigned tid = threadIdx.x, w = tid >> 5, lane = tid & 31u;
+  const uint32_t at = w * (ROUNDS * 32) + lane;
+  uint64_t k[ROUNDS];
+  uint32_t v[ROUNDS], rank[ROUNDS];
+#pragma unroll
+  for (int r = 0; r < ROUNDS; r++) {
+    const uint32_t i = at + r * 32;
+    k[r] = i < n ? keys[i] : 0ull;
+    v[r] = i < n ? vals[i] : 0u;
+  }
+  for (int pass = 0; pass < kSortPasses; pass++) {
+    const int shift = GVIZ_SORT_SKIP_BITS + 8 * pass;
+    for (unsigned d = tid; d < kWarps * 256; d += THREADS) (&s.wcnt[0][0])[d] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+      const bool valid = at + r * 32 < n;
+      const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
+      const uint32_t peers = digit_peers(d, valid);
+      const uint32_t lt = peers & ((1u << lane) - 1u);
+      const uint32_t before = valid ? s.wcnt[w][d] : 0u;
+      rank[r] = before + __popc(lt);
+      __syncwarp();
+      if (valid && lt == 0) s.wcnt[w][d] = before + __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t run = 0;
+    if (tid < 256) {
+#pragma unroll
+      for (int ww = 0; ww < kWarps; ww++) {
+        const uint32_t t = s.wcnt[ww][tid];
+        s.wcnt[ww][tid] = run;
+        run += t;
+      }
+    }
+    uint32_t first;
+    block_exclusive_scan<THREADS>(run, first);
+    if (tid < 256) s.start[tid] = first;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+      if (at + r * 32 >= n) continue;
+      const uint32_t d = (uint32_t)(k[r] >> shift) & 255u;
+      const uint32_t to = s.start[d] + s.wcnt[w][d] + rank[r];
+      s.k[to] = k[r];
+      s.v[to] = v[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+      const uint32_t i = at + r * 32;
+      k[r] = i < n ? s.k[i] : 0ull;
+      v[r] = i < n ? s.v[i] : 0u;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROUNDS; r++) {
+    const uint32_t i = at + r * 32;
+    if (i < n) {
+      keys[i] = k[r];
+      vals[i] = v[r];
+    }
+  }
+}
+
+template <int THREADS, int ROUNDS>
+void small_sort_limit() {
+  cudaFuncSetAttribute(k_radix_small<THREADS, ROUNDS>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(SmallSortSmem<THREADS, ROUNDS>));
+}
+
+template <int THREADS, int ROUNDS>
+void small_sort(gvizCudaForce *h, uint64_t *keys, uint32_t *vals, size_t n) {
+  k_radix_small<THREADS, ROUNDS><<<1, THREADS, sizeof(SmallSortSmem<THREADS, ROUNDS>), h->stream>>>(
+      keys, vals, (uint32_t)n);
+}
+
 }  // namespace
 
 size_t scan_state_entries(size_t n) {
@@ -283,6 +379,10 @@ struct SortShape {
 // (196), 65,537 311 / 316 / 323 (358), 262,144 639 / 636 / 635 (669), 0.75M
 // in 512 graphs 974 / 972 / 951 (983), 1,048,576 1583 / 1570 / 1534 (1575).
 constexpr size_t kSmallSort = 1u << 17;
+// k_radix_small up to here: whole step in us, one block / six launches: 300
+// vertices 72 / 84, 1,024 82 / 96, 2,000 94 / 106, 3,000 104 / 107, 4,000 110
+// / 111; eight rounds for 8,192 keys would take 143 / 125.
+constexpr size_t kBlockSort = 4096;
 
 static SortShape sort_shape(size_t n) {
   if (n <= kSmallSort) return {kSortThreads, 2};
@@ -330,6 +430,9 @@ void scan_exclusive(gvizCudaForce *h, const uint32_t *in, uint32_t *out,
 // The scatter's shared memory exceeds the default per-block budget: opted
 // into once per device, at handle creation (outside any stream capture).
 void sort_set_smem_limits() {
+  small_sort_limit<512, 2>();
+  small_sort_limit<1024, 2>();
+  small_sort_limit<1024, 4>();
   cudaFuncSetAttribute(k_radix_onesweep<kSortThreads, 8>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)scatter_dyn(kSortThreads * 8));
@@ -338,6 +441,13 @@ void sort_set_smem_limits() {
 void radix_sort_pairs(gvizCudaForce *h, uint64_t *keys, uint32_t *vals,
                       uint64_t *keysAlt, uint32_t *valsAlt, size_t n) {
   if (n <= 1) return;
+  if (n <= kBlockSort) {
+    if (n <= 1024) small_sort<512, 2>(h, keys, vals, n);
+    else if (n <= 2048) small_sort<1024, 2>(h, keys, vals, n);
+    else small_sort<1024, 4>(h, keys, vals, n);
+    prof_mark(h, "radix_sort");
+    return;
+  }
   const SortShape shape = sort_shape(n);
   const uint32_t tiles = (uint32_t)sort_tiles(n);
   uint32_t *ghist = sort_digit_counts(h);

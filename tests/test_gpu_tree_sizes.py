@@ -9,7 +9,7 @@ from test_gpu_tree import point_layout
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 257, 1023, 1024, 1025, 2047, 2048, 2049, 4097, 131072, 131073])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 257, 1023, 1024, 1025, 2047, 2048, 2049, 4096, 4097, 131072, 131073])
 @pytest.mark.parametrize("k", [1, 3])
 def test_membership_at_tile_edges(oracle, n, k):
     rng = np.random.default_rng(n)
