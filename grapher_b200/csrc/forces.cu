@@ -651,6 +651,7 @@ __device__ __forceinline__ void walk_task(const WalkArgs &a, uint32_t task, cons
 // Static schedule: warp w of the grid takes task w.
 template <int MODEL, bool OVERLAP, bool COUNT>
 __global__ __launch_bounds__(kWalkMaxThreads, 2) void k_walk_f32(WalkArgs a) {
+  step_order();
   extern __shared__ __align__(16) unsigned char plainDyn[];
   const PlainWarpSmem q = plain_warp_smem(plainDyn, a.stackCap);
   const uint32_t task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -663,6 +664,7 @@ __global__ __launch_bounds__(kWalkMaxThreads, 2) void k_walk_f32(WalkArgs a) {
 // the queue is empty, so warps that drew cheap tasks take more of them.
 template <int MODEL, bool OVERLAP, bool COUNT>
 __global__ __launch_bounds__(kWalkMaxThreads, 2) void k_walk_f32_queue(WalkArgs a) {
+  step_order();
   extern __shared__ __align__(16) unsigned char plainDyn[];
   const PlainWarpSmem q = plain_warp_smem(plainDyn, a.stackCap);
   for (;;) {
@@ -762,6 +764,7 @@ __device__ __forceinline__ void group_centroid(bool act, double2 p, float vxh, f
 
 template <int MODEL, bool OVERLAP, bool COUNT>
 __global__ __launch_bounds__(kFarThreads, 5) void k_walk_f32_far(FarArgs fa) {
+  step_order();
   __shared__ MlpSmem W;
   __shared__ FarWarpSmem Q[kFarThreads / 32];
   mlp_stage(W, fa.mlp);
@@ -1234,6 +1237,7 @@ __device__ __forceinline__ int cell_classify(const CellGroup &g, uint32_t cur, f
 
 template <int MODEL, bool OVERLAP, bool COUNT>
 __global__ __launch_bounds__(kCellThreads, kCellBlocksPerSM) void k_walk_f32_cells(CellArgs ca) {
+  step_order();
   __shared__ MlpSmem W;
   extern __shared__ __align__(16) unsigned char cellDyn[];
   CellWarpSmem *Q = reinterpret_cast<CellWarpSmem *>(cellDyn);  // one per warp
@@ -1533,6 +1537,7 @@ __device__ __forceinline__ void hub_walk_range(const FarHubArgs &a, const HubTar
 
 template <int MODEL, bool OVERLAP>
 __global__ __launch_bounds__(kHubThreads) void k_walk_f32_hubs(FarHubArgs a) {
+  step_order();
   __shared__ uint2 ring[kHubThreads / 32][kHubRing];
   const uint32_t lane = threadIdx.x & 31u;
   uint2 *q = ring[threadIdx.x >> 5];
@@ -1616,6 +1621,7 @@ __global__ __launch_bounds__(kHubThreads) void k_walk_f32_hubs(FarHubArgs a) {
 // The hubs' force epilogues with their plain repulsion, after the learned
 // walk wrote theirs.
 __global__ __launch_bounds__(256) void k_far_hub_epilogue(FarHubArgs a) {
+  step_order();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nHubs) return;
   const uint32_t v = a.hubs[i];
@@ -1657,6 +1663,7 @@ struct ExactArgs {
 // range order.
 template <int MODEL, bool OVERLAP>
 __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
+  step_order();
   // a source's coordinates twice each, as the packed pairs of two targets
   // take them: {x, x, y, y} high parts, then low parts
   __shared__ ulonglong2 sph[kExactTile], spl[kExactTile];
@@ -1861,6 +1868,7 @@ __global__ __launch_bounds__(kExactThreads) void k_exact_f32(ExactArgs a) {
 
 // The split sums of each target added in range order, then its epilogue.
 __global__ __launch_bounds__(256) void k_exact_combine(ExactArgs a) {
+  step_order();
   const uint32_t v = blockIdx.x * 256 + threadIdx.x;
   if (v >= a.V) return;
   const uint32_t g = a.gid ? a.gid[v] : 0u;
@@ -2225,6 +2233,6 @@ void enqueue_exact_f32(gvizCudaForce *h) {
     if (ov) k_exact_f32<GVIZ_CUDA_MODEL_LINLOG, true><<<grid, kExactThreads, 0, h->stream>>>(a);
     else k_exact_f32<GVIZ_CUDA_MODEL_LINLOG, false><<<grid, kExactThreads, 0, h->stream>>>(a);
   }
-  if (a.splits > 1) k_exact_combine<<<blocks(h->V, 256), 256, 0, h->stream>>>(a);
+  if (a.splits > 1) launch_after(h->stream, k_exact_combine, blocks(h->V, 256), 256, 0, a);
   prof_mark(h, "exact_f32");
 }

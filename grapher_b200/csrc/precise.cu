@@ -203,6 +203,7 @@ __device__ __forceinline__ NodeRec load_node(const Walk64Args &a, uint32_t i) {
 
 template <int MODEL>
 __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
+  step_order();
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t s = ((blockIdx.x * kWalkThreads + threadIdx.x) >> 5) * a.targets + lane;
   const bool valid = lane < a.targets && s < a.V;
@@ -289,6 +290,7 @@ struct Exact64Args {
 
 template <int MODEL>
 __global__ __launch_bounds__(kThreads) void k_exact_f64(Exact64Args a) {
+  step_order();
   __shared__ double2 sp[kExactTile];
   __shared__ double2 smr[kExactTile];
   __shared__ uint32_t sRange[2];
@@ -573,6 +575,7 @@ __device__ void fa2_speed(const Fa2Args &a, uint32_t g, double *sh) {
 // time with); every sum keeps its fixed order: strided per-thread partials,
 // the block's tree, the chunks in order.
 __global__ __launch_bounds__(kThreads) void k_fa2_speed(Fa2Args a) {
+  step_order();
   __shared__ double sh[kThreads / 32];
   const uint32_t c = blockIdx.x;
   const uint32_t g = a.chunkGraph[c];
@@ -645,6 +648,7 @@ __device__ void fa2_stats(const Fa2Args &a, uint32_t g, double *sh) {
 // applySpeedRange (:187-197), position update and the statistics' chunk sums
 // (:467-477); the last chunk of a graph to finish adds those up.
 __global__ __launch_bounds__(kThreads) void k_fa2_apply(Fa2Args a) {
+  step_order();
   __shared__ double sh[kThreads / 32];
   const uint32_t c = blockIdx.x;
   const uint32_t g = a.chunkGraph[c];
@@ -696,10 +700,12 @@ __global__ __launch_bounds__(kThreads) void k_fa2_apply(Fa2Args a) {
 
 // Strict reductions: one block per graph, thread 0 sums the vertices in order.
 __global__ __launch_bounds__(kThreads) void k_fa2_speed_strict(Fa2Args a) {
+  step_order();
   __shared__ double sh[kThreads / 32];
   if (a.active[blockIdx.x]) fa2_speed(a, blockIdx.x, sh);
 }
 __global__ __launch_bounds__(kThreads) void k_fa2_stats_strict(Fa2Args a) {
+  step_order();
   __shared__ double sh[kThreads / 32];
   if (a.active[blockIdx.x]) fa2_stats(a, blockIdx.x, sh);
 }
@@ -874,12 +880,12 @@ void enqueue_fa2(gvizCudaForce *h) {
   Fa2Args a = make_fa2(h);
   const uint32_t G = (uint32_t)h->G;
   if (a.strict) {
-    k_fa2_speed_strict<<<G, kThreads, 0, h->stream>>>(a);
-    k_fa2_apply<<<h->nChunks, kThreads, 0, h->stream>>>(a);
-    k_fa2_stats_strict<<<G, kThreads, 0, h->stream>>>(a);
+    launch_after(h->stream, k_fa2_speed_strict, G, kThreads, 0, a);
+    launch_after(h->stream, k_fa2_apply, h->nChunks, kThreads, 0, a);
+    launch_after(h->stream, k_fa2_stats_strict, G, kThreads, 0, a);
   } else {
-    k_fa2_speed<<<h->nChunks, kThreads, 0, h->stream>>>(a);
-    k_fa2_apply<<<h->nChunks, kThreads, 0, h->stream>>>(a);
+    launch_after(h->stream, k_fa2_speed, h->nChunks, kThreads, 0, a);
+    launch_after(h->stream, k_fa2_apply, h->nChunks, kThreads, 0, a);
   }
   prof_mark(h, "fa2_update");
 }

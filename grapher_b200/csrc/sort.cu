@@ -87,6 +87,7 @@ __device__ __forceinline__ uint32_t lookback_digit(const uint32_t *st, uint32_t 
 __global__ __launch_bounds__(kScanThreads) void k_scan_onepass(
     const uint32_t *in, uint32_t *out, uint32_t n, uint64_t *state, uint32_t *total,
     uint32_t *status) {
+  step_order();
   __shared__ uint32_t sTile;
   if (threadIdx.x == 0) sTile = scan_ticket(state);
   __syncthreads();
@@ -117,6 +118,7 @@ constexpr uint32_t kSingleMax = 1u << 13;  // one SM: only for small arrays
 
 __global__ __launch_bounds__(kTopThreads) void k_scan_single(
     const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total) {
+  step_order();
   const uint32_t per = (n + kTopThreads - 1) / kTopThreads;
   const uint32_t b = threadIdx.x * per;
   uint32_t s = 0;
@@ -168,6 +170,7 @@ __global__ __launch_bounds__(THREADS) void k_radix_onesweep(
     uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, uint32_t n,
     int pass, uint32_t *ghist, uint32_t *state, uint32_t *ticket,
     uint32_t *status) {
+  step_order();
   constexpr int kWarps = THREADS / 32;
   constexpr uint32_t kTile = THREADS * ROUNDS;
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -279,6 +282,7 @@ struct SmallSortSmem {
 template <int THREADS, int ROUNDS>
 __global__ __launch_bounds__(THREADS) void k_radix_small(uint64_t *keys, uint32_t *vals,
                                                          uint32_t n) {
+  step_order();
   constexpr int kWarps = THREADS / 32;
   extern __shared__ __align__(16) unsigned char dyn[];
   SmallSortSmem<THREADS, ROUNDS> &s = *reinterpret_cast<SmallSortSmem<THREADS, ROUNDS> *>(dyn);
@@ -357,8 +361,8 @@ void small_sort_limit() {
 
 template <int THREADS, int ROUNDS>
 void small_sort(gvizCudaForce *h, uint64_t *keys, uint32_t *vals, size_t n) {
-  k_radix_small<THREADS, ROUNDS><<<1, THREADS, sizeof(SmallSortSmem<THREADS, ROUNDS>), h->stream>>>(
-      keys, vals, (uint32_t)n);
+  launch_after(h->stream, k_radix_small<THREADS, ROUNDS>, 1, THREADS,
+               sizeof(SmallSortSmem<THREADS, ROUNDS>), keys, vals, (uint32_t)n);
 }
 
 }  // namespace
@@ -414,7 +418,7 @@ void scan_exclusive(gvizCudaForce *h, const uint32_t *in, uint32_t *out,
     return;
   }
   if (n <= kSingleMax) {
-    k_scan_single<<<1, kTopThreads, 0, h->stream>>>(in, out, (uint32_t)n, total);
+    launch_after(h->stream, k_scan_single, 1, kTopThreads, 0, in, out, (uint32_t)n, total);
     return;
   }
   const uint32_t tiles = (uint32_t)((n + kScanTile - 1) / kScanTile);
@@ -458,9 +462,9 @@ void radix_sort_pairs(gvizCudaForce *h, uint64_t *keys, uint32_t *vals,
   for (int pass = 0; pass < kSortPasses; pass++) {
     const auto kernel =
         shape.rounds == 2 ? k_radix_onesweep<kSortThreads, 2> : k_radix_onesweep<kSortThreads, 8>;
-    kernel<<<tiles, shape.threads, scatter_dyn(shape.tile()), h->stream>>>(
-        ka, va, kb, vb, (uint32_t)n, pass, ghist, state + (size_t)pass * 256 * tiles,
-        tickets + pass, h->d_status);
+    launch_after(h->stream, kernel, tiles, shape.threads, scatter_dyn(shape.tile()), ka, va, kb,
+                 vb, (uint32_t)n, pass, ghist, state + (size_t)pass * 256 * tiles,
+                 tickets + pass, h->d_status);
     std::swap(ka, kb);
     std::swap(va, vb);
   }

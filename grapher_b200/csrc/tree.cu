@@ -69,6 +69,7 @@ __global__ __launch_bounds__(kThreads) void k_bbox_chunks(
     const double2 *__restrict__ pos, const uint32_t *__restrict__ cb,
     const uint32_t *__restrict__ ce, const uint32_t *__restrict__ cg, unsigned long long *box,
     uint32_t *status) {
+  step_order();
   const uint32_t b = cb[blockIdx.x], e = ce[blockIdx.x];
   double mnx = INFINITY, mxx = -INFINITY, mny = INFINITY, mxy = -INFINITY;
   int bad = 0;
@@ -189,6 +190,7 @@ __global__ __launch_bounds__(kThreads) void k_keys(
     const double2 *__restrict__ pos, const uint32_t *__restrict__ gid,
     const unsigned long long *__restrict__ box, GraphRoot *roots, uint64_t *ck, uint32_t *idx,
     uint32_t *digits, uint32_t *status, uint32_t V, int gbits) {
+  step_order();
   __shared__ uint32_t cnt[256];
   static_assert(kThreads == 256, "one thread per digit");
   cnt[threadIdx.x] = 0u;
@@ -228,6 +230,7 @@ __global__ __launch_bounds__(kThreads) void k_runs(
     const uint64_t *__restrict__ ck, const uint32_t *__restrict__ idx,
     const double2 *__restrict__ pos, const GraphRoot *__restrict__ roots, uint32_t *counts,
     uint32_t *deep, uint64_t *sHi, uint64_t *sLo, uint32_t V, uint32_t k, int gbits) {
+  step_order();
   const uint32_t s = blockIdx.x * kThreads + threadIdx.x;
   if (s >= V) return;
   const uint64_t full = ck[s];
@@ -280,6 +283,7 @@ __device__ __forceinline__ bool key_less(uint64_t ah, uint64_t al, uint32_t av,
 __global__ __launch_bounds__(512) void k_sort_runs(
     uint64_t *sHi, uint64_t *sLo, uint32_t *idx, const uint32_t *__restrict__ deep,
     const uint32_t *__restrict__ counts, uint32_t *status) {
+  step_order();
   extern __shared__ unsigned char smem[];
   uint64_t *kh = reinterpret_cast<uint64_t *>(smem);
   uint64_t *kl = kh + GVIZ_FIX_MAX;
@@ -354,6 +358,7 @@ __global__ __launch_bounds__(kThreads) void k_buckets(
     const uint64_t *__restrict__ ck, uint32_t *bStart, uint64_t *bHi, uint64_t *bLo,
     uint32_t *bGid, uint2 *upLeaf, uint64_t *state, uint32_t *total, uint32_t *status, uint32_t V,
     int gbits) {
+  step_order();
   constexpr int kRounds = GVIZ_SCAN_TILE / kThreads;
   __shared__ uint32_t sTile;
   if (threadIdx.x == 0) sTile = scan_ticket(state);
@@ -386,8 +391,8 @@ __global__ __launch_bounds__(kThreads) void k_buckets(
     starts[r] = __ballot_sync(0xffffffffu, start);
     count += __popc(starts[r]);
   }
-  uint32_t b = scan_tile_prefix<kThreads>(state, tile, count, (V + GVIZ_SCAN_TILE - 1u) / GVIZ_SCAN_TILE,
-                                          total, status);
+  const uint32_t nTiles = (V + GVIZ_SCAN_TILE - 1u) / GVIZ_SCAN_TILE;
+  uint32_t b = scan_tile_prefix<kThreads>(state, tile, count, nTiles, total, status);
 #pragma unroll
   for (int r = 0; r < kRounds; r++) {
     if ((starts[r] >> lane) & 1u) {
@@ -520,6 +525,7 @@ __global__ __launch_bounds__(kThreads) void k_karras(
     const uint32_t *__restrict__ bGid, const uint32_t *__restrict__ counts,
     uint32_t *nLeft, uint32_t *nRight, uint32_t *nFirst, uint32_t *nLast,
     int32_t *nDelta, uint2 *upInt, uint2 *upLeaf, TopLists top) {
+  step_order();
   __shared__ uint64_t sHi[kKarrasTile], sLo[kKarrasTile];
   __shared__ uint32_t sCount[2], sBase[2];
   const int U = (int)counts[2];
@@ -549,7 +555,8 @@ __global__ __launch_bounds__(kThreads) void k_karras(
   __syncthreads();
   if (level > 0) {
     at += sBase[level - 1];
-    (level == 1 ? top.list1 + ((B0 >> top.superBits) << top.superBits) : top.list2)[at] = (uint32_t)i;
+    uint32_t *const list1 = top.list1 + ((B0 >> top.superBits) << top.superBits);
+    (level == 1 ? list1 : top.list2)[at] = (uint32_t)i;
     top.pre[i] = make_uint2(kPreListed + (uint32_t)level, at);
   } else if (i < U - 1) {
     top.pre[i] = make_uint2(kPreLocal, 0u);
@@ -717,6 +724,7 @@ struct BUShared {
 // sums also go to global memory (k_emit reads them).
 template <bool kQ>
 __global__ __launch_bounds__(kThreads) void k_bottom_up(BU a) {
+  step_order();
   __shared__ BUShared<kQ> s;
   const uint32_t U = a.counts[2];
   const uint32_t B0 = blockIdx.x * kThreads;
@@ -930,10 +938,12 @@ __device__ void top_in_global(const BU &a, const uint32_t *list, uint32_t n, int
 
 template <bool kQ, int LEVEL, int CAP, int THREADS>
 __global__ __launch_bounds__(THREADS) void k_top(BU a) {
+  step_order();
   extern __shared__ __align__(16) unsigned char topDyn[];
   TopShared<kQ, CAP> &s = *reinterpret_cast<TopShared<kQ, CAP> *>(topDyn);
   const uint32_t n = LEVEL == 1 ? a.top.count1[blockIdx.x] : *a.top.count2;
-  const uint32_t *list = LEVEL == 1 ? a.top.list1 + ((size_t)blockIdx.x << a.top.superBits) : a.top.list2;
+  const uint32_t *list =
+      LEVEL == 1 ? a.top.list1 + ((size_t)blockIdx.x << a.top.superBits) : a.top.list2;
   if (n > (uint32_t)CAP) {
     top_in_global<kQ>(a, list, n, LEVEL, a.counts[2]);
     return;
@@ -1058,9 +1068,10 @@ template <bool kQ>
 void launch_top(const BU &bu, uint32_t V, cudaStream_t st) {
   constexpr size_t smem = sizeof(TopShared<kQ, kTopCap>);
   const uint32_t supers = (uint32_t)top_count_entries(V);
-  k_top<kQ, 1, kTopCap, kTop1Threads><<<supers, kTop1Threads, smem, st>>>(bu);
+  launch_after(st, k_top<kQ, 1, kTopCap, kTop1Threads>, supers, kTop1Threads, smem, bu);
   // a layout of one super-range has no nodes above it
-  if (supers > 1) k_top<kQ, 2, kTopCap, kTop2Threads><<<1, kTop2Threads, smem, st>>>(bu);
+  if (supers > 1)
+    launch_after(st, k_top<kQ, 2, kTopCap, kTop2Threads>, 1, kTop2Threads, smem, bu);
 }
 
 template <bool kQ>
@@ -1398,6 +1409,7 @@ __device__ __forceinline__ uint32_t emit_pre(const EM &a, const EmitShared &s, u
 // Node and leaf records in preorder: block j emits internal nodes and
 // buckets [C0, C0 + kEmitSpan), C0 = kEmitSpan j, one per thread.
 __global__ __launch_bounds__(kThreads) void k_emit(EM a) {
+  step_order();
   __shared__ EmitShared s;
   const uint32_t U = a.counts[2];
   const uint32_t nInt = U - 1;
@@ -1487,6 +1499,7 @@ __device__ __forceinline__ uint32_t child_quadrant(const NodeF *nodes, uint32_t 
 // root, or the runs of a leaf bucket); one atomic per warp reserves the
 // warp's slots.
 __global__ __launch_bounds__(kThreads) void k_far_groups(GroupArgs a) {
+  step_order();
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t total = min(a.counts[3], a.maxNodes);
@@ -1696,21 +1709,20 @@ void enqueue_tree_build(gvizCudaForce *h) {
   cudaMemsetAsync(h->d_zero, 0, h->zeroBytes, st);
   k_bbox_chunks<<<h->nChunks, kThreads, 0, st>>>(h->d_pos, h->d_chunkBegin, h->d_chunkEnd,
                                                   h->d_chunkGraph, h->d_box, h->d_status);
-  k_keys<<<std::min(blocks_for(V), 148u * 8u), kThreads, 0, st>>>(h->d_pos, h->d_gid, h->d_box, h->d_roots, h->d_ck,
-                                             h->d_idx, sort_digit_counts(h), h->d_status, V,
-                                             h->gbits);
+  launch_after(st, k_keys, std::min(blocks_for(V), 148u * 8u), kThreads, 0, h->d_pos, h->d_gid,
+               h->d_box, h->d_roots, h->d_ck, h->d_idx, sort_digit_counts(h), h->d_status, V,
+               h->gbits);
   prof_mark(h, "tree_keys");
   radix_sort_pairs(h, h->d_ck, h->d_idx, h->d_ckAlt, h->d_idxAlt, V);
-  k_runs<<<blocks_for(V), kThreads, 0, st>>>(h->d_ck, h->d_idx, h->d_pos, h->d_roots, h->d_counts,
-                                             h->d_deepRuns, h->d_sHi, h->d_sLo, V,
-                                             h->params.nodesPerCell, h->gbits);
+  launch_after(st, k_runs, blocks_for(V), kThreads, 0, h->d_ck, h->d_idx, h->d_pos, h->d_roots,
+               h->d_counts, h->d_deepRuns, h->d_sHi, h->d_sLo, V, h->params.nodesPerCell,
+               h->gbits);
   const size_t fixSmem = (size_t)GVIZ_FIX_MAX * 20;
-  k_sort_runs<<<148, 512, fixSmem, st>>>(h->d_sHi, h->d_sLo, h->d_idx,
-                                          h->d_deepRuns, h->d_counts,
-                                          h->d_status);
-  k_buckets<<<(V + GVIZ_SCAN_TILE - 1) / GVIZ_SCAN_TILE, kThreads, 0, st>>>(
-      h->d_sHi, h->d_sLo, h->d_ck, h->d_bStart, h->d_bHi, h->d_bLo, h->d_bGid, h->d_upLeaf,
-      h->d_scanState, h->d_counts + 2, h->d_status, V, h->gbits);
+  launch_after(st, k_sort_runs, 148, 512, fixSmem, h->d_sHi, h->d_sLo, h->d_idx, h->d_deepRuns,
+               h->d_counts, h->d_status);
+  launch_after(st, k_buckets, (V + GVIZ_SCAN_TILE - 1) / GVIZ_SCAN_TILE, kThreads, 0, h->d_sHi,
+               h->d_sLo, h->d_ck, h->d_bStart, h->d_bHi, h->d_bLo, h->d_bGid, h->d_upLeaf,
+               h->d_scanState, h->d_counts + 2, h->d_status, V, h->gbits);
   prof_mark(h, "tree_buckets");
   TopLists top;
   top.list1 = h->d_flag;  // V entries, free after the sort
@@ -1719,9 +1731,9 @@ void enqueue_tree_build(gvizCudaForce *h) {
   top.count2 = h->d_counts + 4;
   top.pre = h->d_pre;
   top.superBits = super_bits(V);
-  k_karras<<<blocks_for(V), kThreads, 0, st>>>(
-      h->d_bHi, h->d_bLo, h->G > 1 ? h->d_bGid : nullptr, h->d_counts, h->d_nLeft, h->d_nRight,
-      h->d_nFirst, h->d_nLast, h->d_nDelta, h->d_upInt, h->d_upLeaf, top);
+  launch_after(st, k_karras, blocks_for(V), kThreads, 0, h->d_bHi, h->d_bLo,
+               h->G > 1 ? h->d_bGid : nullptr, h->d_counts, h->d_nLeft, h->d_nRight, h->d_nFirst,
+               h->d_nLast, h->d_nDelta, h->d_upInt, h->d_upLeaf, top);
   BU bu;
   bu.idx = h->d_idx;
   bu.bStart = h->d_bStart;
@@ -1758,16 +1770,16 @@ void enqueue_tree_build(gvizCudaForce *h) {
   bu.top = top;
   bu.total = h->G == 1 ? h->d_counts + 3 : nullptr;
   if (bu.bQ) {
-    k_bottom_up<true><<<blocks_for(V), kThreads, 0, st>>>(bu);
+    launch_after(st, k_bottom_up<true>, blocks_for(V), kThreads, 0, bu);
     launch_top<true>(bu, V, st);
   } else {
-    k_bottom_up<false><<<blocks_for(V), kThreads, 0, st>>>(bu);
+    launch_after(st, k_bottom_up<false>, blocks_for(V), kThreads, 0, bu);
     launch_top<false>(bu, V, st);
   }
   // (a single graph starts at slot 0, and its root told the total)
   if (h->G > 1) scan_exclusive(h, h->d_rootT, h->d_graphBase, h->G, h->d_counts + 3);
   EM em = make_em(h);
-  k_emit<<<(uint32_t)((V + kEmitSpan - 1) / kEmitSpan), kThreads, 0, st>>>(em);
+  launch_after(st, k_emit, (uint32_t)((V + kEmitSpan - 1) / kEmitSpan), kThreads, 0, em);
   if (em.cellCnt && !em.f64) {
     GroupArgs ga;
     ga.nodes = reinterpret_cast<const NodeF *>(h->d_nodes);
