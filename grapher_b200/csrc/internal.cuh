@@ -251,11 +251,17 @@ struct gvizCudaForce {
 // ended and its writes are visible. Launched by launch_after a kernel's
 // start-up overlaps its predecessor's end, which takes 5 us off a step (1,024
 // vertices 94.4 -> 89.7, 65,537 195 -> 190, 1,048,576 1214 -> 1209); launched
-// any other way this is a no-op. No kernel lets its successor start earlier:
-// blocks that wait for the whole predecessor then hold the room that the
+// any other way this is a no-op. No kernel of a layout's step lets its
+// successor start earlier: blocks that wait for the whole predecessor then hold the room that the
 // attraction on the side stream needs (65,537 vertices: 223 us).
 __device__ __forceinline__ void step_order() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Lets the next kernel start up to its own step_order. After step_order, and
+// where the kernel and its successor leave most of the chip idle (training).
+__device__ __forceinline__ void step_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }

@@ -24,6 +24,9 @@
 // FP32 master layout (padded like MlpDev): w1t[64][16], b1[64], w2t[64][64],
 // b2[64], w3t[8][64], b3[8]
 #define MLP_PAD (MLP_HID * MLP_INP + MLP_HID + MLP_HID * MLP_HID + MLP_HID + MLP_OUTP * MLP_HID + MLP_OUTP)
+// floats between two blocks' partial gradients: the parameters, the loss, and
+// room that keeps every row 16-byte aligned
+#define MLP_ROW (MLP_PAD + 4)
 #define OFF_W1 0
 #define OFF_B1 (OFF_W1 + MLP_HID * MLP_INP)
 #define OFF_W2 (OFF_B1 + MLP_HID)
@@ -37,7 +40,7 @@ struct gvizCudaMlp {
   float *d_w = nullptr;      // FP32 masters (MLP_PAD)
   float *d_m = nullptr, *d_v = nullptr;  // Adam moments
   MlpDev *d_dev = nullptr;   // BF16 copy used by the kernels
-  float *d_grad = nullptr;   // per-block partials [blocks][MLP_PAD + 1]
+  float *d_grad = nullptr;   // per-block partials [blocks][MLP_ROW]
   float *d_gsum = nullptr;   // reduced gradient + loss
   size_t gradBlocks = 0;
   uint64_t step = 0;
@@ -321,7 +324,7 @@ __global__ __launch_bounds__(32) void k_mlp_grad(const float *__restrict__ w,
     }
     __syncwarp();
   }
-  float *out = partial + (size_t)blockIdx.x * (MLP_PAD + 1);
+  float *out = partial + (size_t)blockIdx.x * MLP_ROW;
   for (int i = l; i < MLP_PAD; i += 32) out[i] = S.g[i];
   if (l == 0) out[MLP_PAD] = S.loss;
 }
@@ -346,8 +349,16 @@ __global__ __launch_bounds__(32) void k_mlp_grad(const float *__restrict__ w,
 // third. Layer 3 (64 -> 2) and dH2 = dY W3 run on the CUDA cores per thread.
 // BF16 rounding happens where the mma.sync kernel (and the oracle) round.
 // Every gradient entry is written by exactly one thread of the CTA.
+// Bound by latency: a mini-batch of 4,096 is 32 CTAs with one chain of four
+// products each. So what no earlier kernel writes is done before step_order,
+// weights are staged in whole 16-byte chunks with their loads in flight
+// together, and partials leave as float4 (18 -> 10.5 us; scalar staging and
+// 64 strided stores per thread before). With the sum and Adam in one kernel
+// and both kernels released early, a batch takes 11.9 us instead of 26.7
+// (196 batches of 512).
 // ---------------------------------------------------------------------------
 constexpr int kTcThreads = 128;
+constexpr int kStepThreads = 64;  // k_mlp_step: the parameters over 91 SMs
 constexpr int kTcTilesPerBlock = 1;
 constexpr uint32_t kTcCols = 256;  // TMEM columns allocated (power of two >= 176)
 constexpr uint32_t kTcColGrad = 64, kTcColW3 = 160;
@@ -473,24 +484,40 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
   unsigned char *astb = reinterpret_cast<unsigned char *>(S.ast);
   unsigned char *a2b = reinterpret_cast<unsigned char *>(S.a2);
   unsigned char *b2b = reinterpret_cast<unsigned char *>(S.b2);
-  // ---- weights and constant operand parts --------------------------------
-  for (uint32_t i = tid; i < 64 * 16; i += kTcThreads) {
-    const uint32_t r = i / 16, k = i % 16;
-    *reinterpret_cast<__nv_bfloat16 *>(w1b + kmaj_off(r, k, 256)) =
-        __float2bfloat16_rn(k < MLP_IN ? w[OFF_W1 + i] : 0.f);
+  // ---- what no earlier kernel writes: barrier, TMEM, constant operand parts,
+  // the first tile's samples ------------------------------------------------
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (uint32_t i = tid; i < 64 * 64; i += kTcThreads) {
-    const uint32_t r = i / 64, k = i % 64;  // w2t master: [out r][in k]
-    const __nv_bfloat16 v = __float2bfloat16_rn(w[OFF_W2 + i]);
-    *reinterpret_cast<__nv_bfloat16 *>(w2b + kmaj_off(r, k, 1024)) = v;
-    *reinterpret_cast<__nv_bfloat16 *>(w2tb + kmaj_off(k, r, 1024)) = v;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&S.tmem)),
+                 "r"(kTcCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  for (uint32_t i = tid; i < 2 * 64; i += kTcThreads) S.w3[i / 64][i % 64] = bfr(w[OFF_W3 + i]);
-  for (uint32_t i = tid; i < 64; i += kTcThreads) {
-    S.b1[i] = w[OFF_B1 + i];
-    S.b2v[i] = w[OFF_B2 + i];
-  }
-  if (tid < 2) S.b3[tid] = w[OFF_B3 + tid];
+  const uint32_t nTiles = (n + kTcThreads - 1) / kTcThreads;
+  const uint32_t t0 = blockIdx.x * kTcTilesPerBlock;
+  const uint32_t t1 = min(t0 + kTcTilesPerBlock, nTiles);
+  float x[16], tg0, tg1, wt;
+  auto load_sample = [&](uint32_t tile) {
+    const uint32_t sIdx = tile * kTcThreads + tid;
+    const bool valid = tile < t1 && sIdx < n;
+    const uint32_t src = valid ? (order ? order[sIdx] : sIdx) : 0u;
+    const float2 *row = reinterpret_cast<const float2 *>(X) + (size_t)src * (MLP_IN / 2);
+#pragma unroll
+    for (int f = 0; f < 8; f++) {
+      const float2 q = valid && f < MLP_IN / 2 ? row[f] : make_float2(0.f, 0.f);
+      x[2 * f] = q.x;
+      x[2 * f + 1] = q.y;
+    }
+    const float2 t = valid ? reinterpret_cast<const float2 *>(T)[src] : make_float2(0.f, 0.f);
+    tg0 = t.x;
+    tg1 = t.y;
+    wt = valid ? (Wt ? Wt[src] : 1.f) : 0.f;
+  };
+  load_sample(t0);
   {
     // per sample: bst n 80..95 = [1, 0 ...], a2 m 64..127 = [1, 0 ...],
     // b2 n 8..15 = 0
@@ -504,17 +531,38 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
       *reinterpret_cast<uint4 *>(a2b + mn_off(n0, k, 2048)) = pack8(zero);
     *reinterpret_cast<uint4 *>(b2b + mn_off(8, k, 256)) = pack8(zero);
   }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  step_order();
+  step_release();
+  // ---- weights, in chunks of the operands' 8 elements ----------------------
+  {
+    const uint32_t r = tid >> 1, k = (tid & 1u) * 8u;  // W1: one chunk per thread
+    float v[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) v[i] = k + i < MLP_IN ? w[OFF_W1 + r * 16 + k + i] : 0.f;
+    *reinterpret_cast<uint4 *>(w1b + kmaj_off(r, k, 256)) = pack8(v);
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&S.tmem)),
-                 "r"(kTcCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (uint32_t c = 0; c < 4; c++) {  // W2 [out r][in k]: 512 chunks along k
+    const uint32_t i = c * kTcThreads + tid, r = i >> 3, k = (i & 7u) * 8u;
+    const float4 *p = reinterpret_cast<const float4 *>(w + OFF_W2 + r * 64 + k);
+    const float4 a = p[0], b = p[1];
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    *reinterpret_cast<uint4 *>(w2b + kmaj_off(r, k, 1024)) = pack8(v);
   }
+#pragma unroll
+  for (uint32_t c = 0; c < 4; c++) {  // its transpose: 512 chunks along r
+    const uint32_t i = c * kTcThreads + tid, k = i & 63u, r = (i >> 6) * 8u;
+    float v[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; j++) v[j] = w[OFF_W2 + (r + j) * 64 + k];
+    *reinterpret_cast<uint4 *>(w2tb + kmaj_off(k, r, 1024)) = pack8(v);
+  }
+  S.w3[tid >> 6][tid & 63u] = bfr(w[OFF_W3 + tid]);
+  if (tid < 64) {
+    S.b1[tid] = w[OFF_B1 + tid];
+    S.b2v[tid] = w[OFF_B2 + tid];
+  }
+  if (tid < 2) S.b3[tid] = w[OFF_B3 + tid];
   proxy_fence();
   tc_fence_before();
   __syncthreads();
@@ -527,9 +575,6 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
   uint32_t phase = 0;
   bool ok = true;
   float lossAcc = 0.f;
-  const uint32_t nTiles = (n + kTcThreads - 1) / kTcThreads;
-  const uint32_t t0 = blockIdx.x * kTcTilesPerBlock;
-  const uint32_t t1 = min(t0 + kTcTilesPerBlock, nTiles);
   // issue (thread 0) a chain of MMAs after the block's shared-memory
   // writes, then wait for it everywhere
   // (ok stays block-uniform: a wait that gave up anywhere stops every thread)
@@ -548,15 +593,7 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
     tc_fence_after();
   };
   for (uint32_t tile = t0; tile < t1 && ok; tile++) {
-    const uint32_t sIdx = tile * kTcThreads + tid;
-    const bool valid = sIdx < n;
-    const uint32_t src = valid ? (order ? order[sIdx] : sIdx) : 0u;
-    float x[16];
-#pragma unroll
-    for (int f = 0; f < 16; f++)
-      x[f] = (valid && f < MLP_IN) ? X[(size_t)src * MLP_IN + f] : 0.f;
-    const float tg0 = valid ? T[(size_t)src * 2] : 0.f, tg1 = valid ? T[(size_t)src * 2 + 1] : 0.f;
-    const float wt = valid ? (Wt ? Wt[src] : 1.f) : 0.f;
+    if (tile != t0) load_sample(tile);
     *reinterpret_cast<uint4 *>(bstb + mn_off(64, tid, 1536)) = pack8(x);
     *reinterpret_cast<uint4 *>(bstb + mn_off(72, tid, 1536)) = pack8(x + 8);
     // ---- layer 1: D_act = X W1^T (K = 16) -------------------------------
@@ -650,7 +687,7 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
     });
   }
   // ---- this CTA's gradient: row tid of D_grad and D_w3 ---------------------
-  float *out = partial + (size_t)blockIdx.x * (MLP_PAD + 1);
+  float *out = partial + (size_t)blockIdx.x * MLP_ROW;
   if (ok && t0 < t1) {
     float g[96], g3[16];
 #pragma unroll
@@ -658,14 +695,20 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
     tc_ld16(lane_base + kTcColW3, g3);
     tc_wait_ld();
     if (tid < 64) {
-      for (int j = 0; j < 64; j++) out[OFF_W2 + tid * 64 + j] = g[j];
+      float4 *o2 = reinterpret_cast<float4 *>(out + OFF_W2 + tid * 64);
+#pragma unroll
+      for (int j = 0; j < 16; j++)
+        o2[j] = make_float4(g[4 * j], g[4 * j + 1], g[4 * j + 2], g[4 * j + 3]);
       out[OFF_B2 + tid] = g[80];
       out[OFF_W3 + tid] = g3[0];
       out[OFF_W3 + 64 + tid] = g3[1];
       for (int o = 2; o < MLP_OUTP; o++) out[OFF_W3 + o * 64 + tid] = 0.f;
     } else {
       const uint32_t r = tid - 64;
-      for (int c = 0; c < MLP_INP; c++) out[OFF_W1 + r * MLP_INP + c] = g[64 + c];
+      float4 *o1 = reinterpret_cast<float4 *>(out + OFF_W1 + r * MLP_INP);
+#pragma unroll
+      for (int j = 0; j < MLP_INP / 4; j++)
+        o1[j] = make_float4(g[64 + 4 * j], g[65 + 4 * j], g[66 + 4 * j], g[67 + 4 * j]);
       out[OFF_B1 + r] = g[80];
       if (tid == 64) {
         out[OFF_B3] = g3[0];
@@ -692,31 +735,47 @@ __global__ __launch_bounds__(kTcThreads, 1) void k_mlp_grad_tc(
   }
 }
 
-// Sum of the per-block partials in block order.
-__global__ void k_mlp_reduce(const float *partial, uint32_t blocks, float *sum) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > MLP_PAD) return;
+// Parameter i's gradient (the loss at i = MLP_PAD): the blocks' partials in
+// block order.
+__device__ __forceinline__ float partial_sum(const float *__restrict__ partial, uint32_t blocks,
+                                             int i) {
   float s = 0.f;
-  for (uint32_t b = 0; b < blocks; b++) s += partial[(size_t)b * (MLP_PAD + 1) + i];
-  sum[i] = s;
+#pragma unroll 8
+  for (uint32_t b = 0; b < blocks; b++) s += partial[(size_t)b * MLP_ROW + i];
+  return s;
 }
 
-__global__ void k_mlp_adam(float *w, float *m, float *v, const float *grad,
-                           float lr, float b1, float b2, float eps,
-                           float c1, float c2, float *epochLoss, float batchSamples) {
+__global__ void k_mlp_reduce(const float *__restrict__ partial, uint32_t blocks, float *sum) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0 && epochLoss) *epochLoss += grad[MLP_PAD] * batchSamples;
-  if (i >= MLP_PAD) return;
+  if (i <= MLP_PAD) sum[i] = partial_sum(partial, blocks, i);
+}
+
+// The gradient's sum and the Adam update of its parameter: one latency chain
+// of loads, so one kernel of small blocks instead of two of 23 blocks each
+// (8 -> 7 us at 32 partials, and a launch less).
+__global__ __launch_bounds__(kStepThreads) void k_mlp_step(
+    const float *__restrict__ partial, uint32_t blocks, float *w, float *m, float *v, float lr,
+    float b1, float b2, float eps, float c1, float c2, float *epochLoss, float batchSamples) {
+  step_order();
+  step_release();
+  const int i = blockIdx.x * kStepThreads + threadIdx.x;
+  if (i > MLP_PAD) return;
+  if (i == MLP_PAD) {
+    if (epochLoss) *epochLoss += partial_sum(partial, blocks, i) * batchSamples;
+    return;
+  }
   if (!is_real_param(i)) {
     w[i] = 0.f;
     return;
   }
-  const float gr = grad[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gr;
-  const float vi = b2 * v[i] + (1.f - b2) * gr * gr;
+  const float m0 = m[i], v0 = v[i], w0 = w[i];
+  const float gr = partial_sum(partial, blocks, i);
+  // the contractions are spelled out: results do not hang on the compiler's choice
+  const float mi = __fmaf_rn(1.f - b1, gr, b1 * m0);
+  const float vi = __fmaf_rn((1.f - b2) * gr, gr, b2 * v0);
   m[i] = mi;
   v[i] = vi;
-  w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  w[i] = w0 - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
 // Batch inference (tests, the error monitor): one warp per 32 rows.
@@ -985,14 +1044,14 @@ int gvizCudaMlpGetWeights(gvizCudaMlp *m, float *w) {
 
 static int mlp_grad_launch(gvizCudaMlp *m, const float *dX, const float *dT,
                            const float *dW, const uint32_t *dOrder, uint32_t n,
-                           float scale) {
+                           float scale, uint32_t *blocksOut) {
   const uint32_t tiles = m->tc ? (n + kTcThreads - 1) / kTcThreads : (n + 31) / 32;
   const uint32_t per = m->tc ? kTcTilesPerBlock : kTilesPerBlock;
   const uint32_t blocks = (tiles + per - 1) / per;
   if (blocks > m->gradBlocks) {
     cudaFree(m->d_grad);
     m->d_grad = nullptr;
-    if (cudaMalloc(&m->d_grad, (size_t)blocks * (MLP_PAD + 1) * 4) != cudaSuccess)
+    if (cudaMalloc(&m->d_grad, (size_t)blocks * MLP_ROW * 4) != cudaSuccess)
       return GVIZ_CUDA_ERR_ALLOC;
     m->gradBlocks = blocks;
   }
@@ -1005,12 +1064,12 @@ static int mlp_grad_launch(gvizCudaMlp *m, const float *dX, const float *dT,
     attr = true;
   }
   if (m->tc)
-    k_mlp_grad_tc<<<blocks, kTcThreads, sizeof(TcSmem), m->stream>>>(
-        m->d_w, dX, dT, dW, dOrder, n, scale, m->d_grad, m->d_status);
+    launch_after(m->stream, k_mlp_grad_tc, dim3(blocks), dim3(kTcThreads), sizeof(TcSmem),
+                 (const float *)m->d_w, dX, dT, dW, dOrder, n, scale, m->d_grad, m->d_status);
   else
     k_mlp_grad<<<blocks, 32, sizeof(TrainSmem), m->stream>>>(m->d_w, dX, dT, dW, dOrder, n,
                                                              scale, m->d_grad);
-  k_mlp_reduce<<<(MLP_PAD + 1 + 255) / 256, 256, 0, m->stream>>>(m->d_grad, blocks, m->d_gsum);
+  *blocksOut = blocks;
   return GVIZ_CUDA_OK;
 }
 
@@ -1045,7 +1104,10 @@ int gvizCudaMlpGradient(gvizCudaMlp *m, const float *X, const float *T,
     cudaMalloc(&dW, n * 4);
     cudaMemcpy(dW, W, n * 4, cudaMemcpyHostToDevice);
   }
-  int rc = mlp_grad_launch(m, dX, dT, dW, nullptr, (uint32_t)n, (float)(1.0 / wsum));
+  uint32_t blocks = 0;
+  int rc = mlp_grad_launch(m, dX, dT, dW, nullptr, (uint32_t)n, (float)(1.0 / wsum), &blocks);
+  if (!rc)
+    k_mlp_reduce<<<(MLP_PAD + 1 + 255) / 256, 256, 0, m->stream>>>(m->d_grad, blocks, m->d_gsum);
   std::vector<float> gs(MLP_PAD + 1);
   if (!rc && cudaMemcpyAsync(gs.data(), m->d_gsum, (MLP_PAD + 1) * 4, cudaMemcpyDeviceToHost,
                              m->stream) == cudaSuccess &&
@@ -1117,13 +1179,15 @@ int gvizCudaMlpTrain(gvizCudaMlp *m, const float *X, const float *T,
       const uint32_t nb = (uint32_t)std::min<size_t>(batch, n - b0);
       double wsum = 0.0;
       for (uint32_t i = 0; i < nb; i++) wsum += W ? W[order[b0 + i]] : 1.0;
-      rc = mlp_grad_launch(m, dX, dT, dW, dOrder + b0, nb, (float)(1.0 / wsum));
+      uint32_t blocks = 0;
+      rc = mlp_grad_launch(m, dX, dT, dW, dOrder + b0, nb, (float)(1.0 / wsum), &blocks);
       if (rc) break;
       m->step++;
       const float c1 = 1.f - powf(b1, (float)m->step), c2 = 1.f - powf(b2, (float)m->step);
-      k_mlp_adam<<<(MLP_PAD + 255) / 256, 256, 0, m->stream>>>(
-          m->d_w, m->d_m, m->d_v, m->d_gsum, lr, b1, b2, eps, c1, c2,
-          lossOut ? m->d_epochLoss + ep : nullptr, (float)nb);
+      launch_after(m->stream, k_mlp_step, dim3((MLP_PAD + kStepThreads) / kStepThreads),
+                   dim3(kStepThreads), 0, (const float *)m->d_grad, blocks, m->d_w, m->d_m,
+                   m->d_v, lr, b1, b2, eps, c1, c2, lossOut ? m->d_epochLoss + ep : nullptr,
+                   (float)nb);
     }
   }
   k_mlp_to_dev<<<(MLP_PAD + 255) / 256, 256, 0, m->stream>>>(m->d_w, m->d_dev);
