@@ -1472,6 +1472,14 @@ __global__ __launch_bounds__(kCellThreads, kCellBlocksPerSM) void k_walk_f32_cel
 constexpr int kHubThreads = 128;
 constexpr uint32_t kHubRing = 1024;  // ring entries per warp
 constexpr int kHubTake = 2;          // entries a lane takes per round
+// Hubs times vertices up to which the hub walk runs beside the learned walk
+// instead of after it. Alone it is a latency chain of about 50 us in a few
+// blocks; beside, each of its blocks takes the room of a learned walk's block
+// and runs three times as long. A step on BA graphs, after -> beside: 30,000
+// vertices and 1,024 hubs 217 -> 196 us, 262,144 and 1,024 (2^28) 470 -> 460,
+// 524,288 and 256 765 -> 742, 900,000 and 256 1204 -> 1191; above, 524,288 and
+// 1,024 766 -> 765, 262,144 and 4,096 499 -> 500, 900,000 and 1,024 1204 -> 1222.
+constexpr uint64_t kHubBeside = 1ull << 28;
 
 struct FarHubArgs {
   WalkArgs w;
@@ -2070,17 +2078,31 @@ static void enqueue_far_hub_walk(gvizCudaForce *h, const FarHubArgs &ha) {
 
 static void enqueue_far_walk(gvizCudaForce *h, const WalkArgs &a, uint64_t *counters);
 
-// The learned walk (see k_walk_f32_far and k_walk_f32_cells), then the hub
-// targets' plain walk when params.farHubTargets asks for one, then the hubs'
-// epilogues, which replace the learned walk's forces of those vertices. (The
-// hub walk on a side stream beside the learned walk was measured slower:
-// 7.15 vs 6.90 ms per R-MAT scale-22 step with 16,384 hub targets.)
+// The learned walk (see k_walk_f32_far and k_walk_f32_cells) and the hub
+// targets' plain walk when params.farHubTargets asks for one, after it or, on
+// the side stream, beside it (kHubBeside); then the hubs' epilogues, which
+// replace the learned walk's forces of those vertices.
 static void enqueue_far(gvizCudaForce *h, const WalkArgs &a, uint64_t *counters) {
-  enqueue_far_walk(h, a, counters);
-  if (!(h->nFarHubs > 0 && h->d_farHubs)) return;
+  if (!(h->nFarHubs > 0 && h->d_farHubs)) {
+    enqueue_far_walk(h, a, counters);
+    return;
+  }
   const FarHubArgs ha = far_hub_args(h, a);
-  enqueue_far_hub_walk(h, ha);
-  prof_mark(h, "bh_walk_hubs");
+  if (h->side && !h->profiling && h->nFarHubs * (uint64_t)h->V <= kHubBeside) {
+    const cudaStream_t st = h->stream;
+    cudaEventRecord(h->evFork, st);
+    cudaStreamWaitEvent(h->side, h->evFork, 0);
+    h->stream = h->side;
+    enqueue_far_hub_walk(h, ha);
+    h->stream = st;
+    cudaEventRecord(h->evJoin, h->side);
+    enqueue_far_walk(h, a, counters);
+    cudaStreamWaitEvent(st, h->evJoin, 0);
+  } else {
+    enqueue_far_walk(h, a, counters);
+    enqueue_far_hub_walk(h, ha);
+    prof_mark(h, "bh_walk_hubs");
+  }
   k_far_hub_epilogue<<<blocks(h->nFarHubs, 256), 256, 0, h->stream>>>(ha);
 }
 

@@ -84,7 +84,8 @@ struct gvizCudaForce {
   int device = 0;
   cudaStream_t stream = nullptr;
   // attraction depends on positions only: it runs on `side`, forked from
-  // and joined back to `stream` around the tree build (null: in order)
+  // and joined back to `stream` around the tree build (null: in order), as is
+  // the hub targets' walk around the learned one
   cudaStream_t side = nullptr;
   cudaEvent_t evFork = nullptr, evJoin = nullptr;
   // gvizCudaForceRunHost: the uploads' stream and its events (made at its
