@@ -1407,8 +1407,12 @@ __device__ __forceinline__ uint32_t emit_pre(const EM &a, const EmitShared &s, u
 }
 
 // Node and leaf records in preorder: block j emits internal nodes and
-// buckets [C0, C0 + kEmitSpan), C0 = kEmitSpan j, one per thread.
-__global__ __launch_bounds__(kThreads) void k_emit(EM a) {
+// buckets [C0, C0 + kEmitSpan), C0 = kEmitSpan j, one per thread. Bound by the
+// latency of its gathers along the tree (15 of 17 cycles between a warp's
+// instructions), so eight blocks share an SM at 32 registers, a few of them
+// spilled: 1,048,576 vertices 100 -> 79 us (five blocks at 48 registers; six
+// at 40: 91).
+__global__ __launch_bounds__(kThreads, 8) void k_emit(EM a) {
   step_order();
   __shared__ EmitShared s;
   const uint32_t U = a.counts[2];
