@@ -77,6 +77,7 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_judgeOut);
   dfree(h->d_judgeRep);
   dfree(h->d_judgePart);
+  dfree(h->d_exactRoom);
   dfree(h->d_rowOff);
   dfree(h->d_cols);
   dfree(h->d_degree);
@@ -1322,6 +1323,8 @@ int64_t gvizCudaForceTreeNodes(gvizCudaForce *h, size_t cap, int32_t *depth,
   return rc ? (int64_t)rc : w;
 }
 
+static constexpr size_t kExactKept = 16u << 20;
+
 int gvizCudaForceExactRepulsion(gvizCudaForce *h, const uint32_t *targets,
                                 size_t n, double *out) {
   if (!h || (n && (!targets || !out))) return GVIZ_CUDA_ERR_ARG;
@@ -1329,20 +1332,27 @@ int gvizCudaForceExactRepulsion(gvizCudaForce *h, const uint32_t *targets,
   for (size_t i = 0; i < n; i++)
     if (targets[i] >= h->V) return set_err(h, GVIZ_CUDA_ERR_ARG);
   DeviceGuard guard(h->device);
-  uint32_t *dt = nullptr;
-  double2 *dout = nullptr, *part = nullptr;
-  int rc = dalloc(h, &dt, n) | dalloc(h, &dout, n) |
-           dalloc(h, &part, (size_t)exact_judge_splits(h->V, n) * n);
-  if (!rc) {
-    cudaMemcpy(dt, targets, n * 4, cudaMemcpyHostToDevice);
-    enqueue_exact_judge(h, dt, n, dout, part);
-    rc = sync_and_check(h);
-    if (!rc && cudaMemcpy(out, dout, n * 16, cudaMemcpyDeviceToHost) != cudaSuccess)
-      rc = set_err(h, GVIZ_CUDA_ERR_CUDA);
+  // the results, the partial sums and the targets; kept for the next call up
+  // to kExactKept bytes (an allocation above 2 MB takes 0.6 ms)
+  const size_t parts = (size_t)exact_judge_splits(h->V, n) * n;
+  const size_t need = n + parts + (n + 3) / 4;
+  if (need > h->exactRoom) {
+    dfree(h->d_exactRoom);
+    h->exactRoom = 0;
+    if (const int rc = dalloc(h, &h->d_exactRoom, need)) return rc;
+    h->exactRoom = need;
   }
-  dfree(dt);
-  dfree(dout);
-  dfree(part);
+  double2 *dout = h->d_exactRoom, *part = dout + n;
+  uint32_t *dt = reinterpret_cast<uint32_t *>(part + parts);
+  cudaMemcpy(dt, targets, n * 4, cudaMemcpyHostToDevice);
+  enqueue_exact_judge(h, dt, n, dout, part);
+  int rc = sync_and_check(h);
+  if (!rc && cudaMemcpy(out, dout, n * 16, cudaMemcpyDeviceToHost) != cudaSuccess)
+    rc = set_err(h, GVIZ_CUDA_ERR_CUDA);
+  if (h->exactRoom * sizeof(double2) > kExactKept) {
+    dfree(h->d_exactRoom);
+    h->exactRoom = 0;
+  }
   return rc;
 }
 

@@ -231,6 +231,8 @@ struct gvizCudaForce {
   double2 *d_judgeExact = nullptr, *d_judgeOut = nullptr;  // n; 2n (learned, plain)
   double2 *d_judgeRep = nullptr;   // V: repulsion of one evaluation
   double2 *d_judgePart = nullptr;  // split sums of the exact repulsion
+  double2 *d_exactRoom = nullptr;  // gvizCudaForceExactRepulsion: results, split sums, targets
+  size_t exactRoom = 0;            // its entries
 
   // --- CUDA graph of one step ---
   cudaGraphExec_t stepExec = nullptr;

@@ -353,9 +353,15 @@ __global__ __launch_bounds__(kThreads) void k_exact_f64(Exact64Args a) {
 // a block's graphs are split into gridDim.y ranges of whole tiles, so that a
 // few thousand targets fill the GPU (4,096 targets are 32 blocks per range);
 // every range's sums go to `partial` and k_judge_combine adds them in range
-// order. FP64 issue bounds the loop: without overlap prevention a term is
-// num / d^2 along d (one division), with it the term of rep_term64. 4,096
-// targets among 131,072 vertices took 48 ms in 16 blocks of one serial sum.
+// order. FP64 issue bounds the loop. Without overlap prevention a term is
+// num / d^2 along d: ten FP64 instructions on a straight-line path with a
+// reciprocal of its own, chunks of 32 sources that meet the target, a
+// coincident point or an extreme distance taken again with the division; with
+// overlap prevention it is the term of rep_term64. 4,096 targets among 131,072
+// vertices: 48 ms in 16 blocks of one serial sum, 0.90 split over blocks with
+// a division and three branches per term, 0.55 now (0.30 at the FP64 pipe's
+// rate). 8 / 16 / 24 / 32 / 48 blocks per SM of the 8 that fit take 0.77 / 0.62
+// / 0.58 / 0.55 / 0.51, the sum of the partials 10 / 14 / 20 / 25 / 36 us.
 struct JudgeArgs {
   Exact64Args e;
   double2 *partial;  // [gridDim.y][n]
@@ -363,12 +369,28 @@ struct JudgeArgs {
 
 constexpr int kJudgeThreads = 128;
 constexpr int kJudgeTile = 128;
+constexpr uint32_t kJudgeChunk = 32;
+constexpr int kJudgeBlocksPerSM = 8;
+constexpr int kCombineThreads = 64;  // a chain of loads per target: over many SMs
+// high words of the squared distances the straight-line terms take:
+// [2^-900, 2^1022), where neither the reciprocal nor its product overflows
+constexpr uint32_t kJudgeLow = (1023u - 900u) << 20, kJudgeSpan = (1022u + 900u) << 20;
+
+// 1 / d for d in [2^-900, 2^1022): the hardware's approximation and one step
+// of the third-order (Chebyshev) iteration r + r (e + e^2), e = 1 - d r, which
+// leaves 2^-52: no branch, three FP64 instructions.
+__device__ __forceinline__ double reciprocal64(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = __fma_rn(-d, r, 1.0);
+  return __fma_rn(r, __fma_rn(e, e, e), r);
+}
 
 template <int MODEL, bool OVERLAP>
-__global__ __launch_bounds__(kJudgeThreads) void k_judge_f64(JudgeArgs ja) {
+__global__ __launch_bounds__(kJudgeThreads, kJudgeBlocksPerSM) void k_judge_f64(JudgeArgs ja) {
   const Exact64Args &a = ja.e;
   __shared__ double2 sp[kJudgeTile];
-  __shared__ double2 smr[kJudgeTile];
+  __shared__ double sm[kJudgeTile], sr[kJudgeTile];
   __shared__ uint32_t sRange[2];
   const uint32_t t = blockIdx.x * kJudgeThreads + threadIdx.x;
   const bool act = t < a.n;
@@ -405,40 +427,62 @@ __global__ __launch_bounds__(kJudgeThreads) void k_judge_f64(JudgeArgs ja) {
       sp[threadIdx.x] = a.pos[j];
       const double m = a.mass[j];
       // FR: the truncated mass times k^2 (src/embedders/gvizForceModel.c:20)
-      smr[threadIdx.x] = make_double2(
-          !OVERLAP && MODEL == GVIZ_CUDA_MODEL_FR ? a.kk * (double)(unsigned long long)m : m,
-          a.radius[j]);
+      sm[threadIdx.x] =
+          !OVERLAP && MODEL == GVIZ_CUDA_MODEL_FR ? a.kk * (double)(unsigned long long)m : m;
+      if (OVERLAP) sr[threadIdx.x] = a.radius[j];
     }
     __syncthreads();
     const uint32_t cnt = min((uint32_t)kJudgeTile, hi - t0);
     if (!act) continue;
-    double bx = 0.0, by = 0.0;
-#pragma unroll 2
-    for (uint32_t q = 0; q < cnt; q++) {
-      const uint32_t jj = t0 + q;
-      if (jj == v || jj < gb || jj >= ge) continue;
-      const double2 u = sp[q];
-      const double2 mr = smr[q];
-      if (OVERLAP) {
-        rep_term64<MODEL>(p.x, p.y, u.x, u.y, mv, mr.x, rv + mr.y, a.kk, a.overlapC, v, jj,
-                          bx, by);
-      } else {
-        const double dx = u.x - p.x, dy = u.y - p.y;
-        const double d2 = __fma_rn(dx, dx, dy * dy);
-        if (d2 > 0.0) {
-          const double s = -mr.x / d2;
+    for (uint32_t c0 = 0; c0 < cnt; c0 += kJudgeChunk) {
+      double bx = 0.0, by = 0.0;
+      // a whole chunk of the target's graph, straight-line: taken again below
+      // when it meets the target, a coincident point or an extreme distance
+      const bool whole = !OVERLAP && c0 + kJudgeChunk <= cnt && t0 + c0 >= gb &&
+                         t0 + c0 + kJudgeChunk <= ge;
+      uint32_t odd = whole ? 0u : kJudgeSpan;
+      if (whole) {
+#pragma unroll 4
+        for (uint32_t q = c0; q < c0 + kJudgeChunk; q++) {
+          const double2 u = sp[q];
+          const double dx = u.x - p.x, dy = u.y - p.y;
+          const double d2 = __fma_rn(dx, dx, dy * dy);
+          odd = max(odd, (uint32_t)__double2hiint(d2) - kJudgeLow);
+          const double s = -sm[q] * reciprocal64(d2);
           bx = __fma_rn(s, dx, bx);
           by = __fma_rn(s, dy, by);
-        } else {
-          double ux, uy;
-          coincident_dir(v, jj, ux, uy);
-          bx -= mr.x * a.overlapC * ux;
-          by -= mr.x * a.overlapC * uy;
         }
       }
+      if (odd >= kJudgeSpan) {
+        bx = by = 0.0;
+        const uint32_t c1 = min(c0 + kJudgeChunk, cnt);
+#pragma unroll 1
+        for (uint32_t q = c0; q < c1; q++) {
+          const uint32_t jj = t0 + q;
+          if (jj == v || jj < gb || jj >= ge) continue;
+          const double2 u = sp[q];
+          if (OVERLAP) {
+            rep_term64<MODEL>(p.x, p.y, u.x, u.y, mv, sm[q], rv + sr[q], a.kk, a.overlapC, v, jj,
+                              bx, by);
+          } else {
+            const double dx = u.x - p.x, dy = u.y - p.y;
+            const double d2 = __fma_rn(dx, dx, dy * dy);
+            if (d2 > 0.0) {
+              const double s = -sm[q] / d2;
+              bx = __fma_rn(s, dx, bx);
+              by = __fma_rn(s, dy, by);
+            } else {
+              double ux, uy;
+              coincident_dir(v, jj, ux, uy);
+              bx -= sm[q] * a.overlapC * ux;
+              by -= sm[q] * a.overlapC * uy;
+            }
+          }
+        }
+      }
+      ax += bx;
+      ay += by;
     }
-    ax += bx;
-    ay += by;
   }
   if (!act) return;
   if (!OVERLAP && MODEL != GVIZ_CUDA_MODEL_FR) {
@@ -448,10 +492,11 @@ __global__ __launch_bounds__(kJudgeThreads) void k_judge_f64(JudgeArgs ja) {
   ja.partial[(size_t)blockIdx.y * a.n + t] = make_double2(ax, ay);
 }
 
-__global__ __launch_bounds__(kThreads) void k_judge_combine(JudgeArgs ja, uint32_t splits) {
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+__global__ __launch_bounds__(kCombineThreads) void k_judge_combine(JudgeArgs ja, uint32_t splits) {
+  const uint32_t t = blockIdx.x * kCombineThreads + threadIdx.x;
   if (t >= ja.e.n) return;
   double sx = 0.0, sy = 0.0;
+#pragma unroll 16
   for (uint32_t s = 0; s < splits; s++) {
     const double2 q = ja.partial[(size_t)s * ja.e.n + t];
     sx += q.x;
@@ -846,11 +891,11 @@ void enqueue_exact_f64(gvizCudaForce *h) {
   prof_mark(h, "exact_f64");
 }
 
-// Source ranges of the judge's kernel for n targets among V vertices: 16
+// Source ranges of the judge's kernel for n targets among V vertices: 32
 // blocks per SM where the tiles allow.
 uint32_t exact_judge_splits(size_t V, size_t n) {
   const size_t tb = (n + kJudgeThreads - 1) / kJudgeThreads;
-  const size_t s = tb ? (148 * 16 + tb - 1) / tb : 1;
+  const size_t s = tb ? 148 * 32 / tb : 1;
   return (uint32_t)std::max<size_t>(1, std::min(s, (V + kJudgeTile - 1) / kJudgeTile));
 }
 
@@ -873,7 +918,7 @@ void enqueue_exact_judge(gvizCudaForce *h, const uint32_t *d_targets, size_t n,
     if (ov) k_judge_f64<GVIZ_CUDA_MODEL_LINLOG, true><<<grid, kJudgeThreads, 0, h->stream>>>(ja);
     else k_judge_f64<GVIZ_CUDA_MODEL_LINLOG, false><<<grid, kJudgeThreads, 0, h->stream>>>(ja);
   }
-  k_judge_combine<<<blocks(n, kThreads), kThreads, 0, h->stream>>>(ja, splits);
+  k_judge_combine<<<blocks(n, kCombineThreads), kCombineThreads, 0, h->stream>>>(ja, splits);
 }
 
 void enqueue_fa2(gvizCudaForce *h) {

@@ -64,3 +64,22 @@ def test_judge_coincident_points_repel():
     # the pair's terms are opposite, of size numer * C = 100; the third's is 1/4
     assert abs(np.linalg.norm(f[0] - [-0.25, 0.0]) - 100.0) <= 1e-10
     assert np.abs(f[0] + f[1] + [0.5, 0.0]).max() <= 1e-10
+
+
+@pytest.mark.parametrize("scale", [1e-140, 1e-130, 1.0, 1e150, 9e153])
+@pytest.mark.parametrize("model", [0, 1])
+def test_judge_at_extreme_distances(scale, model):
+    """Squared distances on both sides of the range whose reciprocals the
+    straight-line terms take (2^-900 to 2^1022), in whole chunks and the rest."""
+    from grapher_b200 import graphs
+    n = 100
+    row, col, _ = graphs.batch([(n,) + graphs.random_connected(n, 0.0, 1)])
+    lay = make_layout(row, col, cfg(model=model))
+    p = np.random.default_rng(3).uniform(0.0, 1.0, (n, 2)) * scale
+    lay.set_positions(p.reshape(-1))
+    mass = np.ones(n) if model == 0 else 1.0 + np.diff(row).astype(np.float64)
+    got = lay.exact_repulsion(np.arange(n, dtype=np.uint32))
+    lay.close()
+    for v in range(n):
+        want, size = _forces(p, v, 0, n, mass, np.zeros(n), model)
+        assert np.abs(got[v] - want).max() <= 1e-12 * size
