@@ -46,6 +46,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWalkThreads = 128;
+constexpr uint32_t kWalkList = 1024;  // listed nodes per warp of the walk
 constexpr int kExactTile = 256;
 constexpr uint32_t kInf = 0xffffffffu;
 
@@ -201,7 +202,14 @@ __device__ __forceinline__ NodeRec load_node(const Walk64Args &a, uint32_t i) {
   return r;
 }
 
-template <int MODEL>
+// Each warp walks `targets` path-sorted targets together, a lane for each.
+// LISTS: a target's lane only lists the nodes whose terms it takes; when a
+// list is full and at the end all lanes compute listed terms side by side, 32 /
+// targets of them per target, added in list order by shuffles. Without, a
+// target's own lane computes each term as the walk meets it, while the others
+// wait: a term (a square root, three divisions) is longer than a step of the
+// walk. The sums are the same to the bit.
+template <int MODEL, bool LISTS>
 __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
   step_order();
   const unsigned lane = threadIdx.x & 31u;
@@ -221,7 +229,42 @@ __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
     mv = a.mass[v];
     rv = a.radius[v];
   }
+  // lane = target * helpers + helper while terms are computed
+  const uint32_t helpers = LISTS ? 32u / a.targets : 1u, mine = lane / helpers;
+  const double tx = __shfl_sync(0xffffffffu, vx, mine), ty = __shfl_sync(0xffffffffu, vy, mine);
+  const double tm = __shfl_sync(0xffffffffu, mv, mine), tr = __shfl_sync(0xffffffffu, rv, mine);
+  const uint32_t tv = __shfl_sync(0xffffffffu, v, mine);
+  __shared__ uint32_t lists[kWalkThreads / 32][LISTS ? kWalkList : 1u];
+  uint32_t *const warpList = lists[threadIdx.x >> 5];
+  const uint32_t room = kWalkList / a.targets;
+  uint32_t cnt = 0;  // listed for the lane's target
   double ax = 0.0, ay = 0.0;
+  const auto take_lists = [&]() {
+    __syncwarp();
+    const uint32_t n = __shfl_sync(0xffffffffu, cnt, mine);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
+    const uint32_t *const list = warpList + mine * room;
+    for (uint32_t k = 0; k < most; k += helpers) {
+      const uint32_t e = k + lane % helpers;
+      double fx = 0.0, fy = 0.0;
+      if (e < n) {
+        const NodeRec r = load_node(a, list[e]);
+        const bool isLeaf = r.n2.y >= 0;
+        rep_term64<MODEL>(tx, ty, r.n0.x, r.n0.y, tm, r.n1.x, isLeaf ? tr + r.n1.y : tr, a.kk,
+                          a.overlapC, tv, isLeaf ? (uint32_t)r.n2.y : tv, fx, fy);
+      }
+      for (uint32_t j = 0; j < helpers; j++) {
+        const double ux = __shfl_sync(0xffffffffu, fx, mine * helpers + j);
+        const double uy = __shfl_sync(0xffffffffu, fy, mine * helpers + j);
+        if (k + j < n) {
+          ax += ux;
+          ay += uy;
+        }
+      }
+    }
+    cnt = 0;
+    __syncwarp();
+  };
   uint32_t nxt = resume < myEnd ? resume : kInf;
   uint32_t cur = __reduce_min_sync(0xffffffffu, nxt);
   // The walk is a chain of node records. The one after `cur` is cur + 1 where
@@ -238,10 +281,12 @@ __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
     const bool active = cur >= resume && cur < myEnd;
     const bool isLeaf = n2.y >= 0;
     const bool massOk = n1.x != 0.0;
-    bool open = false;
+    bool open = false, term = false;
     if (active && massOk) {
       if (isLeaf) {
-        if ((uint32_t)n2.y != v)
+        if (LISTS)
+          term = (uint32_t)n2.y != v;
+        else if ((uint32_t)n2.y != v)
           rep_term64<MODEL>(vx, vy, n0.x, n0.y, mv, n1.x, rv + n1.y, a.kk,
                             a.overlapC, v, (uint32_t)n2.y, ax, ay);
       } else {
@@ -253,12 +298,18 @@ __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
         const double lhs = 4.0 * n1.y * n1.y, rhs = a.theta2 * d2;
         bool accept = lhs < rhs * (1.0 - 1e-12);
         if (!accept && !(lhs > rhs * (1.0 + 1e-12))) accept = (2.0 * n1.y) / sqrt(d2) < a.theta;
-        if (accept)
+        if (!accept)
+          open = true;
+        else if (LISTS)
+          term = true;
+        else
           rep_term64<MODEL>(vx, vy, n0.x, n0.y, mv, n1.x, rv, a.kk,
                             a.overlapC, v, v, ax, ay);
-        else
-          open = true;
       }
+    }
+    if (LISTS) {
+      if (term) warpList[lane * room + cnt++] = cur;
+      if (__any_sync(0xffffffffu, cnt == room)) take_lists();
     }
     if (active) resume = open ? cur + 1u : behind;
     nxt = resume < myEnd ? resume : kInf;
@@ -271,9 +322,16 @@ __global__ __launch_bounds__(kWalkThreads) void k_walk_f64(Walk64Args a) {
     else if (cur != kInf)  // the next graph's tree
       n = load_node(a, cur);
   }
-  if (!act) return;
-  const double2 at = a.attD[v];
-  force_epilogue(a.epi, v, at.x, at.y, ax, ay);
+  if constexpr (LISTS) {
+    take_lists();
+    if (!__shfl_sync(0xffffffffu, act ? 1 : 0, mine) || lane % helpers != 0u) return;
+    const double2 at = a.attD[tv];
+    force_epilogue(a.epi, tv, at.x, at.y, ax, ay);
+  } else {
+    if (!act) return;
+    const double2 at = a.attD[v];
+    force_epilogue(a.epi, v, at.x, at.y, ax, ay);
+  }
 }
 
 struct Exact64Args {
@@ -845,13 +903,24 @@ void enqueue_attraction_f64(gvizCudaForce *h) {
 // Targets per warp of the FP64 walk: 32 path-sorted targets share a walk, but
 // below 148 SMs x 20 warps the walk's latency counts, not the work, and
 // fewer targets per warp make more and shorter walks. A target's sum does not
-// depend on it. Walk in us with 32 / 16 / 8 / 4 targets: 700 vertices 129 /
-// 102 / 82 / 70, 9,000 199 / 154 / 128 / 117, 20,000 205 / 168 / 154 / 217,
-// 40,000 221 / 204 / 280 / 371, 80,000 264 / 355 / 465 / 729.
+// depend on it. Walk in us (LinLog BA, theta 0.8) with 2 / 4 / 8 / 16 / 32
+// targets and lists: 700 vertices 41 / 48 / 57 / 74 / 113, 3,000 55 / 61 / 70 /
+// 96 / 150, 9,000 118 / 83 / 88 / 115 / 178, 20,000 225 / 150 / 113 / 135 / 200,
+// 40,000 436 / 287 / 205 / 168 / 228; without lists 65, 92, 118, 152 and 192 at
+// its best of 4 to 32. With a warp full of targets there are no idle lanes to
+// compute terms and the walk without lists is the faster: 80,000 258 against
+// 272, 200,000 509 against 680.
 static uint32_t walk64_targets(size_t V) {
-  uint32_t t = 4;
+  uint32_t t = 2;
   while (t < 32 && V > (size_t)t * 148 * 20) t *= 2;
   return t;
+}
+
+template <int MODEL>
+static void launch_walk64(const Walk64Args &a, cudaStream_t st) {
+  const uint32_t grid = blocks(((a.V + a.targets - 1) / a.targets) * (size_t)32, kWalkThreads);
+  if (a.targets < 32) k_walk_f64<MODEL, true><<<grid, kWalkThreads, 0, st>>>(a);
+  else k_walk_f64<MODEL, false><<<grid, kWalkThreads, 0, st>>>(a);
 }
 
 void enqueue_walk_f64(gvizCudaForce *h) {
@@ -874,11 +943,8 @@ void enqueue_walk_f64(gvizCudaForce *h) {
   a.targets = walk64_targets(h->V);
   a.V = (uint32_t)h->V;
   a.maxNodes = (uint32_t)h->maxNodes;
-  const uint32_t grid = blocks(((h->V + a.targets - 1) / a.targets) * 32, kWalkThreads);
-  if (h->model == GVIZ_CUDA_MODEL_FR)
-    k_walk_f64<GVIZ_CUDA_MODEL_FR><<<grid, kWalkThreads, 0, h->stream>>>(a);
-  else
-    k_walk_f64<GVIZ_CUDA_MODEL_LINLOG><<<grid, kWalkThreads, 0, h->stream>>>(a);
+  if (h->model == GVIZ_CUDA_MODEL_FR) launch_walk64<GVIZ_CUDA_MODEL_FR>(a, h->stream);
+  else launch_walk64<GVIZ_CUDA_MODEL_LINLOG>(a, h->stream);
   prof_mark(h, "bh_walk_f64");
 }
 

@@ -61,3 +61,36 @@ def test_walk_is_the_same_alone_and_in_a_forest(model):
         want = lay.forces()["structForce"]
         lay.close()
         assert np.array_equal(got[2 * int(offs[g]):2 * int(offs[g + 1])], want), n
+
+
+@pytest.mark.parametrize("model", [0, 1])
+@pytest.mark.parametrize("n", [700, 5921, 11841, 23681])
+def test_listed_terms_add_in_walk_order(n, model):
+    """At every number of targets per warp below 32 the walk lists its terms and
+    helper lanes compute them; with 32 each lane adds its own as it goes. The
+    same bits, with a dense core whose lists fill several times, coincident
+    points and radii."""
+    from grapher_b200 import graphs
+    x = graphs.randomize_positions(n, 80.0, n).reshape(-1, 2)
+    x[: n // 4] *= 1e-3
+    x[n // 2: n // 2 + 5] = x[n // 2]
+    big = 48000  # with this graph beside it every warp holds 32 targets
+    parts = [(n,) + graphs.random_connected(n, 0.0, 3 + n),
+             (big,) + graphs.random_connected(big, 0.0, 4)]
+    row, col, offs = graphs.batch(parts)
+    c = cfg(model=model, theta=0.3, precision="fp64", gravity=1.0, prevent_overlap=True,
+            radius_base=0.01)
+    forest = make_layout(row, col, c, graph_offsets=offs)
+    forest.begin(0, positions=np.concatenate([x.reshape(-1),
+                                              graphs.randomize_positions(big, 80.0, 1)]))
+    forest.step()
+    want = forest.forces()["structForce"][:2 * n]
+    forest.close()
+    r, k = graphs.to_csr(*parts[0])
+    lay = make_layout(r, k, c)
+    lay.begin(0, positions=x.reshape(-1))
+    lay.step()
+    got = lay.forces()["structForce"]
+    lay.close()
+    assert np.all(np.isfinite(want))
+    assert np.array_equal(got, want)
