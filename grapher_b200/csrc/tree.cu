@@ -35,10 +35,14 @@
 #include "scan.cuh"
 
 // Super-ranges such that neither level's lists outgrow k_top's shared memory:
-// about 8 nodes span a block's edge, so 2^12, 2^14 and 2^16 buckets have
-// level-1 lists of ~120, ~500 and ~2,000 nodes, and level 2 has as many per
-// 16, 64 and 256 super-ranges.
-static int super_bits(size_t V) { return V <= (1u << 17) ? 12 : (V <= (1u << 21) ? 14 : 16); }
+// about 8 nodes span a block's edge, so 2^12, 2^14, 2^15 and 2^16 buckets have
+// level-1 lists of ~120, ~500, ~1,000 and ~2,000 nodes, and level 2 has as many
+// per 16, 64, 128 and 256 super-ranges. Node phase in us with 14 / 15 / 16 bits:
+// BA 1,500,000 371 / 358 / 596, 3,000,000 869 / 679 / 893, R-MAT 4,194,304 1,634
+// / 1,342 / 1,601.
+static int super_bits(size_t V) {
+  return V <= (1u << 17) ? 12 : (V <= (1u << 20) ? 14 : (V <= (1u << 22) ? 15 : 16));
+}
 
 // super-ranges of the tree build's nodes above blocks (see node_level)
 size_t top_count_entries(size_t V) { return (V >> super_bits(V)) + 1; }
@@ -1062,24 +1066,36 @@ __global__ __launch_bounds__(THREADS) void k_top(BU a) {
 }
 
 constexpr int kTopCap = 2048;  // 156 KB of shared memory, 188 with second moments
+// With 2^16 buckets to a super-range some lists are longer. All the shared memory
+// there is leaves no L1: 30 us slower where 2,048 suffice (BA 1,500,000 401 against
+// 371), but lists worked off in global memory take longer (R-MAT 4,194,304 with 16
+// bits 1,393 against 1,601).
+template <bool kQ>
+constexpr int kTopCapLarge = kQ ? 2432 : 2944;
 constexpr int kTop1Threads = 512, kTop2Threads = 1024;
 
-template <bool kQ>
-void launch_top(const BU &bu, uint32_t V, cudaStream_t st) {
-  constexpr size_t smem = sizeof(TopShared<kQ, kTopCap>);
-  const uint32_t supers = (uint32_t)top_count_entries(V);
-  launch_after(st, k_top<kQ, 1, kTopCap, kTop1Threads>, supers, kTop1Threads, smem, bu);
+template <bool kQ, int CAP>
+void launch_top_cap(const BU &bu, uint32_t supers, cudaStream_t st) {
+  constexpr size_t smem = sizeof(TopShared<kQ, CAP>);
+  launch_after(st, k_top<kQ, 1, CAP, kTop1Threads>, supers, kTop1Threads, smem, bu);
   // a layout of one super-range has no nodes above it
-  if (supers > 1)
-    launch_after(st, k_top<kQ, 2, kTopCap, kTop2Threads>, 1, kTop2Threads, smem, bu);
+  if (supers > 1) launch_after(st, k_top<kQ, 2, CAP, kTop2Threads>, 1, kTop2Threads, smem, bu);
 }
 
 template <bool kQ>
+void launch_top(const BU &bu, uint32_t V, cudaStream_t st) {
+  const uint32_t supers = (uint32_t)top_count_entries(V);
+  if (super_bits(V) < 16) launch_top_cap<kQ, kTopCap>(bu, supers, st);
+  else launch_top_cap<kQ, kTopCapLarge<kQ>>(bu, supers, st);
+}
+
+template <bool kQ, int CAP>
 void top_smem_limits() {
-  constexpr int smem = (int)sizeof(TopShared<kQ, kTopCap>);
-  cudaFuncSetAttribute(k_top<kQ, 1, kTopCap, kTop1Threads>,
+  constexpr int smem = (int)sizeof(TopShared<kQ, CAP>);
+  static_assert(smem <= 227 * 1024, "a block's shared memory");
+  cudaFuncSetAttribute(k_top<kQ, 1, CAP, kTop1Threads>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_top<kQ, 2, kTopCap, kTop2Threads>,
+  cudaFuncSetAttribute(k_top<kQ, 2, CAP, kTop2Threads>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
@@ -1819,8 +1835,10 @@ void enqueue_group_export(gvizCudaForce *h, uint32_t *groupOf) {
 void tree_set_smem_limits() {
   cudaFuncSetAttribute(k_sort_runs, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        GVIZ_FIX_MAX * 20);
-  top_smem_limits<false>();
-  top_smem_limits<true>();
+  top_smem_limits<false, kTopCap>();
+  top_smem_limits<true, kTopCap>();
+  top_smem_limits<false, kTopCapLarge<false>>();
+  top_smem_limits<true, kTopCapLarge<true>>();
 }
 
 // Inspection: every cell of the compressed tree (branching nodes and

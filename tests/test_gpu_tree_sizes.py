@@ -73,3 +73,18 @@ def test_forest_above_blocks(oracle):
         od, ohi, olo, _ = oracle.quadtree_leaves(p, np.ones(len(p)), 2)
         s = slice(int(offs[g]), int(offs[g + 1]))
         assert np.array_equal(d[s], od) and np.array_equal(hi[s], ohi) and np.array_equal(lo[s], olo)
+
+
+@pytest.mark.parametrize("n", [(1 << 20) + 1, (1 << 22) + 1])
+def test_membership_of_large_layouts(oracle, n):
+    """Just above the sizes at which the ranges above blocks grow."""
+    rng = np.random.default_rng(n)
+    pts = rng.normal(0, 100.0, (n, 2))
+    pts[: n // 3] *= 1e-3
+    mass = np.ones(n)
+    od, ohi, olo, _ = oracle.quadtree_leaves(pts, mass, 1)
+    lay = point_layout(pts, mass, 1)
+    d, hi, lo, _ = lay.tree_leaves()
+    lay.close()
+    assert np.array_equal(d, od)
+    assert np.array_equal(hi, ohi) and np.array_equal(lo, olo)
