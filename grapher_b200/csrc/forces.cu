@@ -2038,7 +2038,7 @@ void forces_set_smem_limits() {
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellDyn);
 }
 
-// The hub targets' plain walk, after the learned walk, on a grid that fills
+// The hub targets' plain walk, after or beside the learned walk, on a grid that fills
 // the GPU; then their epilogues.
 template <int MODEL, bool OVERLAP>
 static void launch_far_hubs(gvizCudaForce *h, const FarHubArgs &ha) {

@@ -1,6 +1,6 @@
 // noalloc.cu -- an allocation-free variant of the ForceAtlas2 global speed
-// update (the swing/traction reduction of precise.cu's k_fa2_chunks and the
-// speed rule of k_fa2_speed), for callers that must not allocate device
+// update (the swing/traction reduction and the speed rule of precise.cu's
+// k_fa2_speed), for callers that must not allocate device
 // memory while they run.
 //
 // Who needs it: a render loop that calls the layout once per frame and is not

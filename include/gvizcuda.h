@@ -109,7 +109,7 @@ typedef struct gvizCudaForceParams {
                                heaviest vertices (model mass, ties to the
                                lower id; at most vertexCount) comes from the
                                plain monopole walk at farHubTheta instead, one
-                               warp per vertex after the learned walk; 0
+                               warp per vertex beside or after the learned walk; 0
                                (default): none. LinLog's force on a vertex
                                scales with its mass, so these carry most of
                                the force-weighted error */
@@ -490,10 +490,11 @@ int gvizCudaForceFarJudgeStatus(const gvizCudaForce *h, uint64_t *checks, double
 
 /* The FP32 Barnes-Hut walks (plain and learned cell-group) expand the tree
  * 32 nodes at a time through a per-warp stack of pending nodes in shared
- * memory (512 entries); an opened cell whose children do not fit is walked
- * in place with the stackless preorder walk instead (the same decisions).
- * Sets the stack entries the walks may use, 32 to 512 (0 restores the
- * default: the autotuner's pick for the plain walk, else the above);
+ * memory (256 entries in the plain walk, 512 in the learned one); an opened
+ * cell whose children do not fit is walked in place with the stackless
+ * preorder walk instead (the same decisions). Sets the stack entries the
+ * walks may use, 32 to 512 (0 restores the default: the autotuner's pick for
+ * the plain walk, else the above);
  * forces agree up to the order of the per-target sums. A tuning and test
  * knob. No reference counterpart. */
 int gvizCudaForceSetWalkStackCap(gvizCudaForce *h, uint32_t entries);
