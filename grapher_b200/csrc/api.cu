@@ -55,6 +55,21 @@ void dfree(T *&p) {
   p = nullptr;
 }
 
+// Copies to the device in the order of h->stream, and waits for them. That
+// stream does not wait for the legacy stream, whose copies from pageable
+// memory and whose memsets may still be on their way when they return: a
+// kernel could read an index array before it is there.
+bool put(gvizCudaForce *h, void *dst, const void *src, size_t bytes) {
+  return !bytes ||
+         cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream) == cudaSuccess;
+}
+
+bool put_zero(gvizCudaForce *h, void *dst, size_t bytes) {
+  return cudaMemsetAsync(dst, 0, bytes, h->stream) == cudaSuccess;
+}
+
+bool put_done(gvizCudaForce *h) { return cudaStreamSynchronize(h->stream) == cudaSuccess; }
+
 bool g_dirUploaded[64] = {false};
 
 int upload_dir_table(gvizCudaForce *h) {
@@ -65,7 +80,8 @@ int upload_dir_table(gvizCudaForce *h) {
     t[2 * k] = cos(a);
     t[2 * k + 1] = sin(a);
   }
-  if (dir_table_upload_forces(t) || dir_table_upload_precise(t))
+  if (dir_table_upload_forces(t, h->stream) || dir_table_upload_precise(t, h->stream) ||
+      !put_done(h))
     return set_err(h, GVIZ_CUDA_ERR_CUDA);
   if (h->device < 64) g_dirUploaded[h->device] = true;
   return GVIZ_CUDA_OK;
@@ -183,8 +199,8 @@ int upload_radius(gvizCudaForce *h) {
       rf[i] = (float)r[i];
     }
   }
-  if (V && (cudaMemcpy(h->d_radius, r.data(), V * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(h->d_radiusF, rf.data(), V * 4, cudaMemcpyHostToDevice) != cudaSuccess))
+  if (!put(h, h->d_radius, r.data(), V * 8) || !put(h, h->d_radiusF, rf.data(), V * 4) ||
+      !put_done(h))
     return set_err(h, GVIZ_CUDA_ERR_CUDA);
   return GVIZ_CUDA_OK;
 }
@@ -336,15 +352,13 @@ int sync_and_check(gvizCudaForce *h) {
   return set_err(h, status_to_code(st));
 }
 
-void set_all_active(gvizCudaForce *h, uint64_t runLeft, double eps) {
+bool set_all_active(gvizCudaForce *h, uint64_t runLeft, double eps) {
   std::vector<uint32_t> one(h->G, 1u);
   std::vector<uint64_t> left(h->G, runLeft);
   std::vector<double> e(h->G, eps);
   uint32_t any = (uint32_t)h->G;
-  cudaMemcpy(h->d_active, one.data(), h->G * 4, cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_runLeft, left.data(), h->G * 8, cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_runEps, e.data(), h->G * 8, cudaMemcpyHostToDevice);
-  cudaMemcpy(h->d_anyActive, &any, 4, cudaMemcpyHostToDevice);
+  return put(h, h->d_active, one.data(), h->G * 4) && put(h, h->d_runLeft, left.data(), h->G * 8) &&
+         put(h, h->d_runEps, e.data(), h->G * 8) && put(h, h->d_anyActive, &any, 4) && put_done(h);
 }
 
 struct DeviceGuard {
@@ -446,7 +460,7 @@ static int far_judge(gvizCudaForce *h) {
     if (!h->d_judgeRep) rc |= dalloc(h, &h->d_judgeRep, h->V);
     if (rc) return set_err(h, GVIZ_CUDA_ERR_ALLOC);
     const std::vector<uint32_t> idx = judge_sample(h->V, n, h->judgeSeed);
-    if (cudaMemcpy(h->d_judgeIdx, idx.data(), n * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (!put(h, h->d_judgeIdx, idx.data(), n * 4) || !put_done(h))
       return set_err(h, GVIZ_CUDA_ERR_CUDA);
     h->judgeN = n;
   }
@@ -730,7 +744,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
       h->d_topCount = reinterpret_cast<uint32_t *>(zero + atTop);
       h->d_scanState = reinterpret_cast<uint64_t *>(zero + atScan);
       h->d_sortState = reinterpret_cast<uint32_t *>(zero + atSort);
-      if (cudaMemset(zero, 0, bytes) != cudaSuccess) rc |= GVIZ_CUDA_ERR_CUDA;
+      if (!put_zero(h, zero, bytes)) rc |= GVIZ_CUDA_ERR_CUDA;
     }
   }
   rc |= dalloc(h, &h->d_roots, G);
@@ -793,7 +807,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   }
   bool ok = true;
   auto up = [&](void *dst, const void *src, size_t bytes) {
-    if (bytes && cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) ok = false;
+    ok = ok && put(h, dst, src, bytes);
   };
   up(h->d_rowOff, row.data(), (V + 1) * 4);
   if (h->E2) up(h->d_cols, g->neighbors, h->E2 * 4);
@@ -816,11 +830,9 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   up(h->d_hubChunkV, hcV.data(), hcV.size() * 4);
   up(h->d_hubChunkE0, hcE0.data(), hcE0.size() * 4);
   up(h->d_hubChunkE1, hcE1.data(), hcE1.size() * 4);
-  ok = ok && cudaMemset(h->d_nCounter, 0, Vs * 4) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_graphBase, 0, G * 4) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_chunksDone, 0, G * 4) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_pos, 0, Vs * 16) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_counters, 0, 64) == cudaSuccess;
+  ok = ok && put_zero(h, h->d_nCounter, Vs * 4) && put_zero(h, h->d_graphBase, G * 4) &&
+       put_zero(h, h->d_chunksDone, G * 4) && put_zero(h, h->d_pos, Vs * 16) &&
+       put_zero(h, h->d_counters, 64) && put_done(h);
   if (!ok || upload_dir_table(h) || upload_radius(h)) {
     gvizCudaForceDestroy(h);
     return GVIZ_CUDA_ERR_CUDA;
@@ -831,16 +843,13 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   for (int i = 0; i < 65; i++) cudaEventCreate(&h->profEv[i]);
   // Init leaves the FA2 state zeroed (src/embedders/gvizForceEmbedder.c:221);
   // Begin sets it up.
-  ok = cudaMemset(h->d_speed, 0, G * 8) == cudaSuccess &&
-       cudaMemset(h->d_eff, 0, G * 8) == cudaSuccess &&
-       cudaMemset(h->d_sf, 0, Vs * 16) == cudaSuccess &&
-       cudaMemset(h->d_iter, 0, G * 8) == cudaSuccess &&
-       cudaMemset(h->d_lastStats, 0, G * 40) == cudaSuccess;
+  ok = put_zero(h, h->d_speed, G * 8) && put_zero(h, h->d_eff, G * 8) &&
+       put_zero(h, h->d_sf, Vs * 16) && put_zero(h, h->d_iter, G * 8) &&
+       put_zero(h, h->d_lastStats, G * 40) && set_all_active(h, ~0ull, -INFINITY);
   if (!ok) {
     gvizCudaForceDestroy(h);
     return GVIZ_CUDA_ERR_CUDA;
   }
-  set_all_active(h, ~0ull, -INFINITY);
   *out = h;
   return GVIZ_CUDA_OK;
 }
@@ -906,8 +915,7 @@ static int select_hubs(gvizCudaForce *h, uint32_t count) {
     h->d_farHubs = nullptr;
     return GVIZ_CUDA_ERR_ALLOC;
   }
-  if (cudaMemcpy(h->d_farHubs, ids.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice) !=
-      cudaSuccess)
+  if (!put(h, h->d_farHubs, ids.data(), count * sizeof(uint32_t)) || !put_done(h))
     return GVIZ_CUDA_ERR_CUDA;
   h->nFarHubs = count;
   return GVIZ_CUDA_OK;
@@ -979,14 +987,13 @@ int gvizCudaForceBegin(gvizCudaForce *h) {
   if (!h) return GVIZ_CUDA_ERR_ARG;
   DeviceGuard guard(h->device);
   std::vector<double> one(h->G, 1.0);
-  bool ok = cudaMemcpy(h->d_speed, one.data(), h->G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-  ok = ok && cudaMemcpy(h->d_eff, one.data(), h->G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_sf, 0, (h->V ? h->V : 1) * 16) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_disp, 0, (h->V ? h->V : 1) * 16) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_iter, 0, h->G * 8) == cudaSuccess;
-  ok = ok && cudaMemset(h->d_lastStats, 0, h->G * 40) == cudaSuccess;
+  const bool ok = put(h, h->d_speed, one.data(), h->G * 8) &&
+                  put(h, h->d_eff, one.data(), h->G * 8) &&
+                  put_zero(h, h->d_sf, (h->V ? h->V : 1) * 16) &&
+                  put_zero(h, h->d_disp, (h->V ? h->V : 1) * 16) &&
+                  put_zero(h, h->d_iter, h->G * 8) && put_zero(h, h->d_lastStats, h->G * 40) &&
+                  set_all_active(h, ~0ull, -INFINITY);
   if (!ok) return set_err(h, GVIZ_CUDA_ERR_CUDA);
-  set_all_active(h, ~0ull, -INFINITY);
   h->begun = true;
   h->hostIteration = 0;
   return GVIZ_CUDA_OK;
@@ -996,10 +1003,10 @@ int gvizCudaForceSetFa2State(gvizCudaForce *h, const double *sf,
                              const double *speed, const double *eff) {
   if (!h) return GVIZ_CUDA_ERR_ARG;
   DeviceGuard guard(h->device);
-  bool ok = true;
-  if (sf && h->V) ok = cudaMemcpy(h->d_sf, sf, h->V * 16, cudaMemcpyHostToDevice) == cudaSuccess;
-  if (speed) ok = ok && cudaMemcpy(h->d_speed, speed, h->G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-  if (eff) ok = ok && cudaMemcpy(h->d_eff, eff, h->G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
+  bool ok = !sf || put(h, h->d_sf, sf, h->V * 16);
+  if (speed) ok = ok && put(h, h->d_speed, speed, h->G * 8);
+  if (eff) ok = ok && put(h, h->d_eff, eff, h->G * 8);
+  ok = put_done(h) && ok;
   return ok ? GVIZ_CUDA_OK : set_err(h, GVIZ_CUDA_ERR_CUDA);
 }
 
@@ -1148,9 +1155,10 @@ int gvizCudaForceRun(gvizCudaForce *h, size_t maxIters, double epsilon,
   if (!h->begun) return set_err(h, GVIZ_CUDA_ERR_NOT_BEGUN);
   DeviceGuard guard(h->device);
   std::vector<uint64_t> it0(h->G), it1(h->G);
+  if (!put_done(h)) return set_err(h, GVIZ_CUDA_ERR_CUDA);  // steps enqueued before are not this run's
   cudaMemcpy(it0.data(), h->d_iter, h->G * 8, cudaMemcpyDeviceToHost);
   if (maxIters > 0 && h->V > 0) {
-    set_all_active(h, maxIters, epsilon);
+    if (!set_all_active(h, maxIters, epsilon)) return set_err(h, GVIZ_CUDA_ERR_CUDA);
     size_t launched = 0;
     while (launched < maxIters) {
       uint32_t n = (uint32_t)std::min<size_t>(kRunBatch, maxIters - launched);
@@ -1164,7 +1172,7 @@ int gvizCudaForceRun(gvizCudaForce *h, size_t maxIters, double epsilon,
       if (sc) return sc;
       if (any == 0) break;
     }
-    set_all_active(h, ~0ull, -INFINITY);
+    if (!set_all_active(h, ~0ull, -INFINITY)) return set_err(h, GVIZ_CUDA_ERR_CUDA);
   }
   cudaMemcpy(it1.data(), h->d_iter, h->G * 8, cudaMemcpyDeviceToHost);
   if (rounds)
@@ -1344,9 +1352,13 @@ int gvizCudaForceExactRepulsion(gvizCudaForce *h, const uint32_t *targets,
   }
   double2 *dout = h->d_exactRoom, *part = dout + n;
   uint32_t *dt = reinterpret_cast<uint32_t *>(part + parts);
-  cudaMemcpy(dt, targets, n * 4, cudaMemcpyHostToDevice);
-  enqueue_exact_judge(h, dt, n, dout, part);
-  int rc = sync_and_check(h);
+  int rc = GVIZ_CUDA_OK;
+  if (put(h, dt, targets, n * 4)) {
+    enqueue_exact_judge(h, dt, n, dout, part);
+    rc = sync_and_check(h);
+  } else {
+    rc = set_err(h, GVIZ_CUDA_ERR_CUDA);  // no kernel reads ids that are not there
+  }
   if (!rc && cudaMemcpy(out, dout, n * 16, cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = set_err(h, GVIZ_CUDA_ERR_CUDA);
   if (h->exactRoom * sizeof(double2) > kExactKept) {
@@ -1683,20 +1695,14 @@ int gvizCudaForceLoadCheckpoint(gvizCudaForce *h, const char *filename, int rest
   }
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return set_err(h, GVIZ_CUDA_ERR_CUDA);
   bool cok = true;
-  if (V) {
-    cok = cudaMemcpy(h->d_pos, pos.data(), V * 16, cudaMemcpyHostToDevice) == cudaSuccess;
-    cok = cok && cudaMemcpy(h->d_sf, sf.data(), V * 16, cudaMemcpyHostToDevice) == cudaSuccess;
-    cok = cok && cudaMemset(h->d_disp, 0, V * 16) == cudaSuccess;
-  }
-  cok = cok && cudaMemcpy(h->d_speed, speed.data(), G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-  cok = cok && cudaMemcpy(h->d_eff, eff.data(), G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-  cok = cok && cudaMemcpy(h->d_iter, iter.data(), G * 8, cudaMemcpyHostToDevice) == cudaSuccess;
-  cok = cok && cudaMemcpy(h->d_lastStats, last.data(), G * 40, cudaMemcpyHostToDevice) == cudaSuccess;
-  if (rows)
-    cok = cok && cudaMemcpy(h->d_stats, ring.data(), ring.size() * 8, cudaMemcpyHostToDevice) ==
-                     cudaSuccess;
+  if (V)
+    cok = put(h, h->d_pos, pos.data(), V * 16) && put(h, h->d_sf, sf.data(), V * 16) &&
+          put_zero(h, h->d_disp, V * 16);
+  cok = cok && put(h, h->d_speed, speed.data(), G * 8) && put(h, h->d_eff, eff.data(), G * 8) &&
+        put(h, h->d_iter, iter.data(), G * 8) && put(h, h->d_lastStats, last.data(), G * 40);
+  if (rows) cok = cok && put(h, h->d_stats, ring.data(), ring.size() * 8);
+  cok = put_done(h) && cok && set_all_active(h, ~0ull, -INFINITY);
   if (!cok) return set_err(h, GVIZ_CUDA_ERR_CUDA);
-  set_all_active(h, ~0ull, -INFINITY);
   h->begun = hd.begun != 0;
   h->hostIteration = hostIt;
   if (nameOut && nameCap) {
