@@ -138,8 +138,9 @@ __device__ __forceinline__ GraphRoot graph_root(const unsigned long long *box) {
 // Sixteen levels (or n < 16) of the descent from centre (cx, cy) and half
 // size h: the digits of 16 levels, the first in the top bits. The sign of
 // p - c, which is exact, gives the side: QuadrantFor's p >= c is its clear
-// sign bit; c moves by h / 2 with that sign. Halving subtracts one from h's
-// exponent (h > 1e-9 here).
+// sign bit unless p is -0.0 (-0.0 - 0.0 is -0.0), which p must not be; c moves
+// by h / 2 with that sign. Halving subtracts one from h's exponent (h > 1e-9
+// here).
 __device__ __forceinline__ uint32_t path_digits(double2 p, double &cx, double &cy, double &h,
                                                 int n) {
   uint32_t w = 0;
@@ -171,6 +172,8 @@ __device__ __forceinline__ uint32_t path_digits(double2 p, double &cx, double &c
 template <bool FULL>
 __device__ __forceinline__ uint64_t quadrant_path(double2 p, const GraphRoot &R, uint64_t &lo) {
   double cx = R.cx, cy = R.cy, h = R.h0;
+  p.x = __dadd_rn(p.x, 0.0);  // -0.0 becomes 0.0, nothing else changes
+  p.y = __dadd_rn(p.y, 0.0);
   const uint32_t w0 = path_digits(p, cx, cy, h, R.D);
   const uint32_t w1 = path_digits(p, cx, cy, h, R.D - 16);
   if (FULL) {
