@@ -139,6 +139,7 @@ void free_all(gvizCudaForce *h) {
   dfree(h->d_lastStats);
   dfree(h->d_chunkStat);
   dfree(h->d_chunksDone);
+  dfree(h->d_emptyGraphs);
   dfree(h->d_zero);
   dfree(h->d_roots);
   dfree(h->d_ck);
@@ -621,7 +622,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
     uint64_t n = goff[gg + 1] - goff[gg];
     mdp[gg] = n ? s / (double)n : 0.0;
   }
-  std::vector<uint32_t> cb, ce, cg, gcb(G), gce(G);
+  std::vector<uint32_t> cb, ce, cg, gcb(G), gce(G), empty;
   for (size_t gg = 0; gg < G; gg++) {
     gcb[gg] = (uint32_t)cb.size();
     for (uint64_t s = goff[gg]; s < goff[gg + 1]; s += GVIZ_CHUNK) {
@@ -630,8 +631,10 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
       cg.push_back((uint32_t)gg);
     }
     gce[gg] = (uint32_t)cb.size();
+    if (goff[gg] == goff[gg + 1]) empty.push_back((uint32_t)gg);
   }
   h->nChunks = (uint32_t)cb.size();
+  h->nEmptyGraphs = (uint32_t)empty.size();
   std::vector<uint32_t> light, heavy, hubV, hubFirst, hcV, hcE0, hcE1;
   for (size_t v = 0; v < V; v++) {
     const uint64_t d = row[v + 1] - row[v];
@@ -722,6 +725,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   rc |= dalloc(h, &h->d_lastStats, G * 5);
   rc |= dalloc(h, &h->d_chunkStat, C);
   rc |= dalloc(h, &h->d_chunksDone, G);
+  if (!empty.empty()) rc |= dalloc(h, &h->d_emptyGraphs, empty.size());
   {
     size_t bytes = 0;
     auto part = [&bytes](size_t count, size_t size) {
@@ -821,6 +825,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   up(h->d_chunkBegin, cb.data(), cb.size() * 4);
   up(h->d_chunkEnd, ce.data(), ce.size() * 4);
   up(h->d_chunkGraph, cg.data(), cg.size() * 4);
+  up(h->d_emptyGraphs, empty.data(), empty.size() * 4);
   up(h->d_gChunkBegin, gcb.data(), G * 4);
   up(h->d_gChunkEnd, gce.data(), G * 4);
   up(h->d_attrLight, light.data(), light.size() * 4);

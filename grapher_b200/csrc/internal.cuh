@@ -106,6 +106,7 @@ struct gvizCudaForce {
   double *h_meanDegPlusOne = nullptr;
   double *h_tail = nullptr;  // pinned: d_lastStats, then the status (finish_step)
   uint32_t nChunks = 0;
+  uint32_t nEmptyGraphs = 0;  // graphs without vertices (no chunk)
 
   // --- structure (device) ---
   uint32_t *d_rowOff = nullptr;  // V+1 (adjacency fits 32 bits)
@@ -160,6 +161,7 @@ struct gvizCudaForce {
   uint32_t walkTunedCap = 0;  // plain walk: the autotuner's stack entries (0: not tuned)
   ChunkStat *d_chunkStat = nullptr;
   uint32_t *d_chunksDone = nullptr;  // per graph: chunks that finished a sum
+  uint32_t *d_emptyGraphs = nullptr;  // the graphs without vertices
   uint32_t *d_status = nullptr;
 
   // --- tree build scratch (device) ---

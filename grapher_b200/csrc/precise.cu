@@ -813,6 +813,16 @@ __global__ __launch_bounds__(kThreads) void k_fa2_stats_strict(Fa2Args a) {
   if (a.active[blockIdx.x]) fa2_stats(a, blockIdx.x, sh);
 }
 
+// The step tail of the graphs without vertices, which have no chunk whose last
+// block would do it: their rounds count and stop like any other's. Launched
+// only where there are any.
+__global__ __launch_bounds__(kThreads) void k_fa2_stats_empty(Fa2Args a, const uint32_t *graphs) {
+  step_order();
+  __shared__ double sh[kThreads / 32];
+  const uint32_t g = graphs[blockIdx.x];
+  if (a.active[g]) fa2_stats(a, g, sh);
+}
+
 inline uint32_t blocks(size_t n, int t) { return (uint32_t)((n + t - 1) / t); }
 
 Fa2Args make_fa2(gvizCudaForce *h) {
@@ -997,6 +1007,9 @@ void enqueue_fa2(gvizCudaForce *h) {
   } else {
     launch_after(h->stream, k_fa2_speed, h->nChunks, kThreads, 0, a);
     launch_after(h->stream, k_fa2_apply, h->nChunks, kThreads, 0, a);
+    if (h->nEmptyGraphs)
+      launch_after(h->stream, k_fa2_stats_empty, h->nEmptyGraphs, kThreads, 0, a,
+                   h->d_emptyGraphs);
   }
   prof_mark(h, "fa2_update");
 }
