@@ -319,25 +319,38 @@ int status_to_code(uint32_t st) {
   return GVIZ_CUDA_OK;
 }
 
+// The pinned memory that finish_step reads into, made at the first step,
+// before anything of the step is enqueued.
+int tail_room(gvizCudaForce *h) {
+  if (h->h_tail) return GVIZ_CUDA_OK;
+  if (cudaMallocHost((void **)&h->h_tail, (h->G * 5 + 1) * sizeof(double)) == cudaSuccess)
+    return GVIZ_CUDA_OK;
+  h->h_tail = nullptr;
+  cudaGetLastError();
+  return set_err(h, GVIZ_CUDA_ERR_ALLOC);
+}
+
+// An error once a step's work or copies may be in flight: waits for them, so
+// that nothing writes the caller's buffer after the return.
+double step_error(gvizCudaForce *h, int rc) {
+  cudaStreamSynchronize(h->stream);
+  if (h->upload) cudaStreamSynchronize(h->upload);
+  return (double)set_err(h, rc);
+}
+
 // Waits for a step and reads its status and statistics: both come back with
-// the step's own work, into pinned memory (made at the first step), instead
-// of two blocking copies after it, which cost a 1,024-vertex step 17 of 168
-// us. Returns graph 0's maxDisp; rc receives the status.
+// the step's own work, into pinned memory (tail_room), instead of two blocking
+// copies after it, which cost a 1,024-vertex step 17 of 168 us. Returns graph
+// 0's maxDisp; rc receives the status.
 double finish_step(gvizCudaForce *h, gvizCudaStepStats *stats, int *rc) {
   const size_t row = h->G * 5 * sizeof(double);
-  if (!h->h_tail && cudaMallocHost((void **)&h->h_tail, row + sizeof(double)) != cudaSuccess) {
-    h->h_tail = nullptr;
-    cudaGetLastError();
-    *rc = set_err(h, GVIZ_CUDA_ERR_ALLOC);
-    return (double)*rc;
-  }
   uint32_t *status = reinterpret_cast<uint32_t *>(h->h_tail + h->G * 5);
   if (cudaMemcpyAsync(h->h_tail, h->d_lastStats, row, cudaMemcpyDeviceToHost, h->stream) !=
           cudaSuccess ||
       cudaMemcpyAsync(status, h->d_status, 4, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
       cudaStreamSynchronize(h->stream) != cudaSuccess) {
-    *rc = set_err(h, GVIZ_CUDA_ERR_CUDA);
-    return (double)*rc;
+    *rc = GVIZ_CUDA_ERR_CUDA;
+    return step_error(h, *rc);
   }
   *rc = set_err(h, status_to_code(*status));
   if (stats) memcpy(stats, h->h_tail, row);
@@ -1040,7 +1053,8 @@ double gvizCudaForceStep(gvizCudaForce *h, gvizCudaStepStats *stats) {
       }
     return 0.0;
   }
-  int rc = launch_steps(h, 1);
+  int rc = tail_room(h);
+  if (!rc) rc = launch_steps(h, 1);
   if (rc) return (double)rc;
   const double md = finish_step(h, stats, &rc);
   h->hostIteration++;
@@ -1053,12 +1067,13 @@ double gvizCudaForceStepHost(gvizCudaForce *h, double *xy,
   if (!h->begun) return (double)set_err(h, GVIZ_CUDA_ERR_NOT_BEGUN);
   DeviceGuard guard(h->device);
   if (h->V == 0) return gvizCudaForceStep(h, stats);
-  if (cudaMemcpyAsync(h->d_pos, xy, h->V * 16, cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
-    return (double)set_err(h, GVIZ_CUDA_ERR_CUDA);
-  int rc = launch_steps(h, 1);
+  int rc = tail_room(h);
   if (rc) return (double)rc;
+  if (!put(h, h->d_pos, xy, h->V * 16)) return step_error(h, GVIZ_CUDA_ERR_CUDA);
+  rc = launch_steps(h, 1);
+  if (rc) return step_error(h, rc);
   if (cudaMemcpyAsync(xy, h->d_pos, h->V * 16, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess)
-    return (double)set_err(h, GVIZ_CUDA_ERR_CUDA);
+    return step_error(h, GVIZ_CUDA_ERR_CUDA);
   const double md = finish_step(h, stats, &rc);
   h->hostIteration++;
   return rc ? (double)rc : md;
@@ -1092,8 +1107,9 @@ double gvizCudaForceRunHost(gvizCudaForce *h, double *xy, uint32_t steps,
   if (!h || (!xy && h->V)) return (double)GVIZ_CUDA_ERR_ARG;
   if (!h->begun) return (double)set_err(h, GVIZ_CUDA_ERR_NOT_BEGUN);
   DeviceGuard guard(h->device);
+  int rc = tail_room(h);
+  if (rc) return (double)rc;
   if (steps == 0) {
-    int rc = GVIZ_CUDA_OK;
     const double md = finish_step(h, stats, &rc);
     return rc ? (double)rc : md;
   }
@@ -1105,7 +1121,7 @@ double gvizCudaForceRunHost(gvizCudaForce *h, double *xy, uint32_t steps,
     }
     return md;
   }
-  int rc = host_pipeline(h);
+  rc = host_pipeline(h);
   if (rc) return (double)rc;
   const size_t doubles = 2 * h->V;
   const size_t piece = (doubles + GVIZ_HOST_PIECES - 1) / GVIZ_HOST_PIECES;
@@ -1114,7 +1130,7 @@ double gvizCudaForceRunHost(gvizCudaForce *h, double *xy, uint32_t steps,
   double *dpos = reinterpret_cast<double *>(h->d_pos);
   for (uint32_t k = 0; ok && k < steps; k++) {
     rc = launch_steps(h, 1);
-    if (rc) return (double)rc;
+    if (rc) return step_error(h, rc);
     const bool again = k + 1 < steps;
     for (int c = 0; ok && c < GVIZ_HOST_PIECES; c++) {
       const size_t off = (size_t)c * piece;
@@ -1133,7 +1149,7 @@ double gvizCudaForceRunHost(gvizCudaForce *h, double *xy, uint32_t steps,
       ok = cudaEventRecord(h->evUp, h->upload) == cudaSuccess &&
            cudaStreamWaitEvent(h->stream, h->evUp, 0) == cudaSuccess;
   }
-  if (!ok) return (double)set_err(h, GVIZ_CUDA_ERR_CUDA);
+  if (!ok) return step_error(h, GVIZ_CUDA_ERR_CUDA);
   const double md = finish_step(h, stats, &rc);
   h->hostIteration += steps;
   return rc ? (double)rc : md;

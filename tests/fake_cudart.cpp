@@ -21,6 +21,7 @@ namespace {
 
 bool legacyPending = false;
 int unordered = 0;
+int launches = 0;  // kernels and graphs
 std::map<cudaStream_t, int> backToHost;  // copies to the host not waited for
 std::map<std::string, int> failAfter;
 dim3 cfgGrid, cfgBlock;
@@ -53,13 +54,14 @@ cudaError_t handle(void **out) {
 extern "C" {
 
 int fake_unordered(void) { return unordered; }
+int fake_launches(void) { return launches; }
 int fake_back_to_host(void) {
   int n = 0;
   for (auto &k : backToHost) n += k.second;
   return n;
 }
 void fake_reset(void) {
-  unordered = 0;
+  unordered = launches = 0;
   legacyPending = false;
   backToHost.clear();
   failAfter.clear();
@@ -154,9 +156,11 @@ cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
 }
 
 cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t st) {
+  launches++;
   return work(st);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) {
+  launches++;
   return work(c->stream);
 }
 
@@ -174,6 +178,7 @@ cudaError_t cudaGraphDestroy(cudaGraph_t g) { return free(g), cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { return free(e), cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {
   if (fails("cudaGraphLaunch")) return cudaErrorUnknown;
+  launches++;
   return work(st);
 }
 

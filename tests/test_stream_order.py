@@ -114,3 +114,43 @@ def test_grip_uploads_are_ordered_before_the_work_that_reads_them(fake):
     g.positions()
     g.close()
     assert fake.fake_unordered() == 0
+
+
+STEPS = [lambda lay, xy: lay.step(), lambda lay, xy: lay.step_host(xy),
+         lambda lay, xy: lay.run_host(xy, 3)]
+
+
+@pytest.mark.parametrize("step", STEPS)
+def test_step_without_memory_for_its_result_does_nothing(fake, step):
+    from grapher_b200._native import GvizCudaError
+    lay = _layout()
+    xy = lay.positions()
+    fake.fake_reset()
+    fake.fake_fail_after(b"cudaMallocHost", 0)
+    with pytest.raises(GvizCudaError) as e:
+        step(lay, xy)
+    assert e.value.code == -1
+    assert fake.fake_launches() == 0 and fake.fake_back_to_host() == 0
+    fake.fake_reset()
+    step(lay, xy)  # the next one is in order
+    assert fake.fake_launches() > 0
+    lay.close()
+
+
+@pytest.mark.parametrize("step", STEPS)
+@pytest.mark.parametrize("call", [b"cudaMemcpyAsync", b"cudaMemcpyAsync to host",
+                                  b"cudaGraphLaunch"])
+@pytest.mark.parametrize("after", range(16))
+def test_failed_step_leaves_no_copy_in_flight(fake, step, call, after):
+    from grapher_b200._native import GvizCudaError
+    lay = _layout()
+    xy = lay.positions()
+    fake.fake_reset()
+    fake.fake_fail_after(call, after)
+    try:
+        step(lay, xy)
+    except GvizCudaError:
+        pass
+    assert fake.fake_back_to_host() == 0
+    fake.fake_reset()
+    lay.close()
