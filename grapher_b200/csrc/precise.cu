@@ -525,15 +525,24 @@ __global__ __launch_bounds__(kJudgeThreads, kJudgeBlocksPerSM) void k_judge_f64(
           } else {
             const double dx = u.x - p.x, dy = u.y - p.y;
             const double d2 = __fma_rn(dx, dx, dy * dy);
-            if (d2 > 0.0) {
+            if ((uint32_t)__double2hiint(d2) - kJudgeLow < kJudgeSpan) {
               const double s = -sm[q] / d2;
               bx = __fma_rn(s, dx, bx);
               by = __fma_rn(s, dy, by);
             } else {
+              // coincident, or so close or far that the quotient by the square
+              // leaves the range: the terms of rep_term64
+              const double dist = sqrt(dx * dx + dy * dy);
+              const double mag = dist > 0.0 ? sm[q] / dist : sm[q] * a.overlapC;
               double ux, uy;
-              coincident_dir(v, jj, ux, uy);
-              bx -= sm[q] * a.overlapC * ux;
-              by -= sm[q] * a.overlapC * uy;
+              if (dist > 0.0) {
+                ux = dx / dist;
+                uy = dy / dist;
+              } else {
+                coincident_dir(v, jj, ux, uy);
+              }
+              bx -= mag * ux;
+              by -= mag * uy;
             }
           }
         }
