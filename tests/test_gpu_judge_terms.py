@@ -38,6 +38,34 @@ def _relative(got, want):
     return abs(Fraction(got) / want - 1)
 
 
+@pytest.mark.parametrize("model", [0, 1])
+def test_reciprocal_over_its_range(model):
+    """Random mantissas at distances from 2^-449 to 2^440 (squares 2^-898 to
+    2^880), the others at 2^60 times the distance."""
+    rng = np.random.default_rng(4 + model)
+    worst = Fraction(0)
+    for e in list(range(-449, 440, 13)) + [-449, -2, -1, 0, 1, 2, 440]:
+        for m in rng.uniform(1.0, 2.0, 2):
+            dx = float(np.ldexp(m, e))
+            got = _term(dx, float(np.ldexp(1.0, e + 66)), model)
+            want = Fraction(-100 if model == 0 else -1) / Fraction(dx)
+            worst = max(worst, _relative(got[0], want))
+            assert got[1] == 0.0
+    assert worst <= Fraction(1, 2 ** 51) * (2 if model == 0 else 1)  # FR: the product with k^2
+
+
+def test_largest_distances():
+    """Every source near the upper end: 95 comparable terms. 2^-51 of each, and
+    at most 96 additions of half an ulp of the sum: 2^-51 + 96 * 2^-53."""
+    for e in (500, 509, 510):
+        far = float(np.ldexp(1.0, e))
+        got = _term(far * 0.75, far)
+        dist = [far * (1.0 + j / 1024.0) for j in range(1, N)]
+        dist[39] = far * 0.75
+        want = -sum(Fraction(1) / Fraction(d) for d in dist)
+        assert _relative(got[0], want) <= Fraction(1, 2 ** 51) + Fraction(96, 2 ** 53)
+
+
 @pytest.mark.parametrize("scale", [1.0, 2.0 ** -448, 2.0 ** -452, 2.0 ** -505, 2.0 ** -511])
 def test_terms_below_the_range(scale):
     """distances whose squares are normal numbers, on both sides of 2^-900"""
