@@ -359,7 +359,10 @@ __global__ __launch_bounds__(512) void k_sort_runs(
 
 // Buckets, the runs of identical full paths, numbered by a single-pass scan
 // (sort.cu): a warp takes 256 consecutive sorted points in rounds of 32, the
-// ballot of bucket starts gives each its number in the warp.
+// ballot of bucket starts gives each its number in the warp. Where k_sort_runs
+// left a run too long for it unsorted (GVIZ_ST_DEEP_RUN, an error of the
+// call), there are no buckets and so no tree: the kernels that follow need
+// sorted keys, without them a node's children may lie outside its range.
 __global__ __launch_bounds__(kThreads) void k_buckets(
     const uint64_t *__restrict__ sHi, const uint64_t *__restrict__ sLo,
     const uint64_t *__restrict__ ck, uint32_t *bStart, uint64_t *bHi, uint64_t *bLo,
@@ -368,8 +371,10 @@ __global__ __launch_bounds__(kThreads) void k_buckets(
   step_order();
   constexpr int kRounds = GVIZ_SCAN_TILE / kThreads;
   __shared__ uint32_t sTile;
+  const uint32_t unsorted = *status & GVIZ_ST_DEEP_RUN;
   if (threadIdx.x == 0) sTile = scan_ticket(state);
   __syncthreads();
+  if (unsorted) return;
   const uint32_t tile = sTile;
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   const uint32_t s0 = tile * GVIZ_SCAN_TILE + w * (32u * kRounds) + lane;
@@ -1644,6 +1649,7 @@ __global__ __launch_bounds__(kThreads) void k_group_members(const NodeF *nodes,
 // Inspection: per point, the depth of the reference leaf holding it.
 __global__ __launch_bounds__(kThreads) void k_leaf_depth(EM a, int32_t *depthOut) {
   const uint32_t U = a.counts[2];
+  if (U == 0) return;  // no tree
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t nInt = U - 1;
   if (t < nInt) {
@@ -1877,6 +1883,7 @@ __device__ void cell_out(const CellOut &o, uint32_t at, int d, uint32_t b,
 
 __global__ __launch_bounds__(kThreads) void k_cell_dump(EM a, CellOut o) {
   const uint32_t U = a.counts[2];
+  if (U == 0) return;  // no tree
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t nInt = U - 1;
   if (t < nInt) {
