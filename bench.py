@@ -2,7 +2,11 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--workload ba1m_learned|rmat4m_learned|ba1m|batch4096|grid32|er65k_exact
-                                |grip_ba200k]
+                                |grip_ba200k] [--details FILE]
+
+Prints one JSON line of less than 3,000 characters; --details writes the whole
+result to FILE, with the error tables over theta and the explanations that the
+line leaves out.
 
 Default workload (the headline metric: learned vs plain Barnes-Hut at equal
 force error): Barabasi-Albert graph, n = 1,048,576, m = 4 (4,194,294 edges,
@@ -424,7 +428,7 @@ def run_reference_arm(args, w):
     else:
         base = cpu_baseline(w)
         v = base["value"]
-        line.update(steps=1, warmup=0)
+        line.update(steps=1, warmup=0, ms_per_step=1e3 / v)
     line.update(value=v, cpu_baseline=base,
                 e2e={"value": v, "unit": "iters/s", "h2d_bytes_per_step": 0,
                      "d2h_bytes_per_step": 0})
@@ -446,6 +450,33 @@ class nvtx_range:
     def __exit__(self, *exc):
         import torch
         torch.cuda.nvtx.range_pop()
+
+
+LONG_KEYS = {"learned_errors", "plain_errors", "learned_errors_by_hub_targets", "timer",
+             "algorithmic", "traffic_source", "peak_source", "train_loss_first_last",
+             "walk_shape"}
+
+
+def brief(x, top=True):
+    """The printed form of a result line: without the error tables over theta
+    and the explanations (--details FILE has them), floats below the top level
+    to six digits. The line stays below 3,000 characters; with the tables it
+    had 20,000, more than a reader of a run's output keeps."""
+    if isinstance(x, dict):
+        return {k: (v if top and not isinstance(v, (dict, list)) else brief(v, False))
+                for k, v in x.items() if k not in LONG_KEYS}
+    if isinstance(x, list):
+        return [brief(v, False) for v in x]
+    if isinstance(x, float) and math.isfinite(x):
+        return float(f"{x:.6g}")
+    return x
+
+
+def print_line(line, args):
+    if args.details:
+        with open(args.details, "w") as f:
+            json.dump(line, f)
+    print(json.dumps(brief(line)))
 
 
 def reduce_max(x, dist=None, device="cpu"):
@@ -904,7 +935,7 @@ def grip_bench(args):
                                           f"own pipeline on the same graph, gvizThreadPool over "
                                           f"{cores} threads"}
     g.close()
-    print(json.dumps(line))
+    print_line(line, args)
     return 0
 
 
@@ -921,6 +952,8 @@ def main():
                     help="learned workloads: hub targets of the learned walk; 'auto' (default) "
                          "times 0, V/1024 and V/256 at their own largest qualifying theta and "
                          "keeps the fastest, a number fixes the count")
+    ap.add_argument("--details", metavar="FILE",
+                    help="write the whole result, error tables over theta included, to FILE")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     if args.workload == "grip_ba200k":
@@ -1089,7 +1122,7 @@ def main():
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(w)
     if rank == 0:
-        print(json.dumps(line))
+        print_line(line, args)
     lay.close()
     if dist:
         dist.destroy_process_group()
