@@ -55,20 +55,22 @@ void dfree(T *&p) {
   p = nullptr;
 }
 
-// Copies to the device in the order of h->stream, and waits for them. That
-// stream does not wait for the legacy stream, whose copies from pageable
-// memory and whose memsets may still be on their way when they return: a
-// kernel could read an index array before it is there.
-bool put(gvizCudaForce *h, void *dst, const void *src, size_t bytes) {
-  return !bytes ||
-         cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream) == cudaSuccess;
+// Copies to the device on the legacy stream, and the wait for them (put_done)
+// before h->stream may read them: that stream does not wait for the legacy
+// one, whose copies from pageable memory and whose memsets may still be on
+// their way when they return, so a kernel could read an index array before it
+// is there. Work in flight on h->stream that reads what they replace is waited
+// for first (idle). (The same copies on h->stream itself cost every later step
+// of a process's third handle and on: 5,000 vertices 148 -> 153 us.)
+bool put(void *dst, const void *src, size_t bytes) {
+  return !bytes || cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
 }
 
-bool put_zero(gvizCudaForce *h, void *dst, size_t bytes) {
-  return cudaMemsetAsync(dst, 0, bytes, h->stream) == cudaSuccess;
-}
+bool put_zero(void *dst, size_t bytes) { return cudaMemset(dst, 0, bytes) == cudaSuccess; }
 
-bool put_done(gvizCudaForce *h) { return cudaStreamSynchronize(h->stream) == cudaSuccess; }
+bool put_done() { return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess; }
+
+bool idle(gvizCudaForce *h) { return cudaStreamSynchronize(h->stream) == cudaSuccess; }
 
 bool g_dirUploaded[64] = {false};
 
@@ -80,8 +82,7 @@ int upload_dir_table(gvizCudaForce *h) {
     t[2 * k] = cos(a);
     t[2 * k + 1] = sin(a);
   }
-  if (dir_table_upload_forces(t, h->stream) || dir_table_upload_precise(t, h->stream) ||
-      !put_done(h))
+  if (dir_table_upload_forces(t) || dir_table_upload_precise(t) || !put_done())
     return set_err(h, GVIZ_CUDA_ERR_CUDA);
   if (h->device < 64) g_dirUploaded[h->device] = true;
   return GVIZ_CUDA_OK;
@@ -200,8 +201,8 @@ int upload_radius(gvizCudaForce *h) {
       rf[i] = (float)r[i];
     }
   }
-  if (!put(h, h->d_radius, r.data(), V * 8) || !put(h, h->d_radiusF, rf.data(), V * 4) ||
-      !put_done(h))
+  if (!idle(h) || !put(h->d_radius, r.data(), V * 8) || !put(h->d_radiusF, rf.data(), V * 4) ||
+      !put_done())
     return set_err(h, GVIZ_CUDA_ERR_CUDA);
   return GVIZ_CUDA_OK;
 }
@@ -366,13 +367,14 @@ int sync_and_check(gvizCudaForce *h) {
   return set_err(h, status_to_code(st));
 }
 
+// (the caller has waited for the steps, and waits for the copies after it)
 bool set_all_active(gvizCudaForce *h, uint64_t runLeft, double eps) {
   std::vector<uint32_t> one(h->G, 1u);
   std::vector<uint64_t> left(h->G, runLeft);
   std::vector<double> e(h->G, eps);
   uint32_t any = (uint32_t)h->G;
-  return put(h, h->d_active, one.data(), h->G * 4) && put(h, h->d_runLeft, left.data(), h->G * 8) &&
-         put(h, h->d_runEps, e.data(), h->G * 8) && put(h, h->d_anyActive, &any, 4) && put_done(h);
+  return put(h->d_active, one.data(), h->G * 4) && put(h->d_runLeft, left.data(), h->G * 8) &&
+         put(h->d_runEps, e.data(), h->G * 8) && put(h->d_anyActive, &any, 4);
 }
 
 struct DeviceGuard {
@@ -474,7 +476,7 @@ static int far_judge(gvizCudaForce *h) {
     if (!h->d_judgeRep) rc |= dalloc(h, &h->d_judgeRep, h->V);
     if (rc) return set_err(h, GVIZ_CUDA_ERR_ALLOC);
     const std::vector<uint32_t> idx = judge_sample(h->V, n, h->judgeSeed);
-    if (!put(h, h->d_judgeIdx, idx.data(), n * 4) || !put_done(h))
+    if (!put(h->d_judgeIdx, idx.data(), n * 4) || !put_done())
       return set_err(h, GVIZ_CUDA_ERR_CUDA);
     h->judgeN = n;
   }
@@ -761,7 +763,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
       h->d_topCount = reinterpret_cast<uint32_t *>(zero + atTop);
       h->d_scanState = reinterpret_cast<uint64_t *>(zero + atScan);
       h->d_sortState = reinterpret_cast<uint32_t *>(zero + atSort);
-      if (!put_zero(h, zero, bytes)) rc |= GVIZ_CUDA_ERR_CUDA;
+      if (!put_zero(zero, bytes)) rc |= GVIZ_CUDA_ERR_CUDA;
     }
   }
   rc |= dalloc(h, &h->d_roots, G);
@@ -824,7 +826,7 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   }
   bool ok = true;
   auto up = [&](void *dst, const void *src, size_t bytes) {
-    ok = ok && put(h, dst, src, bytes);
+    ok = ok && put(dst, src, bytes);
   };
   up(h->d_rowOff, row.data(), (V + 1) * 4);
   if (h->E2) up(h->d_cols, g->neighbors, h->E2 * 4);
@@ -848,9 +850,9 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   up(h->d_hubChunkV, hcV.data(), hcV.size() * 4);
   up(h->d_hubChunkE0, hcE0.data(), hcE0.size() * 4);
   up(h->d_hubChunkE1, hcE1.data(), hcE1.size() * 4);
-  ok = ok && put_zero(h, h->d_nCounter, Vs * 4) && put_zero(h, h->d_graphBase, G * 4) &&
-       put_zero(h, h->d_chunksDone, G * 4) && put_zero(h, h->d_pos, Vs * 16) &&
-       put_zero(h, h->d_counters, 64) && put_done(h);
+  ok = ok && put_zero(h->d_nCounter, Vs * 4) && put_zero(h->d_graphBase, G * 4) &&
+       put_zero(h->d_chunksDone, G * 4) && put_zero(h->d_pos, Vs * 16) &&
+       put_zero(h->d_counters, 64) && put_done();
   if (!ok || upload_dir_table(h) || upload_radius(h)) {
     gvizCudaForceDestroy(h);
     return GVIZ_CUDA_ERR_CUDA;
@@ -861,9 +863,9 @@ int gvizCudaForceCreate(gvizCudaForce **out, const gvizCudaGraphDesc *g) {
   for (int i = 0; i < 65; i++) cudaEventCreate(&h->profEv[i]);
   // Init leaves the FA2 state zeroed (src/embedders/gvizForceEmbedder.c:221);
   // Begin sets it up.
-  ok = put_zero(h, h->d_speed, G * 8) && put_zero(h, h->d_eff, G * 8) &&
-       put_zero(h, h->d_sf, Vs * 16) && put_zero(h, h->d_iter, G * 8) &&
-       put_zero(h, h->d_lastStats, G * 40) && set_all_active(h, ~0ull, -INFINITY);
+  ok = put_zero(h->d_speed, G * 8) && put_zero(h->d_eff, G * 8) &&
+       put_zero(h->d_sf, Vs * 16) && put_zero(h->d_iter, G * 8) &&
+       put_zero(h->d_lastStats, G * 40) && set_all_active(h, ~0ull, -INFINITY) && put_done();
   if (!ok) {
     gvizCudaForceDestroy(h);
     return GVIZ_CUDA_ERR_CUDA;
@@ -933,7 +935,7 @@ static int select_hubs(gvizCudaForce *h, uint32_t count) {
     h->d_farHubs = nullptr;
     return GVIZ_CUDA_ERR_ALLOC;
   }
-  if (!put(h, h->d_farHubs, ids.data(), count * sizeof(uint32_t)) || !put_done(h))
+  if (!put(h->d_farHubs, ids.data(), count * sizeof(uint32_t)) || !put_done())
     return GVIZ_CUDA_ERR_CUDA;
   h->nFarHubs = count;
   return GVIZ_CUDA_OK;
@@ -1005,12 +1007,12 @@ int gvizCudaForceBegin(gvizCudaForce *h) {
   if (!h) return GVIZ_CUDA_ERR_ARG;
   DeviceGuard guard(h->device);
   std::vector<double> one(h->G, 1.0);
-  const bool ok = put(h, h->d_speed, one.data(), h->G * 8) &&
-                  put(h, h->d_eff, one.data(), h->G * 8) &&
-                  put_zero(h, h->d_sf, (h->V ? h->V : 1) * 16) &&
-                  put_zero(h, h->d_disp, (h->V ? h->V : 1) * 16) &&
-                  put_zero(h, h->d_iter, h->G * 8) && put_zero(h, h->d_lastStats, h->G * 40) &&
-                  set_all_active(h, ~0ull, -INFINITY);
+  const bool ok = idle(h) && put(h->d_speed, one.data(), h->G * 8) &&
+                  put(h->d_eff, one.data(), h->G * 8) &&
+                  put_zero(h->d_sf, (h->V ? h->V : 1) * 16) &&
+                  put_zero(h->d_disp, (h->V ? h->V : 1) * 16) &&
+                  put_zero(h->d_iter, h->G * 8) && put_zero(h->d_lastStats, h->G * 40) &&
+                  set_all_active(h, ~0ull, -INFINITY) && put_done();
   if (!ok) return set_err(h, GVIZ_CUDA_ERR_CUDA);
   h->begun = true;
   h->hostIteration = 0;
@@ -1021,10 +1023,10 @@ int gvizCudaForceSetFa2State(gvizCudaForce *h, const double *sf,
                              const double *speed, const double *eff) {
   if (!h) return GVIZ_CUDA_ERR_ARG;
   DeviceGuard guard(h->device);
-  bool ok = !sf || put(h, h->d_sf, sf, h->V * 16);
-  if (speed) ok = ok && put(h, h->d_speed, speed, h->G * 8);
-  if (eff) ok = ok && put(h, h->d_eff, eff, h->G * 8);
-  ok = put_done(h) && ok;
+  bool ok = idle(h) && (!sf || put(h->d_sf, sf, h->V * 16));
+  if (speed) ok = ok && put(h->d_speed, speed, h->G * 8);
+  if (eff) ok = ok && put(h->d_eff, eff, h->G * 8);
+  ok = put_done() && ok;
   return ok ? GVIZ_CUDA_OK : set_err(h, GVIZ_CUDA_ERR_CUDA);
 }
 
@@ -1069,7 +1071,8 @@ double gvizCudaForceStepHost(gvizCudaForce *h, double *xy,
   if (h->V == 0) return gvizCudaForceStep(h, stats);
   int rc = tail_room(h);
   if (rc) return (double)rc;
-  if (!put(h, h->d_pos, xy, h->V * 16)) return step_error(h, GVIZ_CUDA_ERR_CUDA);
+  if (cudaMemcpyAsync(h->d_pos, xy, h->V * 16, cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
+    return step_error(h, GVIZ_CUDA_ERR_CUDA);
   rc = launch_steps(h, 1);
   if (rc) return step_error(h, rc);
   if (cudaMemcpyAsync(xy, h->d_pos, h->V * 16, cudaMemcpyDeviceToHost, h->stream) != cudaSuccess)
@@ -1176,10 +1179,13 @@ int gvizCudaForceRun(gvizCudaForce *h, size_t maxIters, double epsilon,
   if (!h->begun) return set_err(h, GVIZ_CUDA_ERR_NOT_BEGUN);
   DeviceGuard guard(h->device);
   std::vector<uint64_t> it0(h->G), it1(h->G);
-  if (!put_done(h)) return set_err(h, GVIZ_CUDA_ERR_CUDA);  // steps enqueued before are not this run's
-  cudaMemcpy(it0.data(), h->d_iter, h->G * 8, cudaMemcpyDeviceToHost);
-  if (maxIters > 0 && h->V > 0) {
-    if (!set_all_active(h, maxIters, epsilon)) return set_err(h, GVIZ_CUDA_ERR_CUDA);
+  const bool runs = maxIters > 0 && h->V > 0;
+  // steps enqueued before are not this run's; the counters' copy back waits
+  // for the uploads before it
+  if (!idle(h) || (runs && !set_all_active(h, maxIters, epsilon)) ||
+      cudaMemcpy(it0.data(), h->d_iter, h->G * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
+    return set_err(h, GVIZ_CUDA_ERR_CUDA);
+  if (runs) {
     size_t launched = 0;
     while (launched < maxIters) {
       uint32_t n = (uint32_t)std::min<size_t>(kRunBatch, maxIters - launched);
@@ -1195,7 +1201,8 @@ int gvizCudaForceRun(gvizCudaForce *h, size_t maxIters, double epsilon,
     }
     if (!set_all_active(h, ~0ull, -INFINITY)) return set_err(h, GVIZ_CUDA_ERR_CUDA);
   }
-  cudaMemcpy(it1.data(), h->d_iter, h->G * 8, cudaMemcpyDeviceToHost);
+  if (cudaMemcpy(it1.data(), h->d_iter, h->G * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
+    return set_err(h, GVIZ_CUDA_ERR_CUDA);
   if (rounds)
     for (size_t g = 0; g < h->G; g++) rounds[g] = it1[g] - it0[g];
   h->hostIteration += it1[0] - it0[0];
@@ -1374,7 +1381,8 @@ int gvizCudaForceExactRepulsion(gvizCudaForce *h, const uint32_t *targets,
   double2 *dout = h->d_exactRoom, *part = dout + n;
   uint32_t *dt = reinterpret_cast<uint32_t *>(part + parts);
   int rc = GVIZ_CUDA_OK;
-  if (put(h, dt, targets, n * 4)) {
+  // (on the kernel's own stream: 531 us a call at 4,096 of 131,072, 540 with put)
+  if (cudaMemcpyAsync(dt, targets, n * 4, cudaMemcpyHostToDevice, h->stream) == cudaSuccess) {
     enqueue_exact_judge(h, dt, n, dout, part);
     rc = sync_and_check(h);
   } else {
@@ -1717,12 +1725,13 @@ int gvizCudaForceLoadCheckpoint(gvizCudaForce *h, const char *filename, int rest
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return set_err(h, GVIZ_CUDA_ERR_CUDA);
   bool cok = true;
   if (V)
-    cok = put(h, h->d_pos, pos.data(), V * 16) && put(h, h->d_sf, sf.data(), V * 16) &&
-          put_zero(h, h->d_disp, V * 16);
-  cok = cok && put(h, h->d_speed, speed.data(), G * 8) && put(h, h->d_eff, eff.data(), G * 8) &&
-        put(h, h->d_iter, iter.data(), G * 8) && put(h, h->d_lastStats, last.data(), G * 40);
-  if (rows) cok = cok && put(h, h->d_stats, ring.data(), ring.size() * 8);
-  cok = put_done(h) && cok && set_all_active(h, ~0ull, -INFINITY);
+    cok = put(h->d_pos, pos.data(), V * 16) && put(h->d_sf, sf.data(), V * 16) &&
+          put_zero(h->d_disp, V * 16);
+  cok = cok && put(h->d_speed, speed.data(), G * 8) && put(h->d_eff, eff.data(), G * 8) &&
+        put(h->d_iter, iter.data(), G * 8) && put(h->d_lastStats, last.data(), G * 40);
+  if (rows) cok = cok && put(h->d_stats, ring.data(), ring.size() * 8);
+  cok = cok && set_all_active(h, ~0ull, -INFINITY);
+  cok = put_done() && cok;
   if (!cok) return set_err(h, GVIZ_CUDA_ERR_CUDA);
   h->begun = hd.begun != 0;
   h->hostIteration = hostIt;

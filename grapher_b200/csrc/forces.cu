@@ -28,9 +28,9 @@
 #include "internal.cuh"
 #include "mlp.cuh"
 
-int dir_table_upload_forces(const double *t, cudaStream_t st) {
-  return cudaMemcpyToSymbolAsync(c_dirTable, t, sizeof(double) * 2 * GVIZ_DIR_TABLE, 0,
-                                 cudaMemcpyHostToDevice, st) == cudaSuccess ? 0 : -1;
+int dir_table_upload_forces(const double *t) {
+  return cudaMemcpyToSymbol(c_dirTable, t, sizeof(double) * 2 * GVIZ_DIR_TABLE) ==
+                 cudaSuccess ? 0 : -1;
 }
 
 namespace {

@@ -359,8 +359,8 @@ void enqueue_group_export(gvizCudaForce *h, uint32_t *groupOf);
 void mlp_free(gvizCudaForce *h);
 int far_side_alloc(gvizCudaForce *h);
 void far_side_free(gvizCudaForce *h);
-int dir_table_upload_forces(const double *t, cudaStream_t st);
-int dir_table_upload_precise(const double *t, cudaStream_t st);
+int dir_table_upload_forces(const double *t);
+int dir_table_upload_precise(const double *t);
 
 // forces.cu (FP32, fused multiply-add on)
 void enqueue_attraction_f32(gvizCudaForce *h);

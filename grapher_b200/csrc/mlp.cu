@@ -34,7 +34,7 @@
 #define OFF_W3 (OFF_B2 + MLP_HID)
 #define OFF_B3 (OFF_W3 + MLP_OUTP * MLP_HID)
 
-struct gvizCudaMlp {  // everything, copies included, goes in the order of its stream
+struct gvizCudaMlp {
   int device = 0;
   cudaStream_t stream = nullptr;
   float *d_w = nullptr;      // FP32 masters (MLP_PAD)
@@ -970,7 +970,7 @@ int gvizCudaMlpCreate(gvizCudaMlp **out, int device, uint64_t seed) {
       cudaMalloc(&m->d_dev, sizeof(MlpDev)) != cudaSuccess ||
       cudaMalloc(&m->d_gsum, (MLP_PAD + 1) * 4) != cudaSuccess ||
       cudaMalloc(&m->d_status, 4) != cudaSuccess ||
-      cudaMemsetAsync(m->d_status, 0, 4, m->stream) != cudaSuccess) {
+      cudaMemset(m->d_status, 0, 4) != cudaSuccess) {
     gvizCudaMlpDestroy(m);
     return GVIZ_CUDA_ERR_ALLOC;
   }
@@ -1022,22 +1022,22 @@ int gvizCudaMlpSetTrainingKernels(gvizCudaMlp *m, int tcgen05) {
   return GVIZ_CUDA_OK;
 }
 
-// A copy to the device in the order of the model's stream, which does not wait
-// for copies of the legacy stream (those from pageable memory may return
-// before they end).
-static bool mlp_put(gvizCudaMlp *m, void *dst, const void *src, size_t bytes) {
-  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, m->stream) == cudaSuccess;
+// Copies to the device on the legacy stream, and the wait for them before the
+// model's stream, which does not wait for the legacy one, may read them (a copy
+// from pageable memory may return before it ends).
+static bool mlp_put(void *dst, const void *src, size_t bytes) {
+  return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
 }
+
+static bool mlp_put_done() { return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess; }
 
 int gvizCudaMlpSetWeights(gvizCudaMlp *m, const float *w) {
   if (!m || !w) return GVIZ_CUDA_ERR_ARG;
   cudaSetDevice(m->device);
-  if (!mlp_put(m, m->d_w, w, MLP_PAD * 4) ||
-      cudaMemsetAsync(m->d_m, 0, MLP_PAD * 4, m->stream) != cudaSuccess ||
-      cudaMemsetAsync(m->d_v, 0, MLP_PAD * 4, m->stream) != cudaSuccess) {
-    cudaStreamSynchronize(m->stream);  // the caller's weights may be on their way
+  if (!mlp_put(m->d_w, w, MLP_PAD * 4) ||
+      cudaMemset(m->d_m, 0, MLP_PAD * 4) != cudaSuccess ||
+      cudaMemset(m->d_v, 0, MLP_PAD * 4) != cudaSuccess || !mlp_put_done())
     return GVIZ_CUDA_ERR_CUDA;
-  }
   m->step = 0;
   k_mlp_to_dev<<<(MLP_PAD + 255) / 256, 256, 0, m->stream>>>(m->d_w, m->d_dev);
   return cudaStreamSynchronize(m->stream) == cudaSuccess ? GVIZ_CUDA_OK : GVIZ_CUDA_ERR_CUDA;
@@ -1089,7 +1089,8 @@ static int mlp_status(gvizCudaMlp *m) {
   if (cudaMemcpy(&st, m->d_status, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
     return GVIZ_CUDA_ERR_CUDA;
   if (st) {
-    cudaMemsetAsync(m->d_status, 0, 4, m->stream);
+    cudaMemset(m->d_status, 0, 4);
+    mlp_put_done();
     return GVIZ_CUDA_ERR_CUDA;
   }
   return GVIZ_CUDA_OK;
@@ -1107,8 +1108,9 @@ int gvizCudaMlpGradient(gvizCudaMlp *m, const float *X, const float *T,
   for (size_t i = 0; i < n; i++) wsum += W ? W[i] : 1.0;
   if (cudaMalloc(&dX, n * MLP_IN * 4) != cudaSuccess || cudaMalloc(&dT, n * 8) != cudaSuccess)
     return GVIZ_CUDA_ERR_ALLOC;
-  bool up = mlp_put(m, dX, X, n * MLP_IN * 4) && mlp_put(m, dT, T, n * 8);
-  if (W) up = up && cudaMalloc(&dW, n * 4) == cudaSuccess && mlp_put(m, dW, W, n * 4);
+  bool up = mlp_put(dX, X, n * MLP_IN * 4) && mlp_put(dT, T, n * 8);
+  if (W) up = up && cudaMalloc(&dW, n * 4) == cudaSuccess && mlp_put(dW, W, n * 4);
+  up = mlp_put_done() && up;
   uint32_t blocks = 0;
   int rc = up ? GVIZ_CUDA_OK : GVIZ_CUDA_ERR_CUDA;
   if (!rc)
@@ -1148,8 +1150,8 @@ int gvizCudaMlpTrain(gvizCudaMlp *m, const float *X, const float *T,
     rc = GVIZ_CUDA_ERR_ALLOC;
   std::vector<float> wn;
   if (!rc) {
-    if (!mlp_put(m, dX, X, n * MLP_IN * 4) || !mlp_put(m, dT, T, n * 8) ||
-        (W && !mlp_put(m, dW, W, n * 4)))
+    if (!mlp_put(dX, X, n * MLP_IN * 4) || !mlp_put(dT, T, n * 8) ||
+        (W && !mlp_put(dW, W, n * 4)) || !mlp_put_done())
       rc = GVIZ_CUDA_ERR_CUDA;
   }
   std::vector<uint32_t> order(n);
@@ -1223,7 +1225,7 @@ int gvizCudaMlpInfer(gvizCudaMlp *m, const float *X, size_t n, float *Y) {
   float *dX, *dY;
   if (cudaMalloc(&dX, n * MLP_IN * 4) != cudaSuccess || cudaMalloc(&dY, n * 8) != cudaSuccess)
     return GVIZ_CUDA_ERR_ALLOC;
-  int rc = mlp_put(m, dX, X, n * MLP_IN * 4) ? GVIZ_CUDA_OK : GVIZ_CUDA_ERR_CUDA;
+  int rc = mlp_put(dX, X, n * MLP_IN * 4) && mlp_put_done() ? GVIZ_CUDA_OK : GVIZ_CUDA_ERR_CUDA;
   const uint32_t blocks = (uint32_t)((n + 127) / 128);
   if (!rc) k_mlp_infer<<<blocks, 128, 0, m->stream>>>(m->d_dev, dX, (uint32_t)n, dY);
   if (cudaStreamSynchronize(m->stream) != cudaSuccess) rc = GVIZ_CUDA_ERR_CUDA;
@@ -1247,9 +1249,10 @@ int gvizCudaForceSetFarFieldModel(gvizCudaForce *h, gvizCudaMlp *m) {
   if (!h->d_mlp && cudaMalloc(&h->d_mlp, sizeof(MlpDev)) != cudaSuccess)
     return GVIZ_CUDA_ERR_ALLOC;
   cudaStreamSynchronize(m->stream);
-  if (cudaMemcpyAsync(h->d_mlp, m->d_dev, sizeof(MlpDev), cudaMemcpyDeviceToDevice, h->stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(h->stream) != cudaSuccess)  // the model may change or go after this
+  // after the steps in flight, and before anything that follows on either stream
+  if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
+      cudaMemcpy(h->d_mlp, m->d_dev, sizeof(MlpDev), cudaMemcpyDeviceToDevice) != cudaSuccess ||
+      !mlp_put_done())
     return GVIZ_CUDA_ERR_CUDA;
   int rc = far_side_alloc(h);
   h->graphDirty = true;

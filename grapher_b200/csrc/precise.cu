@@ -20,9 +20,9 @@
 #include "epilogue.cuh"
 #include "internal.cuh"
 
-int dir_table_upload_precise(const double *t, cudaStream_t st) {
-  return cudaMemcpyToSymbolAsync(c_dirTable, t, sizeof(double) * 2 * GVIZ_DIR_TABLE, 0,
-                                 cudaMemcpyHostToDevice, st) == cudaSuccess ? 0 : -1;
+int dir_table_upload_precise(const double *t) {
+  return cudaMemcpyToSymbol(c_dirTable, t, sizeof(double) * 2 * GVIZ_DIR_TABLE) ==
+                 cudaSuccess ? 0 : -1;
 }
 
 EpiArgs make_epi(gvizCudaForce *h) {

@@ -39,6 +39,7 @@ cudaError_t work(cudaStream_t st) {
 }
 
 cudaError_t legacy(void *dst, const void *src, size_t n, cudaMemcpyKind kind) {
+  if (kind != cudaMemcpyDeviceToHost && fails("cudaMemcpy")) return cudaErrorUnknown;
   memcpy(dst, src, n);
   legacyPending = kind != cudaMemcpyDeviceToHost;  // a copy to the host waits for the stream
   return cudaSuccess;
@@ -121,10 +122,6 @@ cudaError_t cudaMemset(void *d, int v, size_t n) {
 cudaError_t cudaMemcpyToSymbol(const void *, const void *, size_t, size_t, cudaMemcpyKind) {
   legacyPending = true;
   return cudaSuccess;
-}
-cudaError_t cudaMemcpyToSymbolAsync(const void *, const void *, size_t, size_t, cudaMemcpyKind,
-                                    cudaStream_t st) {
-  return work(st);
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t st) {
   if (fails(k == cudaMemcpyDeviceToHost ? "cudaMemcpyAsync to host" : "cudaMemcpyAsync"))

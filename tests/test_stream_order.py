@@ -78,9 +78,11 @@ def test_judge_targets_are_ordered_before_the_kernel(fake):
     assert fake.fake_unordered() == 0
     # an upload that fails is an error, and nothing runs on what was there before
     from grapher_b200._native import GvizCudaError
+    fake.fake_reset()
     fake.fake_fail_after(b"cudaMemcpyAsync", 0)
     with pytest.raises(GvizCudaError):
         lay.exact_repulsion(np.arange(9))
+    assert fake.fake_launches() == 0
     lay.close()
 
 
