@@ -21,7 +21,7 @@ ERRORS = {
     0: "ok", -1: "allocation failed", -2: "only 2-D layouts are supported",
     -3: "invalid argument", -4: "CUDA runtime error", -5: "Begin has not been called",
     -6: "a vertex position is NaN or infinite",
-    -7: "more than 4096 distinct points share one depth-32 quadtree cell",
+    -7: "more than 4096 distinct points share one quadtree cell of the sorted depth",
     -8: "no usable CUDA device", -9: "size beyond a supported limit",
 }
 

@@ -1533,7 +1533,7 @@ const char *gvizCudaErrorString(int code) {
     case GVIZ_CUDA_ERR_CUDA: return "CUDA runtime error";
     case GVIZ_CUDA_ERR_NOT_BEGUN: return "Begin has not been called";
     case GVIZ_CUDA_ERR_NONFINITE: return "a vertex position is NaN or infinite";
-    case GVIZ_CUDA_ERR_DEEP_RUN: return "more than 4096 distinct points share one depth-32 quadtree cell";
+    case GVIZ_CUDA_ERR_DEEP_RUN: return "more than 4096 distinct points share one quadtree cell of the sorted depth";
     case GVIZ_CUDA_ERR_NO_DEVICE: return "no usable CUDA device";
     case GVIZ_CUDA_ERR_LIMIT: return "size beyond a supported limit";
     default: return "unknown error";

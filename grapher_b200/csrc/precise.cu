@@ -414,8 +414,9 @@ __global__ __launch_bounds__(kThreads) void k_exact_f64(Exact64Args a) {
 // order. FP64 issue bounds the loop. Without overlap prevention a term is
 // num / d^2 along d: ten FP64 instructions on a straight-line path with a
 // reciprocal of its own, chunks of 32 sources that meet the target, a
-// coincident point or an extreme distance taken again with the division; with
-// overlap prevention it is the term of rep_term64. 4,096 targets among 131,072
+// coincident point or an extreme distance taken again with the division (or,
+// beyond the range, the root and divisions of rep_term64); with overlap
+// prevention it is the term of rep_term64. 4,096 targets among 131,072
 // vertices: 48 ms in 16 blocks of one serial sum, 0.90 split over blocks with
 // a division and three branches per term, 0.55 now (0.30 at the FP64 pipe's
 // rate). 8 / 16 / 24 / 32 / 48 blocks per SM of the 8 that fit take 0.77 / 0.62

@@ -427,10 +427,6 @@ void scan_exclusive(gvizCudaForce *h, const uint32_t *in, uint32_t *out,
                                                         total, h->d_status);
 }
 
-// Stable sort by the key bits above GVIZ_SORT_SKIP_BITS (an even number of
-// 8-bit passes, so the result ends in (keys, vals)); keys equal in those bits
-// keep their input order. The sort state is zero but for the first digit's
-// counts.
 // The scatter's shared memory exceeds the default per-block budget: opted
 // into once per device, at handle creation (outside any stream capture).
 void sort_set_smem_limits() {
@@ -442,6 +438,10 @@ void sort_set_smem_limits() {
                        (int)scatter_dyn(kSortThreads * 8));
 }
 
+// Stable sort by the key bits above GVIZ_SORT_SKIP_BITS (an even number of
+// 8-bit passes, so the result ends in (keys, vals)); keys equal in those bits
+// keep their input order. The sort state is zero but for the first digit's
+// counts.
 void radix_sort_pairs(gvizCudaForce *h, uint64_t *keys, uint32_t *vals,
                       uint64_t *keysAlt, uint32_t *valsAlt, size_t n) {
   if (n <= 1) return;

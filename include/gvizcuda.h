@@ -54,7 +54,9 @@ extern "C" {
 #define GVIZ_CUDA_ERR_NOT_BEGUN (-5)  /* Run/Step before Begin */
 #define GVIZ_CUDA_ERR_NONFINITE (-6)  /* a position was NaN or infinite */
 #define GVIZ_CUDA_ERR_DEEP_RUN (-7)   /* > 4096 distinct points share one
-                                         depth-32 quadtree cell */
+                                         quadtree cell of the sorted depth (24;
+                                         less in a batch: its graph number takes
+                                         sort bits) */
 #define GVIZ_CUDA_ERR_NO_DEVICE (-8)  /* no usable CUDA device */
 #define GVIZ_CUDA_ERR_LIMIT (-9)      /* size beyond a documented limit */
 
