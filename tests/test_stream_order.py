@@ -2,7 +2,6 @@
 device): which copies, memsets and launches it gives to which stream, and what
 it has waited for when it returns."""
 import ctypes
-import glob
 import os
 import subprocess
 
@@ -16,7 +15,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 def fake_path(tmp_path_factory):
     from grapher_b200 import build
     build.build()  # the objects, when they are not up to date
-    objs = sorted(glob.glob(os.path.join(build.BUILD, "*.o")))
+    objs = [os.path.join(build.BUILD, src + ".o") for src in build.SOURCES]
     out = str(tmp_path_factory.mktemp("fake") / "libgvizcuda_fake.so")
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic",
                     "-I/usr/local/cuda/include", "-o", out,
